@@ -9,6 +9,7 @@
 // has an inverse and its rows are sorted, otherwise the transpose of the
 // pull CSR built here once per graph by a stable sort on the neighbour id.
 #include "gbx_internal.cuh"
+#include "gbx_sort.cuh"
 
 #include <atomic>
 #include <condition_variable>

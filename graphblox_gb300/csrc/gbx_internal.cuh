@@ -331,6 +331,4 @@ void free_plan(gbx_gather_plan *p);
 int exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint32_t n, cudaStream_t s,
                        uint32_t *total_dev /* may be null */);
 int exclusive_scan_u64(const uint32_t *in, uint64_t *out, uint32_t n, cudaStream_t s);
-// stable LSD radix sort of (key, value) pairs on `bits` low key bits (gbx_sort.cu)
-int radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t n, int bits, cudaStream_t s);
 }  // namespace gbx

@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "gbx_internal.cuh"
+#include "gbx_sort.cuh"
 
 namespace gbx {
 

@@ -5,6 +5,7 @@
 #include <algorithm>
 
 #include "gbx_internal.cuh"
+#include "gbx_sort.cuh"
 
 namespace gbx {
 
@@ -14,30 +15,9 @@ static unsigned grid1d(uint64_t n) {
     return (unsigned)std::max<uint64_t>(1, std::min(b, cap));
 }
 
-__global__ void iota_kernel(uint32_t *a, uint32_t n) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = i;
-}
-
-// symmetric: second half holds every edge reversed (edgeList.c:559-576)
-__global__ void stage_edges_kernel(const uint32_t *src, const uint32_t *dst, const float *w,
-                                   uint32_t E, int symmetric, uint32_t *s, uint32_t *d, float *wo) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < E; i += gridDim.x * blockDim.x) {
-        uint32_t a = src[i], b = dst[i];
-        s[i] = a;
-        d[i] = b;
-        if (wo) wo[i] = w ? w[i] : 1.0f;
-        if (symmetric) {
-            s[i + E] = b;
-            d[i + E] = a;
-            if (wo) wo[i + E] = w ? w[i] : 1.0f;
-        }
-    }
-}
-
-__global__ void max_id_kernel(const uint32_t *s, const uint32_t *d, uint32_t n, uint32_t *out) {
+__global__ void max_u32_of_kernel(const uint32_t *a, uint32_t n, uint32_t *out) {
     uint32_t m = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        m = max(m, max(s[i], d[i]));
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, a[i]);
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
@@ -76,49 +56,40 @@ static int max_edge_id(const uint32_t *s, const uint32_t *d, uint32_t n, cudaStr
     return GBX_OK;
 }
 
-__global__ void gather_u32_kernel(const uint32_t *in, const uint32_t *perm, uint32_t n, uint32_t *out) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = in[perm[i]];
-}
-
-__global__ void gather_f32_kernel(const float *in, const uint32_t *perm, uint32_t n, float *out) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = in[perm[i]];
-}
-
-// removeDulpicatesSelfLoopEdges on a (src,dst)-sorted list: keep edge i when
-// it is not a self loop and differs from edge i-1 (edgeList.c:255-321)
-__global__ void dedup_flags_kernel(const uint32_t *s, const uint32_t *d, uint32_t n, uint32_t *keep) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t a = s[i], b = d[i];
-        bool k = a != b && (i == 0 || a != s[i - 1] || b != d[i - 1]);
-        keep[i] = k ? 1u : 0u;
-    }
-}
-
-// compaction; kept weights are truncated through uint32 as the reference's
-// uint32_t tempWeight does (edgeList.c:260,273)
-__global__ void compact_edges_kernel(const uint32_t *s, const uint32_t *d, const float *w,
-                                     const uint32_t *keep, const uint32_t *pos, uint32_t n,
-                                     uint32_t *so, uint32_t *dout, float *wo) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (!keep[i]) continue;
-        uint32_t p = pos[i];
-        so[p] = s[i];
-        dout[p] = d[i];
-        if (wo) wo[p] = (float)(uint32_t)w[i];
-    }
-}
-
 // mapVerticesWithInOutDegree_base (vertex.c:204-328) on a source-sorted edge
 // list: each run of equal sources writes its first position (idx) and its end
 // (into deg); degrees_from_runs_kernel turns the end into the run length. No
 // atomics: a hub's run would otherwise take one atomic per edge on one address.
-__global__ void map_vertices_kernel(const uint32_t *s, uint32_t n, uint32_t *deg, uint32_t *idx) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t v = s[i] & kIdMask;
-        if (i == 0 || v != (s[i - 1] & kIdMask)) idx[v] = i;
-        if (i + 1 == n || v != (s[i + 1] & kIdMask)) deg[v] = i + 1;
+// kept: the edge count when only the device knows it yet. Four edges per
+// thread and, where the list allows it, per load.
+__global__ void map_vertices_kernel(const uint32_t *s, uint32_t n, const uint32_t *kept, uint32_t V, uint32_t *deg,
+                                    uint32_t *idx) {
+    if (kept) n = min(n, *kept);
+    const bool wide = ((uintptr_t)s & 15u) == 0;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x * 4;
+    for (uint64_t i0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i0 < n; i0 += step) {
+        const uint32_t i = (uint32_t)i0, m = min(4u, n - i);
+        uint32_t v[4];
+        if (wide && m == 4) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(s + i);
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+        } else {
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) v[q] = q < m ? s[i + q] : 0u;
+        }
+        uint32_t before = i ? s[i - 1] & kIdMask : 0u;
+        const uint32_t after = i + m < n ? s[i + m] & kIdMask : 0u;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            if (q >= m) break;
+            const uint32_t x = v[q] & kIdMask;
+            const uint32_t next = q + 1 < m ? v[(q + 1) & 3] & kIdMask : after;
+            if (x < V) {
+                if (i + q == 0 || x != before) idx[x] = i + q;
+                if (i + q + 1 == n || x != next) deg[x] = i + q + 1;
+            }
+            before = x;
+        }
     }
 }
 
@@ -138,16 +109,34 @@ __device__ __forceinline__ void count_keys(uint32_t *deg, uint32_t key, unsigned
     }
 }
 
-__global__ void degree_count_kernel(const uint32_t *s, const uint32_t *d, uint32_t n, int lmode,
-                                    uint32_t *deg) {
+// Degrees and, in the same read of the edges, the largest id: an edge with an
+// end outside [0, V) raises *max_id to at least V and is not counted. Four
+// edges per lane are loaded before the first is counted.
+__global__ void degree_count_kernel(const uint32_t *s, const uint32_t *d, uint32_t n, uint32_t V, int lmode,
+                                    uint32_t *deg, uint32_t *max_id) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t stride = gridDim.x * blockDim.x;  // a multiple of 32
-    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += stride) {
-        const uint32_t i = base + lane;
-        const unsigned active = __ballot_sync(0xffffffffu, i < n);
-        if (lmode == 2 || lmode == 3) count_keys(deg, i < n ? d[i] : 0u, active);
-        if (lmode != 2) count_keys(deg, i < n ? s[i] : 0u, active);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;  // a multiple of 32
+    uint32_t m = 0;
+    for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; base < n; base += 4 * stride) {
+        uint32_t a[4], b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t i = base + q * stride + lane;
+            a[q] = i < n ? s[i] : 0u;
+            b[q] = i < n ? d[i] : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t i = base + q * stride + lane;
+            const uint32_t top = max(a[q], b[q]);
+            m = max(m, top);
+            const unsigned active = __ballot_sync(0xffffffffu, i < n && top < V);
+            if (lmode == 2 || lmode == 3) count_keys(deg, b[q], active);
+            if (lmode != 2) count_keys(deg, a[q], active);
+        }
     }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) atomicMax(max_id, m);
 }
 
 __global__ void new_labels_kernel(const uint32_t *sorted_ids, uint32_t V, uint32_t *newlab) {
@@ -155,10 +144,30 @@ __global__ void new_labels_kernel(const uint32_t *sorted_ids, uint32_t V, uint32
         newlab[sorted_ids[i]] = V - 1 - i;
 }
 
+// Four edges per thread: eight id loads, then eight gathers in flight.
 __global__ void relabel_edges_kernel(uint32_t *s, uint32_t *d, uint32_t n, const uint32_t *newlab) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        s[i] = newlab[s[i]];
-        d[i] = newlab[d[i]];
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += 4 * step) {
+        uint32_t a[4], b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t j = i + q * step;
+            a[q] = j < n ? __ldcs(s + j) : 0u;
+            b[q] = j < n ? __ldcs(d + j) : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            a[q] = __ldg(newlab + a[q]);
+            b[q] = __ldg(newlab + b[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t j = i + q * step;
+            if (j < n) {
+                __stcs(s + j, a[q]);
+                __stcs(d + j, b[q]);
+            }
+        }
     }
 }
 
@@ -271,96 +280,44 @@ extern "C" int gbx_csr_build(uint32_t num_edges, const uint32_t *src, const uint
     InArray<float> iw;
     GBX_TRY(isrc.bind(src, E, s));
     GBX_TRY(idst.bind(dst, E, s));
-    GBX_TRY(iw.bind(w, E, s));
-    const bool want_w = w_out != nullptr;
-    DevBuf<uint32_t> es, ed, perm, keys;
-    DevBuf<float> ew;
-    GBX_TRY(es.alloc(E2, s));
-    GBX_TRY(ed.alloc(E2, s));
-    GBX_TRY(perm.alloc(E2, s));
-    GBX_TRY(keys.alloc(E2, s));
-    if (want_w) GBX_TRY(ew.alloc(E2, s));
-    if (E) {
-        stage_edges_kernel<<<grid1d(E), 256, 0, s>>>(isrc.d, idst.d, iw.d, E, symmetric, es.p, ed.p,
-                                                     want_w ? ew.p : nullptr);
-        GBX_LAUNCH_CHECK();
-    }
-    // ids may carry the mask bits of mask mode: the vertex is the id without
-    // them, the sort key the whole id (the reference radix-sorts all 32 bits)
-    uint32_t hmax = 0, hmasked = 0;
-    GBX_TRY(max_edge_id(es.p, ed.p, E2, s, &hmax, &hmasked));
-    GBX_REQUIRE(E2 == 0 || hmasked < V, GBX_ERR_INVALID, "vertex id %u >= num_vertices %u", hmasked, V);
-    const int bits = bits_for(hmax);
-    // stable sort: destination pass(es) first, then source (LSD on the pair)
-    iota_kernel<<<grid1d(E2), 256, 0, s>>>(perm.p, E2);
-    GBX_LAUNCH_CHECK();
-    if (sort_mode == 1 || sort_mode == 3) {
-        GBX_CUDA(cudaMemcpyAsync(keys.p, ed.p, (size_t)E2 * 4, cudaMemcpyDeviceToDevice, s));
-        GBX_TRY(radix_sort_pairs(keys.p, perm.p, E2, bits, s));
-    }
-    gather_u32_kernel<<<grid1d(E2), 256, 0, s>>>(es.p, perm.p, E2, keys.p);
-    GBX_LAUNCH_CHECK();
-    GBX_TRY(radix_sort_pairs(keys.p, perm.p, E2, bits, s));
-    // apply the permutation
-    DevBuf<uint32_t> ss, sd, keep, pos, tot;
-    DevBuf<float> sw;
-    GBX_TRY(ss.alloc(E2, s));
-    GBX_TRY(sd.alloc(E2, s));
-    if (want_w) GBX_TRY(sw.alloc(E2, s));
-    GBX_CUDA(cudaMemcpyAsync(ss.p, keys.p, (size_t)E2 * 4, cudaMemcpyDeviceToDevice, s));
-    gather_u32_kernel<<<grid1d(E2), 256, 0, s>>>(ed.p, perm.p, E2, sd.p);
-    if (want_w) gather_f32_kernel<<<grid1d(E2), 256, 0, s>>>(ew.p, perm.p, E2, sw.p);
-    GBX_LAUNCH_CHECK();
-    uint32_t Eout = E2;
+    GBX_TRY(iw.bind(w_out ? w : nullptr, E, s));
+    // outputs the caller does not want, or wants in host memory, go to working memory
+    DevBuf<uint32_t> ss, sd;
     OutArray<uint32_t> os, od, odeg, oidx;
     OutArray<float> ow;
-    const uint32_t *fs = ss.p, *fd = sd.p;
-    const float *fw = sw.p;
-    if (dedup && E2) {
-        GBX_TRY(keep.alloc(E2, s));
-        GBX_TRY(pos.alloc(E2, s));
-        GBX_TRY(tot.alloc(1, s));
-        dedup_flags_kernel<<<grid1d(E2), 256, 0, s>>>(ss.p, sd.p, E2, keep.p);
-        GBX_LAUNCH_CHECK();
-        GBX_TRY(exclusive_scan_u32(keep.p, pos.p, E2, s, tot.p));
-        GBX_CUDA(cudaMemcpyAsync(&Eout, tot.p, 4, cudaMemcpyDeviceToHost, s));
-        GBX_CUDA(cudaStreamSynchronize(s));
-        // compact into es/ed/ew (free now)
-        compact_edges_kernel<<<grid1d(E2), 256, 0, s>>>(ss.p, sd.p, sw.p, keep.p, pos.p, E2, es.p,
-                                                        ed.p, want_w ? ew.p : nullptr);
-        GBX_LAUNCH_CHECK();
-        fs = es.p;
-        fd = ed.p;
-        fw = ew.p;
-    }
+    GBX_TRY(os.bind(src_out, E2, s));
+    GBX_TRY(od.bind(dst_out, E2, s));
+    GBX_TRY(ow.bind(w_out, E2, s));
+    if (!src_out) GBX_TRY(ss.alloc(E2, s));
+    if (!dst_out) GBX_TRY(sd.alloc(E2, s));
+    uint32_t *fs = src_out ? os.d : ss.p;
+    DevBuf<SortControl> ctl;
+    GBX_TRY(sort_edges(EdgeView{isrc.d, idst.d, E, symmetric}, iw.d, sort_mode == 1 || sort_mode == 3, dedup != 0, V,
+                       fs, dst_out ? od.d : sd.p, ow.d, &ctl, s));
     GBX_TRY(odeg.bind(out_degree, V, s));
     GBX_TRY(oidx.bind(edges_idx, V, s));
     GBX_CUDA(cudaMemsetAsync(odeg.d, 0, (size_t)V * 4, s));
     GBX_CUDA(cudaMemsetAsync(oidx.d, 0, (size_t)V * 4, s));
-    if (Eout) {
-        map_vertices_kernel<<<grid1d(Eout), 256, 0, s>>>(fs, Eout, odeg.d, oidx.d);
+    if (E2) {
+        map_vertices_kernel<<<grid1d(ceil_div(E2, 4)), 256, 0, s>>>(fs, E2, dedup ? &ctl.p->kept : nullptr, V, odeg.d,
+                                                                    oidx.d);
         GBX_LAUNCH_CHECK();
         degrees_from_runs_kernel<<<grid1d(V), 256, 0, s>>>(odeg.d, oidx.d, V);
         GBX_LAUNCH_CHECK();
     }
+    SortControl h;
+    GBX_CUDA(cudaMemcpyAsync(&h, ctl.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+    GBX_CUDA(cudaStreamSynchronize(s));
+    GBX_TRY(check_sort(h));
+    const uint32_t Eout = dedup ? h.kept : E2;
     GBX_TRY(odeg.finish(s));
     GBX_TRY(oidx.finish(s));
-    if (src_out) {
-        GBX_TRY(os.bind(src_out, Eout, s));
-        GBX_CUDA(cudaMemcpyAsync(os.d, fs, (size_t)Eout * 4, cudaMemcpyDeviceToDevice, s));
-        GBX_TRY(os.finish(s));
-    }
-    if (dst_out) {
-        GBX_TRY(od.bind(dst_out, Eout, s));
-        GBX_CUDA(cudaMemcpyAsync(od.d, fd, (size_t)Eout * 4, cudaMemcpyDeviceToDevice, s));
-        GBX_TRY(od.finish(s));
-    }
-    if (want_w) {
-        GBX_TRY(ow.bind(w_out, Eout, s));
-        GBX_CUDA(cudaMemcpyAsync(ow.d, fw, (size_t)Eout * 4, cudaMemcpyDeviceToDevice, s));
-        GBX_TRY(ow.finish(s));
-    }
-    GBX_CUDA(cudaStreamSynchronize(s));
+    os.n = od.n = ow.n = Eout;
+    GBX_TRY(os.finish(s));
+    GBX_TRY(od.finish(s));
+    GBX_TRY(ow.finish(s));
+    if (odeg.to_host() || oidx.to_host() || os.to_host() || od.to_host() || ow.to_host())
+        GBX_CUDA(cudaStreamSynchronize(s));
     *num_edges_out = Eout;
     return GBX_OK;
 }
@@ -389,29 +346,28 @@ extern "C" int gbx_degree_reorder(uint32_t num_vertices, uint32_t num_edges, uin
     if (os.to_host() && E) GBX_CUDA(cudaMemcpyAsync(os.d, src, (size_t)E * 4, cudaMemcpyHostToDevice, s));
     if (od.to_host() && E) GBX_CUDA(cudaMemcpyAsync(od.d, dst, (size_t)E * 4, cudaMemcpyHostToDevice, s));
     if (ol.to_host()) GBX_CUDA(cudaMemcpyAsync(ol.d, labels, (size_t)V * 4, cudaMemcpyHostToDevice, s));
-    uint32_t id_max = 0, id_masked = 0;
-    GBX_TRY(max_edge_id(os.d, od.d, E, s, &id_max, &id_masked));
-    GBX_REQUIRE(E == 0 || id_max < V, GBX_ERR_INVALID, "vertex id %u >= num_vertices %u", id_max, V);
     DevBuf<uint32_t> deg, ids, newlab, mx;
     GBX_TRY(deg.alloc(V, s));
     GBX_TRY(ids.alloc(V, s));
     GBX_TRY(newlab.alloc(V, s));
-    GBX_TRY(mx.alloc(1, s));
+    GBX_TRY(mx.alloc(2, s));  // largest degree, largest id
     GBX_CUDA(cudaMemsetAsync(deg.p, 0, (size_t)V * 4, s));
+    GBX_CUDA(cudaMemsetAsync(mx.p, 0, 8, s));
     // reorderGraphGenerateInOutDegrees (reorder.c:1483-1552): in-degrees for
     // 2, 5, 7, 9, in + out for 3, out-degrees for every other mode
     const bool in_deg = lmode == 2 || lmode == 5 || lmode == 7 || lmode == 9;
     const int count_mode = in_deg ? 2 : (lmode == 3 ? 3 : 1);
     if (E) {
-        degree_count_kernel<<<grid1d(E), 256, 0, s>>>(os.d, od.d, E, count_mode, deg.p);
+        degree_count_kernel<<<grid1d(ceil_div(E, 4)), 256, 0, s>>>(os.d, od.d, E, V, count_mode, deg.p, mx.p + 1);
         GBX_LAUNCH_CHECK();
     }
-    GBX_CUDA(cudaMemsetAsync(mx.p, 0, 4, s));
-    max_id_kernel<<<grid1d(V), 256, 0, s>>>(deg.p, deg.p, V, mx.p);
+    max_u32_of_kernel<<<grid1d(V), 256, 0, s>>>(deg.p, V, mx.p);
     GBX_LAUNCH_CHECK();
-    uint32_t hmax = 0;
-    GBX_CUDA(cudaMemcpyAsync(&hmax, mx.p, 4, cudaMemcpyDeviceToHost, s));
+    uint32_t hm[2];
+    GBX_CUDA(cudaMemcpyAsync(hm, mx.p, 8, cudaMemcpyDeviceToHost, s));
     GBX_CUDA(cudaStreamSynchronize(s));
+    const uint32_t hmax = hm[0];
+    GBX_REQUIRE(E == 0 || hm[1] < V, GBX_ERR_INVALID, "vertex id %u >= num_vertices %u", hm[1], V);
     // thresholds of the bucketed modes: t0 = avg <= 1 ? 1 : avg/2 (HUBCluster:
     // avg), doubling, last UINT32_MAX; avg = E/V in uint32 as the reference's
     // EdgeList.avg_degree
@@ -426,9 +382,7 @@ extern "C" int gbx_degree_reorder(uint32_t num_vertices, uint32_t num_edges, uin
     if (th.n == 0) {
         // reorderGraphListDegree (reorder.c:296-380): stable ascending sort of
         // (degree, id), label N-1-rank
-        iota_kernel<<<grid1d(V), 256, 0, s>>>(ids.p, V);
-        GBX_LAUNCH_CHECK();
-        GBX_TRY(radix_sort_pairs(deg.p, ids.p, V, bits_for(hmax), s));
+        GBX_TRY(radix_sort_pairs(deg.p, ids.p, V, bits_for(hmax), s, true));
         new_labels_kernel<<<grid1d(V), 256, 0, s>>>(ids.p, V, newlab.p);
         GBX_LAUNCH_CHECK();
     } else if (lmode == 6 || lmode == 7) {
@@ -457,9 +411,7 @@ extern "C" int gbx_degree_reorder(uint32_t num_vertices, uint32_t num_edges, uin
         // highest, ids ascending inside a bucket
         bucket_key_kernel<<<grid1d(V), 256, 0, s>>>(deg.p, V, th, deg.p);
         GBX_LAUNCH_CHECK();
-        iota_kernel<<<grid1d(V), 256, 0, s>>>(ids.p, V);
-        GBX_LAUNCH_CHECK();
-        GBX_TRY(radix_sort_pairs(deg.p, ids.p, V, bits_for(th.n - 1), s));
+        GBX_TRY(radix_sort_pairs(deg.p, ids.p, V, bits_for(th.n - 1), s, true));
         rank_labels_kernel<<<grid1d(V), 256, 0, s>>>(ids.p, V, newlab.p);
         GBX_LAUNCH_CHECK();
     }
@@ -546,15 +498,16 @@ extern "C" int gbx_mask_graph(uint32_t num_vertices, uint32_t num_edges, uint32_
     GBX_TRY(max_edge_id(os.d, od.d, E, s, &id_max, &id_masked));
     GBX_REQUIRE(E == 0 || id_max < V, GBX_ERR_INVALID,
                 "vertex id %u >= num_vertices %u (ids must not carry mask bits yet)", id_max, V);
-    DevBuf<uint32_t> key, ids;
+    DevBuf<uint32_t> key, ids, seen;
     GBX_TRY(key.alloc(V, s));
     GBX_TRY(ids.alloc(V, s));
+    GBX_TRY(seen.alloc(1, s));  // the largest id again, not read
     GBX_CUDA(cudaMemsetAsync(key.p, 0, (size_t)V * 4, s));
     // maskGraphProcessGenerateInOutDegrees (reorder.c:1260-1306): in-degrees
     // for 2, 4, in + out for 5, 6, out-degrees otherwise
     const int count_mode = (mmode == 2 || mmode == 4) ? 2 : (mmode == 5 || mmode == 6) ? 3 : 1;
     if (E) {
-        degree_count_kernel<<<grid1d(E), 256, 0, s>>>(os.d, od.d, E, count_mode, key.p);
+        degree_count_kernel<<<grid1d(ceil_div(E, 4)), 256, 0, s>>>(os.d, od.d, E, V, count_mode, key.p, seen.p);
         GBX_LAUNCH_CHECK();
     }
     // DBG's 11 buckets (reorder.c:1214-1228), highest first, ids ascending
@@ -566,9 +519,7 @@ extern "C" int gbx_mask_graph(uint32_t num_vertices, uint32_t num_edges, uint32_
     th.t[th.n - 1] = 0xFFFFFFFFu;
     bucket_key_kernel<<<grid1d(V), 256, 0, s>>>(key.p, V, th, key.p);
     GBX_LAUNCH_CHECK();
-    iota_kernel<<<grid1d(V), 256, 0, s>>>(ids.p, V);
-    GBX_LAUNCH_CHECK();
-    GBX_TRY(radix_sort_pairs(key.p, ids.p, V, bits_for(th.n - 1), s));
+    GBX_TRY(radix_sort_pairs(key.p, ids.p, V, bits_for(th.n - 1), s, true));
     // region sizes (reorder.c:1329-1345) with cs = cache_size / 4: V/4 each
     // when V - cs < 2 cs, else cs*8, *4, *4 in uint32 as the reference
     const uint32_t cs = cache_size >> 2;

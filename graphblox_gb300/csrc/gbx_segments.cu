@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "gbx_internal.cuh"
+#include "gbx_sort.cuh"
 
 namespace gbx {
 namespace {
