@@ -450,6 +450,7 @@ int gbx_graph_destroy(gbx_graph *g) {
     gbx_free_ms_plan(g->ms_plan);
     gbx_free_pr_cache(g->pr_cache);
     gbx_free_bc_cache(g->bc_cache);
+    gbx_free_pull_layout(g->pull_layout);
     dev_free(g->arena);
     free_plan(g->plan_fwd);
     free_plan(g->plan_inv);

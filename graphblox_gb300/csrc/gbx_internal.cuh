@@ -236,8 +236,12 @@ struct gbx_graph {
     struct gbx_ppr_cache *ppr = nullptr;
     // multi-source BFS: heavy pull-row chunks (gbx_msbfs.cu)
     struct gbx_ms_plan *ms_plan = nullptr;
-    // PageRank working memory and captured iteration loop (gbx_pagerank.cu)
+    // PageRank working memory (gbx_pagerank.cu)
     struct gbx_pr_cache *pr_cache = nullptr;
+    // hot-table pull engine (gbx_pull.cu): its layout, the sweeps asked for
+    // before it was built, and attempts that found no memory for it
+    struct gbx_pull_layout *pull_layout = nullptr;
+    uint32_t pull_sweeps = 0, pull_layout_tries = 0;
     // betweenness centrality: successor CSR with ascending rows (gbx_bc.cu)
     struct gbx_bc_cache *bc_cache = nullptr;
     // device scratch lent to one synchronous call at a time (gbx::Scratch)
@@ -258,6 +262,7 @@ void gbx_free_ppr_cache(struct gbx_ppr_cache *c);
 void gbx_free_ms_plan(struct gbx_ms_plan *p);
 void gbx_free_pr_cache(struct gbx_pr_cache *c);
 void gbx_free_bc_cache(struct gbx_bc_cache *c);
+void gbx_free_pull_layout(struct gbx_pull_layout *l);
 
 namespace gbx {
 // Long-lived device arrays (a graph's arrays, scratch arena and plans) come

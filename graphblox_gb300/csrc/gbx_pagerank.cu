@@ -1,31 +1,36 @@
 // Pull PageRank (the reference's pageRankPullGraphCSR, pageRank.c:245-368).
 //
-// One fused kernel per iteration: for every vertex v the pull engine sums
-// contrib[u] over v's in-edges, and the epilogue computes
+// Per iteration: for every vertex v a pull engine sums contrib[u] over v's
+// in-edges, and the epilogue computes
 //   next = base_pr + damp * sum           (base_pr = 1 - 0.85f, damp = 0.85f)
 //   contrib_next[v] = next / outdeg(v)    (0 for dangling vertices)
 //   |next - prev| -> FP64 error sum, active count (>= epsilon)
 // so the reference's three V-sized passes (contrib, gather, update) become
-// one sweep. Ranks and contributions ping-pong between two buffers.
-//
-// Iterations are launched back to back with no host round trip; iteration
-// `it` returns immediately when iteration it-1 left no active vertex, which
+// one sweep. Ranks and contributions ping-pong between two buffers. An
+// iteration that follows one with no active vertex is not run, which
 // reproduces the reference's early exit (stats->iterations = the index of the
 // iteration with no active vertex). A final kernel divides by N (:344-350).
-// The loop (state reset, initial ranks, the iterations) is captured once per
-// graph and (max_iterations, epsilon) as a CUDA graph on working memory kept
-// with the graph, and replayed by every later call: one graph launch and the
-// finishing kernel per call.
+//
+// From kLayoutSweeps iterations on (over all calls on the graph) the sweeps
+// run on the hot-table engine (gbx_pull.cuh) in one persistent kernel, one
+// CTA per SM: each iteration loads the hot sources' contributions into shared
+// memory, deals the edge units and ends at a grid barrier. Fewer iterations,
+// and those of small graphs, run as one launch each on the row engine
+// (gbx_gather.cuh), which needs no layout; that loop (state reset, initial
+// ranks, the iterations) is captured once per graph and (max_iterations,
+// epsilon) as a CUDA graph and replayed by every later call. With epsilon = 0 no iteration's residual but the last is asked for,
+// so ranks are written in the last two only; a row's epilogue is its degree
+// and one contribution.
 #include <algorithm>
 
-#include "gbx_gather.cuh"
+#include "gbx_pull.cuh"
 
 namespace gbx {
 
 struct PrIterState {
     double err;
     unsigned active;
-    unsigned pad;
+    unsigned cursor;  // next unit of the hot-table engine
 };
 
 struct PrTerm {
@@ -120,7 +125,7 @@ __global__ void pr_finish_kernel(const float *r0, const float *r1, const PrIterS
     }
 }
 
-// Enqueue the iteration loop: state reset, initial ranks, max_it iterations.
+// Enqueue the row engine's loop: state reset, initial ranks, max_it iterations.
 static int pr_enqueue_loop(gbx_graph *g, const gbx_gather_plan &plan, uint32_t max_it, double epsilon, float *rbuf,
                            float *cbuf, PrIterState *st, cudaStream_t s, uint32_t *kernels) {
     const uint32_t V = g->V;
@@ -147,30 +152,167 @@ static int pr_enqueue_loop(gbx_graph *g, const gbx_gather_plan &plan, uint32_t m
     return GBX_OK;
 }
 
+// ---- hot-table engine -----------------------------------------------------------
+
+// Contributions: slots first, then one entry per vertex (used by those
+// without a slot). Other SMs wrote them in the previous iteration, so they are
+// not read through the read-only path; the grid barrier's acquire drops what
+// L1 holds of them.
+struct PrHotTerm {
+    const float *cold;
+    struct Factors {};
+    __device__ __forceinline__ void factors(uint32_t, uint32_t, uint32_t, Factors &) const {}
+    __device__ __forceinline__ void scale(const Factors &, float (&)[4]) const {}
+};
+
+struct PrHotEpi {
+    const float *r_cur;
+    float *r_next;
+    float *c_next;  // slots, then vertices
+    uint32_t hot;
+    const uint32_t *__restrict__ row_degree;  // out-degrees in row order
+    double epsilon, inv_n;
+    double err;
+    unsigned active;
+    bool write, reduce;
+    __device__ __forceinline__ void prefetch(uint32_t row) const {
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(row_degree + row));
+    }
+    __device__ __forceinline__ void operator()(uint32_t row, uint32_t v, uint32_t slot, float sum) {
+        const float next = __fadd_rn(1.0f - 0.85f, __fmul_rn(0.85f, sum));
+        const uint32_t d = __ldg(row_degree + row);
+        // dangling: nobody reads it, and it stays 0 where a graph without an
+        // inverse lists such a vertex as a source
+        if (d) c_next[slot != ~0u ? slot : hot + v] = __fdiv_rn(next, (float)d);
+        if (write) {
+            if (reduce) {
+                const double e = (double)fabsf(__fsub_rn(next, r_cur[v]));
+                err += e * inv_n;
+                active += (e >= epsilon) ? 1u : 0u;
+            }
+            r_next[v] = next;
+        }
+    }
+};
+
+// floats per contribution buffer: the slots of both start on 16 bytes
+__host__ __device__ inline size_t contrib_stride(uint32_t V, uint32_t hot) { return ((size_t)V + hot + 3) & ~(size_t)3; }
+
+// both buffers of ranks and contributions at the first iteration's values
+// (rows without in-edges keep them)
+__global__ void pr_hot_init_kernel(float *r, float *c, const uint32_t *out_degree, uint32_t V, uint32_t hot,
+                                   const uint32_t *hot_ids) {
+    const float base = 1.0f - 0.85f;
+    const uint32_t n = hot + V;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t v = i < hot ? hot_ids[i] : i - hot;
+        const uint32_t d = v < V ? out_degree[v] : 0u;
+        const float x = d ? __fdiv_rn(base, (float)d) : 0.0f;
+        c[i] = x;
+        c[i + contrib_stride(V, hot)] = x;
+        if (i >= hot) {
+            r[v] = base;
+            r[v + V] = base;
+        }
+    }
+}
+
+__global__ void pr_row_degree_kernel(const uint2 *rows, uint32_t n, const uint32_t *out_degree, uint32_t *row_degree) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        row_degree[i] = out_degree[rows[i].x];
+}
+
+struct PrHotArgs {
+    gbx_pull_layout layout;
+    float *r, *c;
+    const uint32_t *row_degree;
+    PrIterState *state;
+    PullPieces pieces;
+    GridSync *sync;
+    uint32_t max_it;
+    double epsilon;
+};
+
+__global__ void __launch_bounds__(kPullThreads, 1) pr_hot_kernel(PrHotArgs a) {
+    extern __shared__ __align__(16) float s_hot[];
+    __shared__ double sd[32];
+    __shared__ unsigned su[32];
+    const uint32_t V = a.layout.V, hot = a.layout.hot;
+    const size_t stride = contrib_stride(V, hot);
+    float *buf = s_hot + hot + 4 + (threadIdx.x >> 5) * kPullBuf;
+    grid_barrier_init();
+    for (uint32_t it = 0; it < a.max_it; ++it) {
+        const uint32_t p = it & 1, q = p ^ 1;
+        PrHotTerm term{a.c + p * stride + hot};
+        // with epsilon = 0 every vertex stays active: only the last
+        // iteration's residual (reported as error_total) is reduced
+        const bool reduce = a.epsilon > 0.0 || it + 1 == a.max_it;
+        const bool write = reduce || it + 2 == a.max_it;
+        PrHotEpi epi{a.r + (size_t)p * V, a.r + (size_t)q * V, a.c + q * stride, hot, a.row_degree, a.epsilon,
+                     1.0 / (double)V, 0.0, 0u, write, reduce};
+        PullSweep<PrHotTerm, PrHotEpi> sweep{a.layout, (uint32_t)__cvta_generic_to_shared(s_hot), buf, term, epi,
+                                               a.pieces};
+        // the first unit's words do not wait for the slots
+        typename PullSweep<PrHotTerm, PrHotEpi>::Start first{};
+        if (first_unit() < a.layout.n_units) first = sweep.start(first_unit());
+        load_hot(a.c + p * stride, hot, s_hot);
+        deal_units(sweep, &a.state[it].cursor, first);
+        if (reduce) {
+            const double te = block_sum(epi.err, sd);
+            const unsigned ta = block_sum(epi.active, su);
+            if (threadIdx.x == 0) {
+                if (te != 0.0) atomicAdd(&a.state[it].err, te);
+                if (ta) atomicAdd(&a.state[it].active, ta);
+            }
+        }
+        if (it + 1 == a.max_it) break;
+        if (!grid_barrier(a.sync)) return;
+        if (a.epsilon > 0.0 && __ldcg(&a.state[it].active) == 0) break;
+    }
+}
+
 }  // namespace gbx
 
-// Per-graph PageRank working memory and the iteration loop captured as a CUDA
-// graph (re-captured when max_iterations or epsilon change). Calls on one
-// graph object are serialised by the caller, as for every other entry point.
+// Per-graph PageRank working memory and the row engine's captured loop
+// (re-captured when max_iterations, epsilon or its buffers change). Calls on
+// one graph object are serialised by the caller, as for every other entry point.
 struct gbx_pr_cache {
-    float *rbuf = nullptr, *cbuf = nullptr;  // 2V each: ping-pong ranks / contributions
-    gbx::PrIterState *st = nullptr;
-    gbx_pr_result *res = nullptr;
-    uint32_t cap = 0;  // slots in st
+    float *rbuf = nullptr;   // 2V: ping-pong ranks
+    float *cbuf = nullptr;   // ping-pong contributions, 2V or 2 (slots + V)
+    size_t cbuf_n = 0;
+    // the result and the grid barrier's words, then one state per iteration
+    struct Tail {
+        gbx_pr_result res;
+        gbx::GridSync sync;
+    } *tail = nullptr;
+    gbx::PrIterState *st = nullptr;  // behind *tail
+    uint32_t cap = 0;                // states
+    // hot-table engine: pieces of cut rows and their tickets (zero between
+    // sweeps), out-degrees in row order
+    float *sums = nullptr;
+    unsigned *tickets = nullptr;
+    uint32_t *row_degree = nullptr;
     cudaStream_t cap_stream = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint32_t key_it = 0, kernels = 0;
     double key_eps = -1.0;
+    void drop_capture() {
+        if (exec) cudaGraphExecDestroy(exec);
+        exec = nullptr;
+    }
 };
+static_assert(sizeof(gbx_pr_cache::Tail) % alignof(gbx::PrIterState) == 0, "states follow on their alignment");
 
 void gbx_free_pr_cache(gbx_pr_cache *c) {
     if (!c) return;
-    if (c->exec) cudaGraphExecDestroy(c->exec);
+    c->drop_capture();
     if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
     cudaFree(c->rbuf);
     cudaFree(c->cbuf);
-    cudaFree(c->st);
-    cudaFree(c->res);
+    cudaFree(c->tail);
+    cudaFree(c->sums);
+    cudaFree(c->tickets);
+    cudaFree(c->row_degree);
     delete c;
 }
 
@@ -178,33 +320,50 @@ using namespace gbx;
 
 namespace {
 
-int pr_cache(gbx_graph *g, uint32_t max_it, gbx_pr_cache **out) {
+int pr_cache(gbx_graph *g, const gbx_pull_layout *l, uint32_t max_it, cudaStream_t s, gbx_pr_cache **out) {
     gbx_pr_cache *c = g->pr_cache;
-    if (!c) {
-        c = new gbx_pr_cache();
-        g->pr_cache = c;
-        GBX_CUDA(cudaMalloc(&c->rbuf, sizeof(float) * 2 * (size_t)g->V));
-        GBX_CUDA(cudaMalloc(&c->cbuf, sizeof(float) * 2 * (size_t)g->V));
-        GBX_CUDA(cudaMalloc(&c->res, sizeof(gbx_pr_result)));
-        GBX_CUDA(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
+    if (!c) c = g->pr_cache = new gbx_pr_cache();
+    const size_t need = 2 * contrib_stride(g->V, l ? l->hot : 0);
+    if (!c->rbuf) GBX_CUDA(cudaMalloc(&c->rbuf, sizeof(float) * 2 * (size_t)g->V));
+    if (c->cbuf_n < need) {
+        c->drop_capture();
+        cudaFree(c->cbuf);
+        c->cbuf = nullptr;
+        c->cbuf_n = 0;
+        GBX_CUDA(cudaMalloc(&c->cbuf, sizeof(float) * need));
+        c->cbuf_n = need;
     }
     if (c->cap < std::max(max_it, 1u)) {
-        if (c->exec) cudaGraphExecDestroy(c->exec);
-        c->exec = nullptr;
-        cudaFree(c->st);
-        c->st = nullptr;
-        c->cap = std::max(max_it, 64u);
-        GBX_CUDA(cudaMalloc(&c->st, sizeof(PrIterState) * c->cap));
+        c->drop_capture();
+        cudaFree(c->tail);
+        c->tail = nullptr;
+        c->cap = 0;
+        const uint32_t cap = std::max(max_it, 64u);
+        GBX_CUDA(cudaMalloc(&c->tail, sizeof(*c->tail) + sizeof(PrIterState) * cap));
+        c->st = reinterpret_cast<PrIterState *>(c->tail + 1);
+        c->cap = cap;
+    }
+    if (!l) {
+        if (!c->cap_stream) GBX_CUDA(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
+    } else if (!c->row_degree) {
+        if (!c->sums) GBX_CUDA(cudaMalloc(&c->sums, sizeof(float) * 2 * (size_t)l->n_units));
+        if (!c->tickets) {
+            GBX_CUDA(cudaMalloc(&c->tickets, sizeof(unsigned) * (size_t)l->n_units));
+            GBX_CUDA(cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * (size_t)l->n_units, s));
+        }
+        GBX_CUDA(cudaMalloc(&c->row_degree, sizeof(uint32_t) * (size_t)l->n_rows));
+        pr_row_degree_kernel<<<std::min<unsigned>(ceil_div(l->n_rows, 256), (unsigned)num_sms() * 8), 256, 0, s>>>(
+            l->rows, l->n_rows, g->out_degree, c->row_degree);
+        GBX_LAUNCH_CHECK();
     }
     *out = c;
     return GBX_OK;
 }
 
-// (Re)capture the loop on the cache's own stream.
+// (Re)capture the row engine's loop on the cache's own stream.
 int pr_capture(gbx_graph *g, const gbx_gather_plan &plan, uint32_t max_it, double epsilon, gbx_pr_cache *c) {
     if (c->exec && c->key_it == max_it && c->key_eps == epsilon) return GBX_OK;
-    if (c->exec) cudaGraphExecDestroy(c->exec);
-    c->exec = nullptr;
+    c->drop_capture();
     GBX_CUDA(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal));
     uint32_t kernels = 0;
     const int st = pr_enqueue_loop(g, plan, max_it, epsilon, c->rbuf, c->cbuf, c->st, c->cap_stream, &kernels);
@@ -224,6 +383,25 @@ int pr_capture(gbx_graph *g, const gbx_gather_plan &plan, uint32_t max_it, doubl
     return GBX_OK;
 }
 
+// the persistent kernel over the hot-table layout
+int pr_run_hot(gbx_graph *g, const gbx_pull_layout &l, uint32_t max_it, double epsilon, gbx_pr_cache *c,
+               cudaStream_t s) {
+    const uint32_t V = g->V;
+    GBX_CUDA(cudaMemsetAsync(c->tail, 0, sizeof(*c->tail) + sizeof(PrIterState) * max_it, s));
+    const int grid = (int)std::min<uint64_t>((V + l.hot + 255ull) / 256, (uint64_t)num_sms() * 8);
+    pr_hot_init_kernel<<<grid, 256, 0, s>>>(c->rbuf, c->cbuf, g->out_degree, V, l.hot, l.hot_ids);
+    GBX_LAUNCH_CHECK();
+    PrHotArgs a{l, c->rbuf, c->cbuf, c->row_degree, c->st, {c->sums, c->tickets}, &c->tail->sync, max_it, epsilon};
+    const size_t smem = pull_smem(l);
+    GBX_CUDA(cudaFuncSetAttribute(pr_hot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // a CTA per SM, fewer where there is less than a unit per warp
+    const unsigned ctas = std::min<unsigned>((unsigned)num_sms(), ceil_div(l.n_units, kPullWarps));
+    void *args[] = {&a};
+    GBX_CUDA(cudaLaunchCooperativeKernel((const void *)pr_hot_kernel, dim3(ctas), dim3(kPullThreads), args, smem, s));
+    GBX_LAUNCH_CHECK();
+    return GBX_OK;
+}
+
 }  // namespace
 
 extern "C" int gbx_pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon,
@@ -234,25 +412,34 @@ extern "C" int gbx_pagerank_pull(gbx_graph *g, uint32_t max_iterations, double e
     GBX_TRY(ensure_device());
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t V = g->V;
+    gbx_pull_layout *layout = nullptr;
+    GBX_TRY(get_pull_layout(g, max_iterations, s, &layout));
+    if (max_iterations == 0) layout = nullptr;
     gbx_gather_plan *plan = nullptr;
-    GBX_TRY(get_pull_plan(g, s, &plan));
+    if (!layout) GBX_TRY(get_pull_plan(g, s, &plan));
     OutArray<float> out;
     GBX_TRY(out.bind(ranks, V, s));
     gbx_pr_cache *c = nullptr;
-    GBX_TRY(pr_cache(g, max_iterations, &c));
-    GBX_TRY(pr_capture(g, *plan, max_iterations, epsilon, c));
-    GBX_CUDA(cudaGraphLaunch(c->exec, s));
-    for (uint32_t k = 0; k < c->kernels; ++k) note_launch();
-    float *r[2] = {c->rbuf, c->rbuf + V};
+    GBX_TRY(pr_cache(g, layout, max_iterations, s, &c));
+    if (layout) {
+        GBX_TRY(pr_run_hot(g, *layout, max_iterations, epsilon, c, s));
+    } else {
+        GBX_TRY(pr_capture(g, *plan, max_iterations, epsilon, c));
+        GBX_CUDA(cudaGraphLaunch(c->exec, s));
+        for (uint32_t k = 0; k < c->kernels; ++k) note_launch();
+    }
     const int grid = (int)std::min<uint64_t>((V + 255) / 256, (uint64_t)num_sms() * 8);
-    gbx_pr_result *res = c->res;
-    pr_finish_kernel<<<grid, 256, 0, s>>>(r[0], r[1], c->st, max_iterations, epsilon > 0.0 ? 1u : 0u, V, out.d,
-                                          nullptr, res);
+    pr_finish_kernel<<<grid, 256, 0, s>>>(c->rbuf, c->rbuf + V, c->st, max_iterations, epsilon > 0.0 ? 1u : 0u, V,
+                                          out.d, nullptr, &c->tail->res);
     GBX_LAUNCH_CHECK();
     GBX_TRY(out.finish(s));
-    gbx_pr_result hres;
-    GBX_CUDA(cudaMemcpyAsync(&hres, res, sizeof(hres), cudaMemcpyDeviceToHost, s));
+    gbx_pr_cache::Tail h;
+    GBX_CUDA(cudaMemcpyAsync(&h, c->tail, sizeof(h), cudaMemcpyDeviceToHost, s));
     GBX_CUDA(cudaStreamSynchronize(s));
-    if (result) *result = hres;
+    if (layout && h.sync.error) {
+        GBX_CUDA(cudaMemset(c->tickets, 0, sizeof(unsigned) * (size_t)layout->n_units));  // a sweep was left half done
+        GBX_REQUIRE(false, GBX_ERR_DEVICE_TIMEOUT, "PageRank: a grid barrier wait ran out");
+    }
+    if (result) *result = h.res;
     return GBX_OK;
 }

@@ -1,8 +1,12 @@
 // SpMV pull (the reference's SPMVPullGraphCSR, SPMV.c:117-215):
 // y[v] += sum over pull edges (u->v) of w_uv * x[u], repeated `iterations`
 // times with y never reset. The pull engine (gbx_gather.cuh) computes each
-// row's sum (Kahan-compensated on medium and heavy rows) and adds it to y.
-#include "gbx_gather.cuh"
+// row's sum (Kahan-compensated on medium and heavy rows) and adds it to y;
+// from the fourth sweep of a graph on the hot-table engine (gbx_pull.cuh) does,
+// with the hot vertices' x gathered once per call.
+#include <algorithm>
+
+#include "gbx_pull.cuh"
 
 namespace gbx {
 
@@ -25,6 +29,81 @@ struct SpmvEpi {
     __device__ __forceinline__ void block_finish() {}
 };
 
+// ---- hot-table engine -----------------------------------------------------------
+
+struct SpmvHotTerm {
+    const float *__restrict__ val;  // may be null
+    float dflt;
+    const float *cold;  // x
+    bool wide;  // val starts on a 16-byte boundary
+    struct Factors {
+        float w[4];
+    };
+    __device__ __forceinline__ void factors(uint32_t e, uint32_t e0, uint32_t e1, Factors &f) const {
+        if (!val) {
+            f.w[0] = f.w[1] = f.w[2] = f.w[3] = dflt;
+        } else if (wide && e >= e0 && e + 4 <= e1) {
+            const float4 w = __ldcs(reinterpret_cast<const float4 *>(val + e));
+            f.w[0] = w.x, f.w[1] = w.y, f.w[2] = w.z, f.w[3] = w.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f.w[k] = e + k >= e0 && e + k < e1 ? __ldcs(val + e + k) : 0.f;
+        }
+    }
+    __device__ __forceinline__ void scale(const Factors &f, float (&v)[4]) const {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = __fmul_rn(f.w[k], v[k]);
+    }
+};
+
+struct SpmvHotEpi {
+    float *__restrict__ y;
+    __device__ __forceinline__ void prefetch(uint32_t) const {}
+    __device__ __forceinline__ void operator()(uint32_t, uint32_t v, uint32_t, float sum) const { y[v] = __fadd_rn(y[v], sum); }
+};
+
+__global__ void spmv_hot_values_kernel(const float *x, const uint32_t *hot_ids, uint32_t hot, uint32_t V, float *out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= hot) return;
+    const uint32_t v = hot_ids[i];
+    out[i] = v < V ? x[v] : 0.f;
+}
+
+__global__ void __launch_bounds__(kPullThreads, 1)
+    spmv_hot_kernel(gbx_pull_layout layout, const float *hot_x, SpmvHotTerm term, SpmvHotEpi epi, PullPieces pieces,
+                    unsigned *cursor) {
+    extern __shared__ __align__(16) float s_hot[];
+    PullSweep<SpmvHotTerm, SpmvHotEpi> sweep{layout, (uint32_t)__cvta_generic_to_shared(s_hot),
+                                             s_hot + layout.hot + 4 + (threadIdx.x >> 5) * kPullBuf, term, epi, pieces};
+    typename PullSweep<SpmvHotTerm, SpmvHotEpi>::Start first{};
+    if (first_unit() < layout.n_units) first = sweep.start(first_unit());
+    load_hot(hot_x, layout.hot, s_hot);
+    deal_units(sweep, cursor, first);
+}
+
+// Working memory is the call's own: calls on one graph may overlap.
+static int spmv_run_hot(const gbx_pull_layout &l, SpmvHotTerm term, float *y, uint32_t iterations, cudaStream_t s) {
+    DevBuf<float> hot_x, sums;
+    DevBuf<unsigned> tickets;  // then one cursor per iteration
+    GBX_TRY(hot_x.alloc(std::max(l.hot, 4u), s));
+    GBX_TRY(sums.alloc(2 * (size_t)l.n_units, s));
+    GBX_TRY(tickets.alloc((size_t)l.n_units + iterations, s));
+    GBX_CUDA(cudaMemsetAsync(tickets.p, 0, ((size_t)l.n_units + iterations) * sizeof(unsigned), s));
+    if (l.hot) {
+        spmv_hot_values_kernel<<<ceil_div(l.hot, 256), 256, 0, s>>>(term.cold, l.hot_ids, l.hot, l.V, hot_x.p);
+        GBX_LAUNCH_CHECK();
+    }
+    const size_t smem = pull_smem(l);
+    GBX_CUDA(cudaFuncSetAttribute(spmv_hot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned ctas = std::min<unsigned>((unsigned)num_sms(), ceil_div(l.n_units, kPullWarps));
+    for (uint32_t it = 0; it < iterations; ++it) {
+        spmv_hot_kernel<<<ctas, kPullThreads, smem, s>>>(l, hot_x.p, term, SpmvHotEpi{y},
+                                                         PullPieces{sums.p, tickets.p}, tickets.p + l.n_units + it);
+        GBX_LAUNCH_CHECK();
+    }
+    return GBX_OK;
+}
+
 }  // namespace gbx
 
 using namespace gbx;
@@ -36,8 +115,10 @@ extern "C" int gbx_spmv(gbx_graph *g, const float *values, float default_value, 
     GBX_TRY(ensure_device());
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t V = g->V;
+    gbx_pull_layout *layout = nullptr;
+    GBX_TRY(get_pull_layout(g, iterations, s, &layout));
     gbx_gather_plan *plan = nullptr;
-    GBX_TRY(get_pull_plan(g, s, &plan));
+    if (!layout) GBX_TRY(get_pull_plan(g, s, &plan));
     InArray<float> xin, vin;
     GBX_TRY(xin.bind(x, V, s));
     const float *vals = nullptr;
@@ -51,10 +132,15 @@ extern "C" int gbx_spmv(gbx_graph *g, const float *values, float default_value, 
     OutArray<float> yout;
     GBX_TRY(yout.bind(y, V, s));
     if (yout.to_host()) GBX_CUDA(cudaMemcpyAsync(yout.d, y, (size_t)V * 4, cudaMemcpyHostToDevice, s));
-    SpmvTerm term{g->pull_src(), vals, default_value, xin.d};
-    SpmvEpi epi{yout.d};
-    for (uint32_t it = 0; it < iterations; ++it)
-        GBX_TRY(launch_gather(g->pull_offsets(), V, *plan, term, epi, s));
+    if (layout) {
+        const bool wide = ((uintptr_t)vals & 15u) == 0;
+        GBX_TRY(spmv_run_hot(*layout, SpmvHotTerm{vals, default_value, xin.d, wide}, yout.d, iterations, s));
+    } else {
+        SpmvTerm term{g->pull_src(), vals, default_value, xin.d};
+        SpmvEpi epi{yout.d};
+        for (uint32_t it = 0; it < iterations; ++it)
+            GBX_TRY(launch_gather(g->pull_offsets(), V, *plan, term, epi, s));
+    }
     GBX_TRY(yout.finish(s));
     if (yout.to_host()) GBX_CUDA(cudaStreamSynchronize(s));
     return GBX_OK;

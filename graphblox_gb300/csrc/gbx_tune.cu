@@ -170,7 +170,21 @@ extern "C" int gbx_autotune(gbx_graph *g, uint32_t flags, uint32_t num_samples, 
         g->sssp_delta = best_d;
     }
     if (flags & 4u) {
-        // pull-engine row classes, timed on pull PageRank iterations
+        // row classes of the row engine, timed on pull PageRank iterations
+        // with the hot-table engine (which has none) held off
+        struct RowsOnly {
+            gbx_graph *g;
+            gbx_pull_layout *layout;
+            uint32_t tries;
+            explicit RowsOnly(gbx_graph *gr) : g(gr), layout(gr->pull_layout), tries(gr->pull_layout_tries) {
+                g->pull_layout = nullptr;
+                g->pull_layout_tries = ~0u;
+            }
+            ~RowsOnly() {
+                g->pull_layout = layout;
+                g->pull_layout_tries = tries;
+            }
+        } rows_only(g);
         const uint32_t cands[] = {1024, 4096, 16384};
         DevBuf<float> ranks;
         GBX_TRY(ranks.alloc(g->V, s));
@@ -178,7 +192,7 @@ extern "C" int gbx_autotune(gbx_graph *g, uint32_t flags, uint32_t num_samples, 
         uint32_t best_h = g->pull_heavy_min;
         for (uint32_t c : cands) {
             GBX_TRY(gbx_graph_set_tuning(g, "pull_heavy_min", c));
-            GBX_TRY(gbx_pagerank_pull(g, 5, 0.0, ranks.p, nullptr, stream));  // builds the plan, captures
+            GBX_TRY(gbx_pagerank_pull(g, 5, 0.0, ranks.p, nullptr, stream));  // builds the plan
             float ms = 0.f;
             GBX_TRY(time_ms([&]() { return gbx_pagerank_pull(g, 5, 0.0, ranks.p, nullptr, stream); }, s, &ms));
             if (trace_enabled()) fprintf(stderr, "| autotune pull_heavy_min %-5u | %9.3f ms |\n", c, ms);

@@ -119,7 +119,8 @@ int gbx_graph_device_arrays(const gbx_graph *g, const uint32_t **offsets, const 
  * exceed unexplored edges / alpha; the reference fixes 15), "bfs_beta" (stay
  * bottom-up while the frontier exceeds V / beta; 18), "sssp_delta" (bucket
  * width, 0 = default), "pull_heavy_min" (in-degree above which PR/SpMV cut a
- * row into CTA-sized chunks; 4096). SSSP distances never change; PR and SpMV
+ * row into CTA-sized chunks; 4096; sweeps of small graphs and a graph's first
+ * three only: later ones are cut by edges). SSSP distances never change; PR and SpMV
  * sums may change their FP32 summation order only. BFS results do not depend
  * on alpha/beta when the graph has an inverse CSR or is symmetric; without an
  * inverse CSR the reference pulls over out-edges, and on an asymmetric graph
