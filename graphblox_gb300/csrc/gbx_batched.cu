@@ -17,12 +17,12 @@
 //        frontier vertices per warp; bottom-up gives each warp 32 unvisited
 //        vertices, one lane each, scanning in-edges until a frontier parent.
 //   PR:  contributions (4V bytes) in shared memory; the gather streams the
-//        graph's in-edge ids from global memory and reads contributions from
-//        shared memory. Rows above 32 in-edges are summed by the whole warp
-//        with per-lane Kahan compensation.
+//        graph's in-edges as words (a batch's first PageRank call lays them
+//        out) and reads contributions from shared memory.
 // Graphs too large for the shared-memory capacity use the same code on a
 // per-CTA global scratch slot.
 #include <algorithm>
+#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -39,6 +39,15 @@ struct gbx_batch {
     uint32_t *in_src = nullptr;      // E or null
     uint32_t *order = nullptr;       // G, graph ids by descending edge count
     std::vector<uint32_t> h_vbase;   // host copy of vbase
+    std::vector<uint32_t> h_edges;   // edges per graph
+    // PageRank's in-edge words (built by its first call): graph g's start
+    // wbase[g] units of 16 bytes into words, its rows with edges at rows + vbase[g]
+    uint4 *words = nullptr;
+    uint32_t *wbase = nullptr;       // G
+    uint2 *rows = nullptr;           // V: {vertex, out-degree}
+    // G * 33: where each warp's part begins: {edge, row | top bit: it began earlier}
+    uint2 *starts = nullptr;
+    std::mutex words_mutex;
     const uint32_t *poff() const { return in_offsets ? in_offsets : offsets; }
     const uint32_t *psrc() const { return in_offsets ? in_src : dest; }
 };
@@ -50,7 +59,9 @@ constexpr int kBbWarps = kBbThreads / 32;
 constexpr uint32_t kBbWordsCap = 4096;  // bitmap words in shared memory: V <= 131072
 constexpr int kBpThreads = 1024;
 constexpr int kBpWarps = kBpThreads / 32;
-constexpr uint32_t kBpSmemV = 49152;  // contributions in shared memory: V <= 49152 (192 KiB)
+constexpr uint32_t kBpSmemV = 46976;   // contributions in shared memory (188 KB), a multiple of 32
+constexpr uint32_t kBpShortV = 32768;  // ids that leave a 16-bit word's top bit free
+constexpr uint32_t kBpBuf = 288;       // pending row sums of a warp: fewer than 32, and a group's 256
 
 __device__ __forceinline__ uint32_t bb_next_graph(uint32_t *cursor, uint32_t G, const uint32_t *order,
                                                   uint32_t *s_slot) {
@@ -265,25 +276,40 @@ __global__ void __launch_bounds__(kBbThreads, 2) bfs_batched_kernel(BbArgs a) {
 }
 
 // ---- PageRank --------------------------------------------------------------------
+// A graph's in-edges are a stream of words in row order: the source's id and,
+// in the top bit, whether the edge is its row's last; 16 bits each for graphs
+// of up to 32,768 vertices, else 32. The CTA's 32 warps take equal parts of
+// the stream, 256 edges at a time, eight consecutive ones per lane: a lane adds
+// up its row pieces and a segmented scan joins them across the warp, so no
+// row is too long or too short for its lane and no offsets are read. Row sums
+// collect in shared memory and leave 32 at a time through the epilogue, which
+// writes the vertex's next contribution. A row cut by a part's end leaves
+// pieces that one warp joins after the barrier. Every order of additions is
+// fixed: ranks repeat bit for bit.
+//
+// Bound: the shared-memory pipe (65%: a gather of 32 random words takes 3 to 4
+// cycles, and scans' shuffles go the same way) and the issue slots (65%: 190
+// instructions per 256 edges). 2,048 graphs, 30 iterations, 6.5G edge visits:
+// 7.9 ms; 11.0 without spreading the banks and with a scan per group of a long
+// row, 9.1 with equal edges per warp. Rows taken one per lane or one per warp,
+// ids in 32 bits: 20.9 ms.
 struct BpArgs {
     uint32_t G;
-    const uint32_t *vbase, *off, *poff, *psrc, *order;
-    float *ranks;    // output, also one rank buffer
-    float *rother;   // second rank buffer (V)
-    float *scratch;  // per CTA contributions for graphs above kBpSmemV
-    uint32_t scratch_v;
+    const uint32_t *vbase, *off, *poff, *order;
+    const uint4 *words;
+    const uint32_t *wbase;
+    const uint2 *starts, *rows;
+    float *ranks;       // output, also one rank buffer
+    float *rother;      // second rank buffer (V)
+    float *next;        // per CTA: next contributions where two buffers do not fit shared memory
+    float *scratch;     // per CTA: contributions of graphs above kBpSmemV
+    uint32_t max_v;     // floats per CTA in next and scratch
+    uint32_t smem_v;    // floats of contributions in shared memory
     uint32_t *cursor;
     uint32_t max_it;
     double epsilon;
     gbx_pr_result *res;
 };
-
-// Shared memory of one PageRank CTA (dynamic): contributions, then the
-// partial sums of heavy-row pieces, then the heavy-row table.
-constexpr uint32_t kBpHeavyMax = 1024;                // heavy rows per graph
-constexpr uint32_t kBpSlots = 4096 + kBpHeavyMax;     // piece partials
-constexpr uint32_t kBpHeavyMin = 512;                 // in-degree above which a row is split
-constexpr size_t kBpSmemBytes = (size_t)kBpSmemV * 4 + (size_t)kBpSlots * 4 + (size_t)(2 * kBpHeavyMax + 1) * 4;
 
 __device__ __forceinline__ void kahan_add(float &sum, float &comp, float x) {
     const float y = __fsub_rn(x, comp);
@@ -292,235 +318,290 @@ __device__ __forceinline__ void kahan_add(float &sum, float &comp, float x) {
     sum = t;
 }
 
-// Exclusive scan of one value per thread over the block (blockDim.x = kBpThreads);
-// returns the thread's prefix, *total the sum. Uses s_tmp[32].
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t *s_tmp, uint32_t *total) {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = x;
+// A warp's part of a graph's word stream: whole groups of 256 edges, with an
+// equal share of the cost; a row costs about as much as this many edges (its
+// sum and epilogue against a group's 150 instructions).
+constexpr uint32_t kBpRowCost = 4;
+constexpr uint32_t kBpStarts = kBpWarps + 1;
+
+// inclusive segmented scan over the warp: lane's value added to those below it
+// down to the nearest lane (itself included) that starts a segment
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+template <class T>
+__device__ __forceinline__ T segmented_scan(T x, bool starts) {
+    const uint32_t lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(0xffffffffu, starts) & (0xffffffffu >> (31 - lane));
+    const uint32_t back = m ? lane - (31u - __clz(m)) : lane;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= (uint32_t)o) incl += t;
+        const T t = __shfl_up_sync(0xffffffffu, x, o);
+        if ((uint32_t)o <= back) x = add_rn(x, t);
     }
-    __syncthreads();
-    if (lane == 31) s_tmp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kBpWarps ? s_tmp[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, w, o);
-            if (lane >= (uint32_t)o) w += t;
-        }
-        s_tmp[lane] = w;  // inclusive warp totals
-    }
-    __syncthreads();
-    const uint32_t before = warp ? s_tmp[warp - 1] : 0u;
-    *total = s_tmp[kBpWarps - 1];
-    return before + incl - x;
+    return x;
 }
 
-// Rows of one graph, per iteration, as tasks dealt to warps by a
-// shared-memory counter (so a slow task does not hold a fixed share):
-//   pieces  kBpHeavyMin..-edge slices of the heavy rows (in-degree > T); a
-//           warp sums one with per-lane Kahan and a warp reduction, and the
-//           partial goes to its slot;
-//   units   32 consecutive rows: light rows (<= 32 in-edges) one lane each,
-//           four index loads in flight, medium rows by the whole warp with
-//           per-lane Kahan; heavy rows are skipped here.
-// After the barrier one thread per heavy row adds its pieces' partials in
-// piece order. Every sum has a fixed order, so ranks are deterministic.
+// bank-spreading place of a contribution inside its 32 vertices: R-MAT ids have
+// few one bits, and a quarter of the edges would meet in bank 0
+__host__ __device__ __forceinline__ uint32_t bp_place(uint32_t v) { return v ^ (((v >> 5) ^ (v >> 10)) & 31u); }
+
+struct BpRow {  // one row's epilogue
+    float *rc, *rn, *c_next;
+    double epsilon, inv_n;
+    bool write, reduce;
+    double err;
+    uint32_t active;
+    __device__ __forceinline__ void operator()(uint2 row, float sum) {
+        const float next = __fadd_rn(1.0f - 0.85f, __fmul_rn(0.85f, sum));
+        if (row.y) c_next[bp_place(row.x)] = __fdiv_rn(next, (float)row.y);
+        if (write) {
+            if (reduce) {
+                const double d = (double)fabsf(__fsub_rn(next, rc[row.x]));
+                err += d * inv_n;
+                active += d >= epsilon ? 1u : 0u;
+            }
+            rn[row.x] = next;
+        }
+    }
+};
+
+// Shared memory of the parts' ends: a row begun in an earlier part and ended
+// here leaves its piece in head; what follows the part's last row end (or the
+// whole part) in tail. Pieces of the largest rows meet here: joined in 64 bits,
+// the sum is rounded once.
+struct BpEnds {
+    double head[kBpWarps], tail[kBpWarps];
+    uint32_t has_end[kBpWarps];
+};
+
+// This warp's part of one sweep. kShort: 16-bit words.
+//
+// The open row -- the one whose end is not reached yet -- is held as `carry`
+// (its edges in the group where it began) and, for groups without any row end,
+// a compensated sum per lane; a long row therefore costs no scan until its
+// end, where the lanes are joined in 64 bits. What decides when an iteration
+// stops is the ranks of the largest rows: their sums are rounded once.
+template <bool kShort>
+__device__ __forceinline__ void bp_sweep(const uint4 *words, uint2 start, uint32_t e1, const uint2 *rows, const float *c,
+                                         float *buf, BpEnds &ends_of, BpRow &epi) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    const uint32_t e0 = start.x;
+    uint32_t row = start.y & 0x7FFFFFFFu, pending = 0;
+    bool cut = start.y >> 31, any = false, spread = false;  // spread: the lanes hold some of the open row
+    float carry = 0.f, ls = 0.f, lc = 0.f;
+    constexpr uint32_t kPerLane = kShort ? 1 : 2;  // 16-byte loads per group
+    const uint4 *w = words + (size_t)(e0 / 8 + lane) * kPerLane;
+    uint4 ahead[kPerLane];
+    if (e0 < e1) {
+#pragma unroll
+        for (uint32_t i = 0; i < kPerLane; ++i) ahead[i] = __ldcs(w + i);
+    }
+    for (uint32_t at = e0; at < e1; at += 256) {
+        uint32_t id[8], ends;
+        if constexpr (kShort) {
+            const uint4 x = ahead[0];
+            id[0] = x.x & 0x7FFFu, id[1] = (x.x >> 16) & 0x7FFFu;
+            id[2] = x.y & 0x7FFFu, id[3] = (x.y >> 16) & 0x7FFFu;
+            id[4] = x.z & 0x7FFFu, id[5] = (x.z >> 16) & 0x7FFFu;
+            id[6] = x.w & 0x7FFFu, id[7] = (x.w >> 16) & 0x7FFFu;
+            // flags of word i to bits 2i and 2i + 16, the upper ones then down to 2i + 1
+            const uint32_t f = ((x.x & 0x80008000u) >> 15) | ((x.y & 0x80008000u) >> 13) |
+                               ((x.z & 0x80008000u) >> 11) | ((x.w & 0x80008000u) >> 9);
+            ends = (f | (f >> 15)) & 0xFFu;
+        } else {
+            const uint4 x = ahead[0], y = ahead[kPerLane - 1];
+            const uint32_t z[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+            ends = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                id[k] = z[k] & 0x7FFFFFFFu;
+                ends |= (z[k] >> 31) << k;
+            }
+        }
+        w += 32 * kPerLane;
+        const uint32_t left = e1 - at;
+        if (left > 256) {
+#pragma unroll
+            for (uint32_t i = 0; i < kPerLane; ++i) ahead[i] = __ldcs(w + i);
+        }
+        float x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = c[id[k]];
+        if (left < 256) {  // words past the stream's end are vertex 0 without a row end
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (lane * 8 + k >= left) x[k] = 0.f;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, ends != 0);
+        if (m == 0) {
+            float acc = x[0];
+#pragma unroll
+            for (int k = 1; k < 8; ++k) acc = __fadd_rn(acc, x[k]);
+            kahan_add(ls, lc, acc);
+            spread = true;
+            continue;
+        }
+        // where this lane's row sums go
+        const uint32_t mine = __popc(ends);
+        uint32_t upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= (uint32_t)o) upto += t;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, upto, 31);
+        float *out = buf + pending + upto - mine;
+        float *const first_out = out;
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            acc = __fadd_rn(acc, x[k]);
+            if ((ends >> k) & 1u) {
+                *out++ = acc;
+                acc = 0.f;
+            }
+        }
+        const float scan = segmented_scan(acc, ends != 0);
+        float in = __shfl_up_sync(0xffffffffu, scan, 1);
+        if (lane == 0) in = 0.f;
+        double open = 0.0;  // the open row's earlier groups
+        if (spread) open = warp_sum((double)ls - (double)lc);
+        if (ends) {
+            const float sum = __fadd_rn(in, *first_out);
+            if (m & lt) {
+                *first_out = sum;
+            } else if (spread || cut) {
+                const double whole = open + (double)carry + (double)in + (double)*first_out;
+                *first_out = __double2float_rn(whole);
+                if (cut) ends_of.head[warp] = whole;
+            } else {
+                *first_out = __fadd_rn(sum, carry);
+            }
+        }
+        carry = __shfl_sync(0xffffffffu, scan, 31);
+        ls = lc = 0.f;
+        spread = false;
+        any = true;
+        __syncwarp();
+        pending += total;
+        uint32_t first = cut;
+        row += first;
+        cut = false;
+        for (; pending - first >= 32; first += 32, row += 32) epi(__ldg(rows + row + lane), buf[first + lane]);
+        if (first) {
+            pending -= first;
+            const float t = lane < pending ? buf[first + lane] : 0.f;
+            __syncwarp();
+            if (lane < pending) buf[lane] = t;
+        }
+        __syncwarp();
+    }
+    if (lane < pending) epi(__ldg(rows + row + lane), buf[lane]);
+    double tail = (double)carry;
+    if (spread) tail += warp_sum((double)ls - (double)lc);
+    if (lane == 0) {
+        ends_of.tail[warp] = tail;
+        ends_of.has_end[warp] = any;
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(kBpThreads, 1) pr_batched_kernel(BpArgs a) {
-    extern __shared__ float s_mem[];
-    float *s_contrib = s_mem;
-    float *s_part = s_mem + kBpSmemV;
-    uint32_t *s_hrow = reinterpret_cast<uint32_t *>(s_part + kBpSlots);
-    uint32_t *s_hfirst = s_hrow + kBpHeavyMax;
-    __shared__ uint32_t s_slot, s_active, s_task, s_cnt, s_tmp[32];
-    __shared__ unsigned long long s_hedges;
+    extern __shared__ __align__(16) float s_mem[];  // contributions [smem_v], pending row sums
+    __shared__ BpEnds s_ends;
+    __shared__ uint32_t s_slot, s_active;
     __shared__ double s_err;
-    const uint32_t lane = threadIdx.x & 31;
-    const float damp = 0.85f;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *buf = s_mem + a.smem_v + warp * kBpBuf;
     const float base = 1.0f - 0.85f;
     const bool can_stop = a.epsilon > 0.0;
     for (;;) {
         const uint32_t g = bb_next_graph(a.cursor, a.G, a.order, &s_slot);
         if (g == 0xFFFFFFFFu) break;
         const uint32_t vb = a.vbase[g], Vg = a.vbase[g + 1] - vb;
-        float *contrib = Vg <= kBpSmemV ? s_contrib : a.scratch + (size_t)blockIdx.x * a.scratch_v;
         const uint32_t *off = a.off + vb;
-        const uint32_t *poff = a.poff + vb;
+        const uint4 *words = a.words + a.wbase[g];
+        const uint2 *rows = a.rows + vb;
+        const uint2 start = a.starts[g * kBpStarts + warp];
+        const uint32_t stop = a.starts[g * kBpStarts + warp + 1].x;
+        // lane i of warp 0 finishes the row that the end of part i - 1 cuts
+        const uint32_t part = a.starts[g * kBpStarts + lane].y;
+        const uint2 part_row = part >> 31 ? rows[part & 0x7FFFFFFFu] : make_uint2(0u, 0u);
+        // contributions: two buffers in shared memory, or one there and the
+        // next ones in global memory, or both in global memory
+        const uint32_t room = (Vg + 31) & ~31u;
+        const bool in_smem = room <= a.smem_v, both = 2 * room <= a.smem_v;
+        float *c = in_smem ? s_mem : a.scratch + (size_t)blockIdx.x * a.max_v;
+        float *cn = both ? s_mem + room : a.next + (size_t)blockIdx.x * a.max_v;
+        uint32_t cur = 0;  // c within s_mem, where it is there
         float *rc = a.ranks + vb, *rn = a.rother + vb;
-        const double inv_n = 1.0 / (double)Vg;
-        // heavy rows: the smallest threshold T >= kBpHeavyMin with at most
-        // kBpHeavyMax rows above it
-        uint32_t T = kBpHeavyMin;
-        for (;;) {
-            if (threadIdx.x == 0) {
-                s_cnt = 0;
-                s_hedges = 0;
-            }
-            __syncthreads();
-            uint32_t c = 0;
-            unsigned long long he = 0;
-            for (uint32_t v = threadIdx.x; v < Vg; v += blockDim.x) {
-                const uint32_t d = poff[v + 1] - poff[v];
-                if (d > T) {
-                    ++c;
-                    he += d;
-                }
-            }
-            c = warp_sum(c);
-            he = warp_sum(he);
-            if (lane == 0 && c) {
-                atomicAdd(&s_cnt, c);
-                atomicAdd(&s_hedges, he);
-            }
-            __syncthreads();
-            if (s_cnt <= kBpHeavyMax) break;
-            T *= 2;
-            __syncthreads();
-        }
-        const uint32_t nh = s_cnt;
-        // piece length: a multiple of 32 that keeps the pieces within the slots
-        const unsigned long long want = (s_hedges + (kBpSlots - kBpHeavyMax) - 1) / (kBpSlots - kBpHeavyMax);
-        const uint32_t P = (uint32_t)max(512ull, (want + 31) / 32 * 32);
-        __syncthreads();
-        if (threadIdx.x == 0) s_cnt = 0;
-        __syncthreads();
-        for (uint32_t v = threadIdx.x; v < Vg; v += blockDim.x)
-            if (poff[v + 1] - poff[v] > T) s_hrow[atomicAdd(&s_cnt, 1u)] = v;
-        __syncthreads();
-        uint32_t np = 0;
-        if (threadIdx.x < nh) {
-            const uint32_t h = s_hrow[threadIdx.x];
-            np = (poff[h + 1] - poff[h] + P - 1) / P;
-        }
-        uint32_t n_pieces = 0;
-        const uint32_t first = block_exclusive_scan(np, s_tmp, &n_pieces);
-        if (threadIdx.x < nh) s_hfirst[threadIdx.x] = first;
-        if (threadIdx.x == 0) s_hfirst[nh] = n_pieces;
         for (uint32_t v = threadIdx.x; v < Vg; v += blockDim.x) {
-            rc[v] = base;
+            rc[v] = rn[v] = base;  // rows without in-edges keep it
             const uint32_t d = off[v + 1] - off[v];
-            contrib[v] = d ? __fdiv_rn(base, (float)d) : 0.0f;
+            c[bp_place(v)] = cn[bp_place(v)] = d ? __fdiv_rn(base, (float)d) : 0.0f;
         }
         if (threadIdx.x == 0) {
             s_active = 0;
             s_err = 0.0;
-            s_task = 0;
         }
         __syncthreads();
-        const uint32_t units = (Vg + 31) / 32;
-        const uint32_t n_tasks = n_pieces + units;
         uint32_t k = a.max_it, executed = 0, active_last = 0;
         double err_last = 0.0;
         for (uint32_t it = 0; it < a.max_it; ++it) {
+            // with epsilon = 0 only the last iteration's residual is asked
+            // for, and ranks are written in the last two
             const bool reduce = can_stop || it + 1 == a.max_it;
-            double err = 0.0;
-            uint32_t active = 0;
-            for (;;) {
-                uint32_t t = 0;
-                if (lane == 0) t = atomicAdd(&s_task, 1u);
-                t = __shfl_sync(0xFFFFFFFFu, t, 0);
-                if (t >= n_tasks) break;
-                if (t < n_pieces) {
-                    uint32_t lo = 0, hi = nh - 1;  // last heavy row with first piece <= t
-                    while (lo < hi) {
-                        const uint32_t mid = (lo + hi + 1) >> 1;
-                        if (s_hfirst[mid] <= t) lo = mid; else hi = mid - 1;
-                    }
-                    const uint32_t h = s_hrow[lo];
-                    const uint32_t pb = poff[h] + (t - s_hfirst[lo]) * P;
-                    const uint32_t pe = min(pb + P, poff[h + 1]);
-                    float s = 0.f, c = 0.f;
-                    for (uint32_t j = pb + lane; j < pe; j += 32) kahan_add(s, c, contrib[__ldg(a.psrc + j)]);
-                    s = warp_sum(s);
-                    if (lane == 0) s_part[t] = s;
-                    continue;
-                }
-                const uint32_t v = (t - n_pieces) * 32 + lane;
-                const bool ok = v < Vg;
-                const uint32_t b = ok ? poff[v] : 0, e = ok ? poff[v + 1] : 0;
-                const uint32_t d = e - b;
-                float sum = 0.f;
-                if (d <= 32) {
-                    uint32_t j = b;
-                    for (; j + 4 <= e; j += 4) {
-                        const uint32_t u0 = __ldg(a.psrc + j), u1 = __ldg(a.psrc + j + 1);
-                        const uint32_t u2 = __ldg(a.psrc + j + 2), u3 = __ldg(a.psrc + j + 3);
-                        const float x0 = contrib[u0], x1 = contrib[u1], x2 = contrib[u2], x3 = contrib[u3];
-                        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, x0), x1), x2), x3);
-                    }
-                    for (; j < e; ++j) sum = __fadd_rn(sum, contrib[__ldg(a.psrc + j)]);
-                }
-                uint32_t mv = __ballot_sync(0xFFFFFFFFu, d > 32 && d <= T);
-                while (mv) {
-                    const uint32_t kk = __ffs(mv) - 1;
-                    mv &= mv - 1;
-                    const uint32_t hb = __shfl_sync(0xFFFFFFFFu, b, kk), hd = __shfl_sync(0xFFFFFFFFu, e, kk);
-                    float s = 0.f, c = 0.f;
-                    for (uint32_t j = hb + lane; j < hd; j += 32) kahan_add(s, c, contrib[__ldg(a.psrc + j)]);
-                    s = warp_sum(s);
-                    if (lane == kk) sum = s;
-                }
-                if (ok && d <= T) {
-                    const float next = __fadd_rn(base, __fmul_rn(damp, sum));
-                    const float prev = rc[v];
-                    rn[v] = next;
-                    if (reduce) {
-                        const double dd = (double)fabsf(__fsub_rn(next, prev));
-                        err += dd * inv_n;
-                        active += dd >= a.epsilon ? 1u : 0u;
-                    }
-                }
-            }
+            BpRow epi{rc, rn, cn, a.epsilon, 1.0 / (double)Vg, reduce || it + 2 == a.max_it, reduce, 0.0, 0u};
+            if (in_smem && Vg <= kBpShortV)
+                bp_sweep<true>(words, start, stop, rows, s_mem + cur, buf, s_ends, epi);
+            else if (in_smem)
+                bp_sweep<false>(words, start, stop, rows, s_mem + cur, buf, s_ends, epi);
+            else
+                bp_sweep<false>(words, start, stop, rows, c, buf, s_ends, epi);
             __syncthreads();
-            // heavy rows: pieces in order
-            if (threadIdx.x < nh) {
-                const uint32_t h = s_hrow[threadIdx.x];
-                float s = 0.f, c = 0.f;
-                for (uint32_t p = s_hfirst[threadIdx.x]; p < s_hfirst[threadIdx.x + 1]; ++p) kahan_add(s, c, s_part[p]);
-                const float next = __fadd_rn(base, __fmul_rn(damp, s));
-                const float prev = rc[h];
-                rn[h] = next;
-                if (reduce) {
-                    const double dd = (double)fabsf(__fsub_rn(next, prev));
-                    err += dd * inv_n;
-                    active += dd >= a.epsilon ? 1u : 0u;
-                }
+            if (warp == 0) {  // rows cut by a part's end
+                const bool cut = part >> 31, ended = s_ends.has_end[lane];
+                const double scan = segmented_scan(s_ends.tail[lane], ended || !cut);
+                const double in = __shfl_up_sync(0xffffffffu, scan, 1);
+                if (cut && ended)
+                    epi(part_row, __double2float_rn(in + s_ends.head[lane]));
             }
             if (reduce) {
-                err = warp_sum(err);
-                active = warp_sum(active);
+                const double err = warp_sum(epi.err);
+                const uint32_t active = warp_sum(epi.active);
                 if (lane == 0) {
                     atomicAdd(&s_err, err);
                     atomicAdd(&s_active, active);
                 }
             }
             __syncthreads();
-            // next contributions from the new ranks (shared memory is rewritten only now)
-            for (uint32_t v = threadIdx.x; v < Vg; v += blockDim.x) {
-                const uint32_t d = off[v + 1] - off[v];
-                contrib[v] = d ? __fdiv_rn(rn[v], (float)d) : 0.0f;
-            }
-            const uint32_t act = s_active;
-            const double er = s_err;
-            if (threadIdx.x == 0) s_task = 0;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                s_active = 0;
-                s_err = 0.0;
+            if (both || !in_smem) {
+                float *t = c;
+                c = cn;
+                cn = t;
+                cur = room - cur;
+            } else {
+                for (uint32_t i = threadIdx.x; i < room / 4; i += blockDim.x)
+                    reinterpret_cast<float4 *>(c)[i] = reinterpret_cast<const float4 *>(cn)[i];
             }
             float *t = rc;
             rc = rn;
             rn = t;
             executed = it + 1;
-            active_last = can_stop ? act : Vg;
-            err_last = er;
-            if (can_stop && act == 0) {
-                k = it;
-                break;
+            if (!both && in_smem) __syncthreads();  // the copy
+            if (reduce) {
+                active_last = can_stop ? s_active : Vg;
+                err_last = s_err;
+                __syncthreads();
+                if (can_stop && active_last == 0) {
+                    k = it;
+                    break;
+                }
+                if (threadIdx.x == 0) {
+                    s_active = 0;
+                    s_err = 0.0;
+                }
+                __syncthreads();
             }
         }
         // final ranks / N into the output buffer
@@ -534,6 +615,76 @@ __global__ void __launch_bounds__(kBpThreads, 1) pr_batched_kernel(BpArgs a) {
             r.error_total = executed ? err_last : 0.0;
             a.res[g] = r;
         }
+    }
+}
+
+// One CTA lays a graph's words out.
+__global__ void __launch_bounds__(kBpThreads)
+    bp_layout_kernel(uint32_t G, const uint32_t *order, const uint32_t *vbase, const uint32_t *off, const uint32_t *poff, const uint32_t *psrc,
+                     const uint32_t *wbase, uint32_t smem_v, uint4 *words, uint2 *rows, uint2 *starts) {
+    __shared__ uint32_t s_wsum[kBpWarps], s_base;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint32_t i = blockIdx.x; i < G; i += gridDim.x) {
+        const uint32_t g = order[i];
+        const uint32_t vb = vbase[g], Vg = vbase[g + 1] - vb;
+        const uint32_t *po = poff + vb;
+        const uint32_t first = po[0], edges = po[Vg] - first;
+        const bool is_short = Vg <= kBpShortV && ((Vg + 31) & ~31u) <= smem_v;
+        uint16_t *w16 = reinterpret_cast<uint16_t *>(words + wbase[g]);
+        uint32_t *w32 = reinterpret_cast<uint32_t *>(words + wbase[g]);
+        if (threadIdx.x == 0) s_base = 0;
+        __syncthreads();
+        // rows with edges, in order
+        for (uint32_t v0 = 0; v0 < Vg; v0 += kBpThreads) {
+            const uint32_t v = v0 + threadIdx.x;
+            const bool has = v < Vg && po[v + 1] != po[v];
+            const unsigned b = __ballot_sync(0xffffffffu, has);
+            if (lane == 0) s_wsum[warp] = __popc(b);
+            __syncthreads();
+            uint32_t p = s_base + __popc(b & ((1u << lane) - 1u));
+            for (uint32_t w = 0; w < warp; ++w) p += s_wsum[w];
+            if (has) rows[vb + p] = make_uint2(v, off[vb + v + 1] - off[vb + v]);
+            __syncthreads();
+            if (threadIdx.x == kBpThreads - 1) s_base = p + has;
+            __syncthreads();
+        }
+        const uint32_t rows_g = s_base;
+        // words (the stream is padded to whole groups with vertex 0)
+        for (uint32_t e = threadIdx.x; e < (edges + 255) / 256 * 256; e += kBpThreads) {
+            const uint32_t u = e < edges ? bp_place(psrc[first + e]) : 0u;
+            if (is_short) w16[e] = (uint16_t)u; else w32[e] = u;
+        }
+        __syncthreads();
+        for (uint32_t v = threadIdx.x; v < Vg; v += kBpThreads) {
+            if (po[v + 1] == po[v]) continue;
+            const uint32_t e = po[v + 1] - 1 - first;
+            if (is_short) w16[e] |= 0x8000u; else w32[e] |= 0x80000000u;
+        }
+        // the parts' first edges: part k begins at the first group with at
+        // least k / 32 of the cost before it
+        const uint32_t groups = (edges + 255) / 256;
+        const uint64_t total = (uint64_t)edges + (uint64_t)kBpRowCost * rows_g;
+        auto row_at = [&](uint32_t e) {  // the last row that begins at or before e
+            uint32_t lo = 0, hi = rows_g;
+            while (hi - lo > 1) {
+                const uint32_t mid = lo + (hi - lo) / 2;
+                if (po[rows[vb + mid].x] - first <= e) lo = mid; else hi = mid;
+            }
+            return lo;
+        };
+        for (uint32_t j = threadIdx.x; j <= groups; j += blockDim.x) {
+            const uint32_t e = min(j * 256, edges);
+            const uint32_t row = j < groups ? row_at(e) : rows_g;
+            const uint64_t cost = (uint64_t)e + (uint64_t)kBpRowCost * row;
+            const uint64_t before = j ? (uint64_t)(j - 1) * 256 + (uint64_t)kBpRowCost * row_at((j - 1) * 256) : 0;
+            for (uint32_t k = 0; k < kBpStarts; ++k) {
+                const uint64_t want = total * k / kBpWarps;
+                if (cost < want || (j && before >= want)) continue;
+                const bool cut = e < edges && po[rows[vb + row].x] - first < e;
+                starts[g * kBpStarts + k] = make_uint2(e, e < edges ? row | (cut ? 0x80000000u : 0u) : 0u);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -599,7 +750,8 @@ int batch_create(gbx_batch *b, uint32_t G, const uint32_t *vertex_base, const ui
     std::vector<uint32_t> order(G);
     std::vector<uint64_t> eg(G);
     for (uint32_t g = 0; g < G; ++g) {
-        eg[g] = (uint64_t)off[vb[g + 1]] - off[vb[g]] + (vb[g + 1] - vb[g]);
+        b->h_edges.push_back(off[vb[g + 1]] - off[vb[g]]);
+        eg[g] = (uint64_t)b->h_edges[g] + (vb[g + 1] - vb[g]);
         b->max_v = std::max(b->max_v, vb[g + 1] - vb[g]);
     }
     std::iota(order.begin(), order.end(), 0u);
@@ -640,7 +792,59 @@ void batch_free(gbx_batch *b) {
     cudaFree(b->in_offsets);
     cudaFree(b->in_src);
     cudaFree(b->order);
+    dev_free(b->words);
+    dev_free(b->wbase);
+    dev_free(b->rows);
+    dev_free(b->starts);
     delete b;
+}
+
+// Shared memory of pr_batched_kernel: contributions (room for two buffers of
+// the largest graph where that fits) and the warps' pending row sums.
+uint32_t bp_smem_v(const gbx_batch *b) {
+    const uint32_t room = (b->max_v + 31) & ~31u;
+    return std::min(kBpSmemV, 2 * (uint64_t)room <= kBpSmemV ? 2 * room : room);
+}
+
+// The word layout, complete on return (any stream may use it).
+int bp_layout(gbx_batch *b, cudaStream_t s) {
+    std::lock_guard<std::mutex> lock(b->words_mutex);
+    if (b->starts) return GBX_OK;
+    const uint32_t smem_v = bp_smem_v(b);
+    std::vector<uint32_t> wbase(b->G);
+    uint64_t at = 0;
+    for (uint32_t g = 0; g < b->G; ++g) {
+        const uint32_t v = b->h_vbase[g + 1] - b->h_vbase[g];
+        wbase[g] = (uint32_t)at;
+        at += ((uint64_t)b->h_edges[g] + 255) / 256 * (v <= kBpShortV && ((v + 31) & ~31u) <= smem_v ? 32 : 64);
+    }
+    auto build = [&]() -> int {
+        GBX_TRY(dev_alloc((void **)&b->words, std::max<uint64_t>(at, 1) * sizeof(uint4), s));
+        GBX_TRY(dev_alloc((void **)&b->wbase, (size_t)b->G * 4, s));
+        GBX_TRY(dev_alloc((void **)&b->rows, (size_t)b->V * sizeof(uint2), s));
+        uint2 *starts = nullptr;
+        GBX_TRY(dev_alloc((void **)&starts, (size_t)b->G * kBpStarts * sizeof(uint2), s));
+        b->starts = starts;
+        GBX_CUDA(cudaMemcpyAsync(b->wbase, wbase.data(), (size_t)b->G * 4, cudaMemcpyHostToDevice, s));
+        const unsigned grid = std::min<unsigned>(b->G, (unsigned)num_sms() * 2);
+        bp_layout_kernel<<<grid, kBpThreads, 0, s>>>(b->G, b->order, b->vbase, b->offsets, b->poff(), b->psrc(), b->wbase, smem_v,
+                                              b->words, b->rows, b->starts);
+        GBX_LAUNCH_CHECK();
+        GBX_CUDA(cudaStreamSynchronize(s));
+        return GBX_OK;
+    };
+    const int st = build();
+    if (st != GBX_OK) {
+        cudaStreamSynchronize(s);
+        dev_free(b->words);
+        dev_free(b->wbase);
+        dev_free(b->rows);
+            dev_free(b->starts);
+        b->words = nullptr;
+        b->wbase = nullptr;
+        b->rows = b->starts = nullptr;
+    }
+    return st;
 }
 
 }  // namespace
@@ -755,36 +959,38 @@ extern "C" int gbx_pr_batched(gbx_batch *b, uint32_t max_iterations, double epsi
     GBX_REQUIRE(epsilon >= 0.0, GBX_ERR_INVALID, "epsilon must be >= 0");
     GBX_TRY(ensure_device());
     cudaStream_t s = (cudaStream_t)stream;
+    GBX_TRY(bp_layout(b, s));
     OutArray<float> out;
     OutArray<gbx_pr_result> res;
     GBX_TRY(out.bind(ranks, b->V, s));
     GBX_TRY(res.bind(results, b->G, s));
-    DevBuf<float> other, scratch;
+    DevBuf<float> other, next, scratch;
     DevBuf<uint32_t> cursor;
     GBX_TRY(other.alloc(b->V, s));
     GBX_TRY(cursor.alloc(1, s));
     GBX_CUDA(cudaMemsetAsync(cursor.p, 0, 4, s));
-    const size_t smem = kBpSmemBytes;
+    const uint32_t smem_v = bp_smem_v(b), room = (b->max_v + 31) & ~31u;
+    const size_t smem = ((size_t)smem_v + kBpWarps * kBpBuf) * sizeof(float);
     GBX_CUDA(cudaFuncSetAttribute(pr_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int occ = 0;
-    GBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pr_batched_kernel, kBpThreads, smem));
-    const unsigned grid = std::max(1u, std::min<unsigned>((unsigned)num_sms() * std::max(occ, 1), b->G));
+    const unsigned grid = std::min<unsigned>((unsigned)num_sms(), b->G);
+    if (2 * (uint64_t)room > smem_v) GBX_TRY(next.alloc((size_t)grid * room, s));
+    if (room > smem_v) GBX_TRY(scratch.alloc((size_t)grid * room, s));
     BpArgs a;
-    a.scratch = nullptr;
-    a.scratch_v = 0;
-    if (b->max_v > kBpSmemV) {
-        a.scratch_v = b->max_v;
-        GBX_TRY(scratch.alloc((size_t)grid * b->max_v, s));
-        a.scratch = scratch.p;
-    }
     a.G = b->G;
     a.vbase = b->vbase;
     a.off = b->offsets;
     a.poff = b->poff();
-    a.psrc = b->psrc();
     a.order = b->order;
+    a.words = b->words;
+    a.wbase = b->wbase;
+    a.starts = b->starts;
+    a.rows = b->rows;
     a.ranks = out.d;
     a.rother = other.p;
+    a.next = next.p;
+    a.scratch = scratch.p;
+    a.max_v = room;
+    a.smem_v = smem_v;
     a.cursor = cursor.p;
     a.max_it = max_iterations;
     a.epsilon = epsilon;
