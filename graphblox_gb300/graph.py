@@ -814,7 +814,9 @@ def generate_values(count: int, kind: int, lo: int = 0, hi: int = 0, seed: int =
 
 
 def _results_dict(arr, fields):
-    return {f: np.array([getattr(r, f) for r in arr]) for f in fields}
+    """{field: array} of a ctypes array of result structs (64-bit integers and floats)."""
+    view = np.ctypeslib.as_array(arr)
+    return {f: view[f].astype(np.float64 if view.dtype[f].kind == "f" else np.int64) for f in fields}
 
 
 @dataclass
