@@ -689,6 +689,230 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
     }
 }
 
+// ---- small graphs: one CTA ---------------------------------------------------
+// A traversal of a small graph is a chain of latencies: the persistent kernel
+// spends 8 to 9 us per step on a grid barrier, the counters' round trip and
+// three or four dependent loads through L2, whatever the step holds. One CTA
+// keeps the bitmaps in shared memory, ends a step with __syncthreads, and
+// finds the graph in its L1 after the first steps; it also writes the initial
+// levels and parents, so a traversal is one plain launch. The state machine is
+// bfs_persistent_kernel's, line for line; only the order in which a step's
+// vertices are claimed differs (which of several parents wins is a race there
+// too). Above kSmallEdges one SM's throughput loses against 152.
+constexpr int kSmallThreads = 1024;
+constexpr uint32_t kSmallWords = 2048;  // V <= 65,536
+// 8,000-vertex R-MAT graph, 80k edges: 38 us against 54 for one traversal;
+// 16,000 and 160k: 62 against 58; crawl graph of 80k edges: 138 against 136.
+constexpr uint32_t kSmallEdges = 65536;
+constexpr uint32_t kSmallBatch = 64;  // traversals per launch, one CTA each
+constexpr uint32_t kSmallHub = 128;   // out-degree above which the whole CTA takes a row
+constexpr uint32_t kSmallHubs = 1024;
+
+struct SmallSources {
+    uint32_t v[kSmallBatch];
+};
+
+// CTA i traverses from sources.v[i] into level / parent + i * stride (either may be null)
+__global__ void __launch_bounds__(kSmallThreads, 1)
+    bfs_small_kernel(BfsArgs a, SmallSources sources, uint64_t stride) {
+    a.source = sources.v[blockIdx.x];
+    if (a.level) a.level += blockIdx.x * stride;
+    if (a.parent) a.parent += blockIdx.x * stride;
+    if (a.slot) a.slot += blockIdx.x;
+    __shared__ uint32_t s_visited[kSmallWords], s_bm[2][kSmallWords];
+    __shared__ uint32_t s_pre[kSmallThreads / 32][33], s_row[kSmallThreads / 32][32];
+    __shared__ uint32_t s_hub[kSmallHubs], s_hubs;
+    __shared__ uint32_t s_cnt[2][2];               // nf, mf; alternating per step
+    __shared__ unsigned long long s_edges[2];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kSmallThreads / 32;
+    uint32_t mu = a.E, mf = __ldg(a.outdeg + a.source), qsize = 1, nf_prev = 0, L = 0;
+    uint32_t processed = 1, iteration = 1, td = 0, bu = 0;
+    unsigned long long edges_total = mf;
+    bool in_bu = false, done = false, failed = false;
+    for (uint32_t v = threadIdx.x; v < a.V; v += kSmallThreads) {
+        const uint32_t d = __ldg(a.outdeg + v);
+        if (a.level) a.level[v] = 0u;
+        if (a.parent) a.parent[v] = v == a.source ? (int32_t)v : (d ? -(int32_t)d : -1);
+    }
+    for (uint32_t w = threadIdx.x; w < a.words; w += kSmallThreads) {
+        const uint32_t bit = w == (a.source >> 5) ? 1u << (a.source & 31) : 0u;
+        s_visited[w] = bit;
+        s_bm[0][w] = bit;
+        s_bm[1][w] = 0;
+    }
+    if (threadIdx.x < 2) {
+        s_cnt[threadIdx.x][0] = s_cnt[threadIdx.x][1] = 0;
+        s_edges[threadIdx.x] = 0;
+        s_hubs = 0;
+    }
+    const uint32_t max_steps = 2 * a.V + 16;
+    for (uint32_t s = 0; !done; ++s) {
+        __syncthreads();
+        if (s >= max_steps) {
+            failed = true;
+            break;
+        }
+        const uint32_t ib = s & 1;
+        uint32_t *cur = s_bm[ib], *next = s_bm[ib ^ 1];
+        uint32_t nf_mine = 0, mf_mine = 0, edges_mine = 0;
+        auto claim = [&](uint32_t v, uint32_t from) {
+            const uint32_t bit = 1u << (v & 31);
+            if (s_visited[v >> 5] & bit) return;
+            if (atomicOr(&s_visited[v >> 5], bit) & bit) return;
+            atomicOr(&next[v >> 5], bit);
+            const uint32_t d = __ldg(a.outdeg + v);
+            if (a.level) a.level[v] = L + 1;
+            if (a.parent) a.parent[v] = (int32_t)from;
+            ++nf_mine;
+            mf_mine += d ? d : 1u;
+            edges_mine += d;
+        };
+        const bool use_bu = a.mode == 0 || (a.mode == 2 && (in_bu || mf > mu / a.alpha));
+        if (use_bu) {
+            if (!in_bu) {
+                nf_prev = qsize;
+                in_bu = true;
+            }
+            for (uint32_t w = warp; w < a.words; w += warps) {
+                const uint32_t v = w * 32 + lane;
+                const bool open = ((~s_visited[w] & __ldg(a.live + w)) >> lane) & 1u;
+                uint32_t j = open ? __ldg(a.poff + v) : 0u;
+                const uint32_t e = open ? __ldg(a.poff + v + 1) : 0u;
+                uint32_t found = ~0u;
+                // up to 32 in-edges a lane alone, four loads in flight
+                for (uint32_t probes = 0; probes < 32 && found == ~0u && j < e; probes += 4, j += 4) {
+                    uint32_t u[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) u[q] = j + q < e ? __ldg(a.psrc + j + q) : ~0u;
+#pragma unroll
+                    for (int q = 3; q >= 0; --q)
+                        if (u[q] != ~0u && ((cur[u[q] >> 5] >> (u[q] & 31)) & 1u)) found = u[q];
+                }
+                // the rest of long rows by the whole warp
+                unsigned more = __ballot_sync(0xffffffffu, found == ~0u && j < e);
+                while (more) {
+                    const int k = __ffs(more) - 1;
+                    more &= more - 1;
+                    const uint32_t b0 = __shfl_sync(0xffffffffu, j, k), e0 = __shfl_sync(0xffffffffu, e, k);
+                    for (uint32_t b = b0; b < e0; b += 32) {
+                        const uint32_t u = b + lane < e0 ? __ldg(a.psrc + b + lane) : ~0u;
+                        const unsigned hit =
+                            __ballot_sync(0xffffffffu, u != ~0u && ((cur[u >> 5] >> (u & 31)) & 1u));
+                        if (!hit) continue;
+                        const uint32_t from = __shfl_sync(0xffffffffu, u, __ffs(hit) - 1);
+                        if ((int)lane == k) found = from;
+                        break;
+                    }
+                }
+                const unsigned hit = __ballot_sync(0xffffffffu, found != ~0u);
+                if (found != ~0u) {
+                    if (a.level) a.level[v] = L + 1;
+                    if (a.parent) a.parent[v] = (int32_t)found;
+                    edges_mine += __ldg(a.outdeg + v);
+                    ++nf_mine;
+                }
+                if (lane == 0) {  // the warp owns the word
+                    s_visited[w] |= hit;
+                    next[w] = hit;
+                }
+            }
+        } else {
+            mu -= mf;
+            for (uint32_t w = warp; w < a.words; w += warps) {
+                const uint32_t fw = cur[w];
+                if (!fw) continue;
+                const uint32_t u = w * 32 + lane;
+                const bool mine = (fw >> lane) & 1u;
+                const uint32_t b = mine ? __ldg(a.off + u) : 0u;
+                uint32_t d = mine ? __ldg(a.off + u + 1) - b : 0u;
+                if (d > kSmallHub) {
+                    const uint32_t at = atomicAdd(&s_hubs, 1u);
+                    if (at < kSmallHubs) {
+                        s_hub[at] = u;
+                        d = 0;
+                    }
+                }
+                uint32_t incl = d;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= (uint32_t)o) incl += t;
+                }
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                s_pre[warp][lane] = incl - d;
+                s_row[warp][lane] = b;
+                __syncwarp();
+                for (uint32_t j = lane; j < total; j += 32) {
+                    uint32_t k = 0;  // the last row that begins at or before j
+#pragma unroll
+                    for (uint32_t step = 16; step; step >>= 1)
+                        if (s_pre[warp][k + step] <= j) k += step;
+                    claim(__ldg(a.dest + s_row[warp][k] + (j - s_pre[warp][k])), w * 32 + k);
+                }
+                __syncwarp();
+            }
+            __syncthreads();
+            const uint32_t hubs = min(s_hubs, kSmallHubs);
+            for (uint32_t h = 0; h < hubs; ++h) {
+                const uint32_t u = s_hub[h], b = __ldg(a.off + u), e = __ldg(a.off + u + 1);
+                for (uint32_t j = b + threadIdx.x; j < e; j += kSmallThreads) claim(__ldg(a.dest + j), u);
+            }
+        }
+        nf_mine = __reduce_add_sync(0xffffffffu, nf_mine);
+        mf_mine = __reduce_add_sync(0xffffffffu, mf_mine);
+        edges_mine = __reduce_add_sync(0xffffffffu, edges_mine);
+        if (lane == 0 && nf_mine) {
+            atomicAdd(&s_cnt[ib][0], nf_mine);
+            atomicAdd(&s_cnt[ib][1], mf_mine);
+            atomicAdd(&s_edges[ib], (unsigned long long)edges_mine);
+        }
+        __syncthreads();
+        const uint32_t nf = s_cnt[ib][0];
+        const uint32_t step_mf = s_cnt[ib][1];
+        edges_total += s_edges[ib];
+        // this step's frontier becomes the one after next's output
+        for (uint32_t w = threadIdx.x; w < a.words; w += kSmallThreads) cur[w] = 0;
+        if (threadIdx.x == 0) {
+            s_cnt[ib ^ 1][0] = s_cnt[ib ^ 1][1] = 0;
+            s_edges[ib ^ 1] = 0;
+            s_hubs = 0;
+        }
+        processed += nf;
+        iteration++;
+        if (nf) L++;
+        if (use_bu) {
+            bu++;
+            const bool again = a.mode == 0 ? nf > 0 : (nf > nf_prev || nf > a.V / a.beta);
+            nf_prev = nf;
+            if (!again) {
+                in_bu = false;
+                qsize = nf;
+                if (nf == 0 || a.mode == 0) done = true;
+                mf = 1;
+            }
+        } else {
+            td++;
+            mf = step_mf;
+            qsize = nf;
+            if (nf == 0) done = true;
+        }
+    }
+    if (threadIdx.x == 0) {
+        if (!a.slot) {
+            BfsState *st = a.st;
+            st->gs.error = 0;
+            st->processed = processed;
+            st->iteration = iteration;
+            st->td_steps = td;
+            st->bu_steps = bu;
+            st->depth = L;
+            st->edges_total = edges_total;
+            st->status = failed ? 1u : 0u;
+        } else
+            *a.slot = BfsSlot{processed, iteration, td, bu, L, failed ? 1u : 0u, 0u, 0u, edges_total};
+    }
+}
+
 // Per traversal: levels, parents, visited and both frontier bitmaps, the
 // traversal state (zeroed as 32-bit words by the grid), and the generation-0
 // lists: the source alone, as a hub when its degree is large. The state
@@ -815,27 +1039,17 @@ int bfs_graph_setup(gbx_graph *g, cudaStream_t s) {
     return GBX_OK;
 }
 
-// One traversal from `source` on stream s: the init kernel, then the
-// persistent kernel, levels into lev and parents into parp (device arrays
-// of V entries).
-int bfs_enqueue(gbx_graph *g, const BfsWork &w, uint32_t source, int mode, uint32_t *lev, int32_t *parp,
-                BfsSlot *slot, cudaStream_t s) {
-    const uint32_t V = g->V, words = (V + 31) / 32;
-    const unsigned grid1 = std::min<unsigned>(ceil_div(V, 256), (unsigned)num_sms() * 8);
-    bfs_init_kernel<<<grid1, 256, 0, s>>>(lev, parp, w.visited, w.bm0, w.bm1, V, words, source, g->out_degree,
-                                          w.q0, w.hv0, w.hc0, w.st);
-    GBX_LAUNCH_CHECK();
-    BfsArgs a;
+BfsArgs bfs_args(const gbx_graph *g, const BfsWork &w, int mode, uint32_t *lev, int32_t *parp, BfsSlot *slot) {
+    BfsArgs a{};
     a.off = g->offsets;
     a.dest = g->dest;
     a.poff = g->pull_offsets();
     a.psrc = g->pull_src();
     a.outdeg = g->out_degree;
-    a.V = V;
-    a.words = words;
+    a.V = g->V;
+    a.words = (g->V + 31) / 32;
     a.E = g->E;
     a.mode = (uint32_t)mode;
-    a.source = source;
     a.alpha = g->bfs_alpha;
     a.beta = g->bfs_beta;
     a.pull_live = g->pull_sources_live == 1 ? 1u : 0u;
@@ -854,6 +1068,35 @@ int bfs_enqueue(gbx_graph *g, const BfsWork &w, uint32_t source, int mode, uint3
     a.hc[1] = w.hc1;
     a.st = w.st;
     a.slot = slot;
+    return a;
+}
+
+// n traversals of g that may run at once are taken by bfs_small_kernel
+bool bfs_is_small(const gbx_graph *g, uint32_t n) {
+    return (g->V + 31) / 32 <= kSmallWords && g->E <= (uint64_t)kSmallEdges * std::min(n, 8u) && !trace_enabled();
+}
+
+// n <= kSmallBatch traversals, one CTA each, outputs `stride` entries apart
+int bfs_enqueue_small(const BfsArgs &a, const uint32_t *sources, uint32_t n, uint64_t stride, cudaStream_t s) {
+    SmallSources src{};
+    std::copy(sources, sources + n, src.v);
+    bfs_small_kernel<<<n, kSmallThreads, 0, s>>>(a, src, stride);
+    GBX_LAUNCH_CHECK();
+    return GBX_OK;
+}
+
+// One traversal from `source` on stream s (the small-graph kernel, or the init
+// kernel and the persistent kernel), levels into lev and parents into parp
+// (device arrays of V entries).
+int bfs_enqueue(gbx_graph *g, const BfsWork &w, uint32_t source, int mode, uint32_t *lev, int32_t *parp,
+                BfsSlot *slot, cudaStream_t s) {
+    BfsArgs a = bfs_args(g, w, mode, lev, parp, slot);
+    if (bfs_is_small(g, 1)) return bfs_enqueue_small(a, &source, 1, 0, s);
+    a.source = source;
+    const unsigned grid1 = std::min<unsigned>(ceil_div(a.V, 256), (unsigned)num_sms() * 8);
+    bfs_init_kernel<<<grid1, 256, 0, s>>>(lev, parp, w.visited, w.bm0, w.bm1, a.V, a.words, source, g->out_degree,
+                                          w.q0, w.hv0, w.hc0, w.st);
+    GBX_LAUNCH_CHECK();
     int grid = 0;
     static int grid_cache[64] = {0};
     GBX_TRY(coop_grid(bfs_persistent_kernel, kBfsThreads, 0, &grid, &grid_cache));
@@ -988,9 +1231,17 @@ extern "C" int gbx_bfs_trials(gbx_graph *g, const uint32_t *sources, uint32_t nu
     if (par_host) GBX_TRY(pstage.alloc(2 * (size_t)V, s));
     CopyLane copies;
     if (dist_host || par_host) GBX_TRY(copies.create());
+    // small graphs, each trial with outputs of its own: many trials per launch
+    const bool at_once = !copies.cs && (out_stride || (!distances && !parents)) && bfs_is_small(g, num_sources);
+    for (uint32_t i = 0; at_once && i < num_sources; i += kSmallBatch) {
+        const size_t off = (size_t)i * out_stride;
+        BfsArgs a = bfs_args(g, w, mode, distances ? distances + off : nullptr, parents ? parents + off : nullptr,
+                             slots.p + i);
+        GBX_TRY(bfs_enqueue_small(a, sources + i, std::min(kSmallBatch, num_sources - i), out_stride, s));
+    }
     // every traversal re-initialises the shared work arrays on the stream, so
     // the traversals run back to back without the host in between
-    for (uint32_t i = 0; i < num_sources; ++i) {
+    for (uint32_t i = 0; !at_once && i < num_sources; ++i) {
         const uint32_t b = i & 1;
         const size_t off = (size_t)i * out_stride;
         uint32_t *lev = dist_host ? dstage.p + (size_t)b * V : distances ? distances + off : w.level;
