@@ -190,14 +190,27 @@ __device__ __forceinline__ bool ppr_done(const PprCtl *ctl) {
 }
 
 // One sweep: each chunk's P-weighted sum of neighbour rows; whole-row chunks
-// finish their row, chunks of split rows leave partials.
+// finish their row, chunks of split rows leave partials. A chunk's ids and
+// weights come 32 at a time, one per lane, and kBatch neighbour rows are in
+// flight, the last, partial batch included; the order of a row's additions is
+// that of its edges. One resident wave of CTAs: chunks are dealt by a fixed
+// stride, and a second wave would wait for the first.
+//
+// Bound by what the L2s deliver to the SMs: 7.4 of the 9.5 TB/s that random
+// sectors reach (RMAT-20, K = 64: 147M sectors in 0.63 ms), with DRAM at 1.5 GB
+// a sweep. Forward and adjoint, RMAT-20 K = 64: 110 -> 106 ms; 200,000
+// vertices, K = 32: 22.2 -> 18.2, K = 128: 37.2 -> 30.5, K = 256: 64.6 -> 59.7;
+// 1,000 vertices, whose longest chunk is the sweep: 6.0 -> 4.7. Slower, RMAT-20:
+// walking units of rows as one stream with rows gathered across row ends 127,
+// through a cp.async ring 131; descriptors and ids fetched a chunk ahead 124.
 template <int KPL>
-__global__ void __launch_bounds__(kPprThreads)
+__global__ void __launch_bounds__(kPprThreads, KPL <= 2 ? 6 : KPL == 4 ? 5 : 1)
     ppr_sweep_kernel(const PprChunk *__restrict__ chunks, uint32_t n_chunks, const uint32_t *__restrict__ col,
                      const float *__restrict__ P, const float *__restrict__ X, float *__restrict__ Xn,
                      const float *__restrict__ B, float bscale, float d, float *__restrict__ partials,
                      double *res_out, const PprCtl *ctl) {
     if (ppr_done(ctl)) return;
+    constexpr int kBatch = KPL <= 2 ? 8 : 4;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -209,29 +222,38 @@ __global__ void __launch_bounds__(kPprThreads)
         float acc[KPL];
 #pragma unroll
         for (int i = 0; i < KPL; ++i) acc[i] = 0.f;
-        uint32_t e = ck.eb;
-        for (; e + 4 <= ck.ee; e += 4) {
-            uint32_t u[4];
-            float p[4];
+        // ids and weights 32 at a time, one per lane; kBatch rows in flight
+        for (uint32_t e = ck.eb; e < ck.ee; e += 32) {
+            const uint32_t m = min(ck.ee - e, 32u);
+            const uint32_t ids = lane < m ? __ldg(col + e + lane) : 0u;
+            const float wts = lane < m ? __ldg(P + e + lane) : 0.f;
+            uint32_t j = 0;
+            for (; j + kBatch <= m; j += kBatch) {
+                Vec<KPL> x[kBatch];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                u[q] = __ldg(col + e + q);
-                p[q] = __ldg(P + e + q);
+                for (int q = 0; q < kBatch; ++q)
+                    x[q] = load_row<KPL>(X, __shfl_sync(0xffffffffu, ids, j + q), lane);
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) {
+                    const float p = __shfl_sync(0xffffffffu, wts, j + q);
+#pragma unroll
+                    for (int i = 0; i < KPL; ++i) acc[i] = __fmaf_rn(p, x[q].v[i], acc[i]);
+                }
             }
-            Vec<KPL> x[4];
+            if (j < m) {  // the last, partial batch: rows past it are its last one again, unused
+                Vec<KPL> x[kBatch];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) x[q] = load_row<KPL>(X, u[q], lane);
+                for (int q = 0; q < kBatch; ++q)
+                    x[q] = load_row<KPL>(X, __shfl_sync(0xffffffffu, ids, min(j + q, m - 1)), lane);
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
+                for (int q = 0; q < kBatch; ++q) {
+                    const float p = __shfl_sync(0xffffffffu, wts, (j + q) & 31);
+                    if (j + q < m) {
 #pragma unroll
-                for (int i = 0; i < KPL; ++i) acc[i] = __fmaf_rn(p[q], x[q].v[i], acc[i]);
-        }
-        for (; e < ck.ee; ++e) {
-            const uint32_t u = __ldg(col + e);
-            const float p = __ldg(P + e);
-            const Vec<KPL> x = load_row<KPL>(X, u, lane);
-#pragma unroll
-            for (int i = 0; i < KPL; ++i) acc[i] = __fmaf_rn(p, x.v[i], acc[i]);
+                        for (int i = 0; i < KPL; ++i) acc[i] = __fmaf_rn(p, x[q].v[i], acc[i]);
+                    }
+                }
+            }
         }
         if (ck.slot == kNoSlot)
             ppr_finish_row<KPL>(ck.row, lane, acc, X, Xn, B, bscale, d, res);
@@ -259,10 +281,18 @@ __global__ void __launch_bounds__(kPprThreads)
         float acc[KPL];
 #pragma unroll
         for (int i = 0; i < KPL; ++i) acc[i] = 0.f;
-        for (uint32_t s = split_first[h]; s < split_first[h + 1]; ++s) {
-            const Vec<KPL> p = load_row<KPL>(partials, s, lane);
+        constexpr int kAhead = KPL <= 2 ? 8 : 4;  // partials in flight; added in slot order
+        const uint32_t s1 = split_first[h + 1];
+        for (uint32_t s = split_first[h]; s < s1; s += kAhead) {
+            Vec<KPL> p[kAhead];
 #pragma unroll
-            for (int i = 0; i < KPL; ++i) acc[i] = __fadd_rn(acc[i], p.v[i]);
+            for (int q = 0; q < kAhead; ++q) p[q] = load_row<KPL>(partials, min(s + q, s1 - 1), lane);
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q)
+                if (s + q < s1) {
+#pragma unroll
+                    for (int i = 0; i < KPL; ++i) acc[i] = __fadd_rn(acc[i], p[q].v[i]);
+                }
         }
         ppr_finish_row<KPL>(split_rows[h], lane, acc, X, Xn, B, bscale, d, res);
     }
@@ -545,10 +575,15 @@ int ppr_solve(const PprPlan &plan, const uint32_t *col, const float *P, const fl
     GBX_LAUNCH_CHECK();
     float *X[2] = {X0, X1};
     PprCtl h{};
+    // no CTA without a chunk: each one adds its K column sums to the same words
+    int per_sm = 0;
+    GBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ppr_sweep_kernel<KPL>, kPprThreads, 0));
+    const unsigned sgrid = std::max(1u, std::min<unsigned>((unsigned)(num_sms() * std::max(per_sm, 1)),
+                                                           ceil_div(plan.n_chunks, kPprWarps)));
     const unsigned cgrid = std::max(1u, std::min<unsigned>(grid, ceil_div((uint64_t)plan.n_split * 32, 256)));
     for (uint32_t it = 0; it < max_it; ++it) {
         double *rc = resb.p + (it & 1) * K, *rn = resb.p + ((it + 1) & 1) * K;
-        ppr_sweep_kernel<KPL><<<grid, kPprThreads, 0, s>>>(plan.chunks, plan.n_chunks, col, P, X[it & 1],
+        ppr_sweep_kernel<KPL><<<sgrid, kPprThreads, 0, s>>>(plan.chunks, plan.n_chunks, col, P, X[it & 1],
                                                            X[(it + 1) & 1], B, bscale, d, partials, rc, ctl.p);
         GBX_LAUNCH_CHECK();
         if (plan.n_split) {
