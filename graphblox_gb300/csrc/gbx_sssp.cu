@@ -594,6 +594,158 @@ __global__ void sssp_finish_kernel(const uint32_t *dist, const uint32_t *outdeg,
     }
 }
 
+// ---- small graphs: one CTA ---------------------------------------------------
+// As for BFS (gbx_bfs.cu): a round of the persistent kernel costs 10 to 12 us
+// however little it holds. One CTA keeps distances and frontier bitmaps in
+// shared memory and relaxes the whole frontier every round (no buckets: a
+// small graph has few rounds, and a vertex relaxed early is relaxed again),
+// in one launch that also writes the distances and counts what was reached.
+// The distances are the same fixed point.
+constexpr int kSsspSmallThreads = 1024;
+constexpr uint32_t kSsspSmallV = 24576;  // 96 KB of distances
+// R-MAT, 1,000 vertices, 10k edges: 172 -> 72 us; 4,000 and 40k: 175 -> 184.
+constexpr uint32_t kSsspSmallE = 24576;
+constexpr uint32_t kSsspSmallHub = 128;  // out-degree above which the whole CTA takes a row
+constexpr uint32_t kSsspSmallHubs = 1024;
+
+struct SsspSmallResult {
+    unsigned long long reached, edges, relaxed;
+    unsigned rounds, status;
+};
+
+__global__ void __launch_bounds__(kSsspSmallThreads, 1)
+    sssp_small_kernel(const uint32_t *off, const uint32_t *dest, const float *w, uint32_t V, uint32_t source,
+                      uint32_t max_rounds, uint32_t *out, SsspSmallResult *result) {
+    extern __shared__ uint32_t s_dist[];  // [V]
+    __shared__ uint32_t s_bm[2][kSsspSmallV / 32];
+    __shared__ uint32_t s_pre[kSsspSmallThreads / 32][33], s_row[kSsspSmallThreads / 32][32], s_d[kSsspSmallThreads / 32][32];
+    __shared__ uint32_t s_hub[kSsspSmallHubs], s_hubs;
+    __shared__ unsigned long long s_sum[3];  // reached, edges, relaxed
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kSsspSmallThreads / 32;
+    const uint32_t words = (V + 31) / 32;
+    for (uint32_t v = threadIdx.x; v < V; v += kSsspSmallThreads) s_dist[v] = v == source ? 0u : kSsspInf;
+    for (uint32_t i = threadIdx.x; i < words; i += kSsspSmallThreads) {
+        s_bm[0][i] = i == (source >> 5) ? 1u << (source & 31) : 0u;
+        s_bm[1][i] = 0;
+    }
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_hubs = 0;
+    __syncthreads();
+    unsigned long long relaxed = 0;
+    uint32_t rounds = 0;
+    bool failed = false;
+    for (;; ++rounds) {
+        if (rounds >= max_rounds) {
+            failed = true;
+            break;
+        }
+        uint32_t *cur = s_bm[rounds & 1], *next = s_bm[(rounds & 1) ^ 1];
+        bool any = false;
+        auto relax = [&](uint32_t d, uint32_t e) {
+            const uint32_t u = __ldg(dest + e);
+            const uint32_t nd = sssp_add(d, w ? __ldg(w + e) : 1.0f);
+            ++relaxed;
+            if (nd >= *(volatile uint32_t *)(s_dist + u)) return;
+            if (nd < atomicMin(s_dist + u, nd)) {
+                atomicOr(next + (u >> 5), 1u << (u & 31));
+                any = true;
+            }
+        };
+        for (uint32_t i = warp; i < words; i += warps) {
+            const uint32_t bits = cur[i];
+            if (!bits) continue;
+            const uint32_t v = i * 32 + lane;
+            const bool mine = (bits >> lane) & 1u;
+            const uint32_t b = mine ? __ldg(off + v) : 0u;
+            uint32_t n = mine ? __ldg(off + v + 1) - b : 0u;
+            if (n > kSsspSmallHub) {
+                const uint32_t at = atomicAdd(&s_hubs, 1u);
+                if (at < kSsspSmallHubs) {
+                    s_hub[at] = v;
+                    n = 0;
+                }
+            }
+            uint32_t incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += t;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            s_pre[warp][lane] = incl - n;
+            s_row[warp][lane] = b;
+            s_d[warp][lane] = mine ? *(volatile uint32_t *)(s_dist + v) : 0u;
+            __syncwarp();
+            for (uint32_t j = lane; j < total; j += 32) {
+                uint32_t k = 0;  // the last row that begins at or before j
+#pragma unroll
+                for (uint32_t step = 16; step; step >>= 1)
+                    if (s_pre[warp][k + step] <= j) k += step;
+                relax(s_d[warp][k], s_row[warp][k] + (j - s_pre[warp][k]));
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        const uint32_t hubs = min(s_hubs, kSsspSmallHubs);
+        for (uint32_t h = 0; h < hubs; ++h) {
+            const uint32_t v = s_hub[h], e = __ldg(off + v + 1), d = *(volatile uint32_t *)(s_dist + v);
+            for (uint32_t j = __ldg(off + v) + threadIdx.x; j < e; j += kSsspSmallThreads) relax(d, j);
+        }
+        const bool more = __syncthreads_or(any);
+        // this round's frontier becomes the one after next's output
+        for (uint32_t i = threadIdx.x; i < words; i += kSsspSmallThreads) cur[i] = 0;
+        if (threadIdx.x == 0) s_hubs = 0;
+        __syncthreads();
+        if (!more) {
+            ++rounds;
+            break;
+        }
+    }
+    unsigned long long reached = 0, edges = 0;
+    for (uint32_t v = threadIdx.x; v < V; v += kSsspSmallThreads) {
+        const uint32_t d = s_dist[v];
+        out[v] = d;
+        if (d != kSsspInf) {
+            ++reached;
+            edges += __ldg(off + v + 1) - __ldg(off + v);
+        }
+    }
+    reached = warp_sum(reached);
+    edges = warp_sum(edges);
+    relaxed = warp_sum(relaxed);
+    if (lane == 0) {
+        atomicAdd(s_sum, reached);
+        atomicAdd(s_sum + 1, edges);
+        atomicAdd(s_sum + 2, relaxed);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *result = SsspSmallResult{s_sum[0], s_sum[1], s_sum[2], rounds, failed ? 1u : 0u};
+}
+
+int sssp_small(gbx_graph *g, uint32_t source, uint32_t *distances, gbx_sssp_result *result, cudaStream_t s) {
+    const uint32_t V = g->V;
+    OutArray<uint32_t> out;
+    GBX_TRY(out.bind(distances, V, s));
+    DevBuf<SsspSmallResult> res;
+    GBX_TRY(res.alloc(1, s));
+    GBX_CUDA(cudaFuncSetAttribute(sssp_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSsspSmallV * 4)));
+    sssp_small_kernel<<<1, kSsspSmallThreads, (size_t)V * 4, s>>>(g->offsets, g->dest, g->weight, V, source,
+                                                                 4 * V + 64, out.d, res.p);
+    GBX_LAUNCH_CHECK();
+    GBX_TRY(out.finish(s));
+    SsspSmallResult h;
+    GBX_CUDA(cudaMemcpyAsync(&h, res.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+    GBX_CUDA(cudaStreamSynchronize(s));
+    GBX_REQUIRE(h.status == 0, GBX_ERR_ITER_CAP, "SSSP round cap reached");
+    if (result) {
+        result->reached = (uint32_t)h.reached;
+        result->rounds = h.rounds;
+        result->edges_relaxed = h.relaxed;
+        result->edges_traversed = h.edges;
+    }
+    return GBX_OK;
+}
+
 }  // namespace gbx
 
 using namespace gbx;
@@ -606,7 +758,12 @@ extern "C" int gbx_sssp(gbx_graph *g, uint32_t source, uint32_t delta, uint32_t 
     GBX_TRY(ensure_device());
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t V = g->V;
-    if (delta == 0) delta = g->sssp_delta ? g->sssp_delta : (g->weight ? 256u : 1u);
+    if (V <= kSsspSmallV && g->E <= kSsspSmallE && !trace_enabled()) return sssp_small(g, source, distances, result, s);
+    // Bucket width where neither the caller nor the graph's tuning gives one:
+    // up to a few million edges a round is mostly latency, so fewer, wider
+    // buckets (R-MAT of 250,000 vertices and 2.5M edges: 535 us with 256, 472
+    // with 1024; crawl of 1M edges: 711, 581; R-MAT of 8M edges: 1226, 1301)
+    if (delta == 0) delta = g->sssp_delta ? g->sssp_delta : !g->weight ? 1u : g->E <= 6'000'000u ? 1024u : 256u;
     // working arrays from the graph's scratch arena (plus staging for a
     // host-memory result)
     const int out_dev = is_device_ptr(distances) ? 1 : 0;
