@@ -11,7 +11,7 @@
 // Each level either pushes from a compacted frontier list (atomicOr of F[u]
 // into Fn of every out-neighbour; few frontier edges) or pulls over in-edges
 // (OR of F[u] over v's in-edges, stopping once every bit v still misses is
-// found). A group of NW lanes owns one vertex, lane k its k-th mask word, so a
+// found; a source whose frontier is empty is missed by nobody any more). A group of NW lanes owns one vertex, lane k its k-th mask word, so a
 // mask is one 4*NW-byte access. Pull rows above kMsLight in-edges are cut into
 // kMsChunk-edge chunks worked by whole warps and OR-ed into Fn with atomics
 // (OR is order-free, so the result is deterministic). An update pass then
@@ -45,6 +45,7 @@ struct MsCounters {
     uint32_t qn;                // next frontier list length
     uint32_t pad;
     unsigned long long mf;      // out-edges of the next frontier
+    uint32_t alive[8];          // sources whose next frontier holds any vertex
 };
 
 // ---- expansion: push ----------------------------------------------------------
@@ -57,12 +58,15 @@ __global__ void __launch_bounds__(kMsThreads)
     const uint32_t lane = threadIdx.x & 31, k = lane % NW;
     const uint32_t grp = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * GPW + lane / NW;
     const uint32_t ngrp = ((gridDim.x * blockDim.x) >> 5) * GPW;
-    for (uint32_t i = grp; i < qn; i += ngrp) {
-        const uint32_t u = q[i];
+    // a short list's rows are each shared by several groups (a hub among the
+    // sources: 118 us for its one group, 8 when shared)
+    const uint32_t share = max(1u, min(64u, ngrp / qn));
+    for (uint32_t i = grp; i < qn * share; i += ngrp) {
+        const uint32_t u = q[i / share];
         const uint32_t fu = F[(size_t)u * NW + k];
         if (!fu) continue;  // lane-local: other lanes of the group may still push
-        const uint32_t eb = off[u], ee = off[u + 1];
-        for (uint32_t e = eb; e < ee; e += 4) {
+        const uint32_t ee = off[u + 1];
+        for (uint32_t e = off[u] + 4 * (i % share); e < ee; e += 4 * share) {
             // four out-edges per round: targets, then their seen words
             uint32_t v[4], sw[4];
 #pragma unroll
@@ -80,13 +84,18 @@ __global__ void __launch_bounds__(kMsThreads)
 
 // ---- expansion: pull -----------------------------------------------------------
 // Light rows: one NW-lane group per vertex; the warp's groups step through
-// their rows together so the early-exit vote is warp-uniform.
+// their rows together so the early-exit vote is warp-uniform. A level of
+// RMAT-20 with 256 sources takes 233 us for light and heavy rows while every
+// source is alive (283 with four edges a round and ids fetched in the round)
+// and 50 to 70 once few are: bits of finished sources are not looked for.
 template <int NW>
 __global__ void __launch_bounds__(kMsThreads)
     ms_pull_light_kernel(const uint32_t *__restrict__ poff, const uint32_t *__restrict__ psrc, uint32_t V, uint32_t S,
-                         const uint32_t *__restrict__ F, const uint32_t *__restrict__ seen, uint32_t *__restrict__ Fn) {
-    constexpr int GPW = 32 / NW;
+                         const MsCounters *__restrict__ cnt, const uint32_t *__restrict__ F,
+                         const uint32_t *__restrict__ seen, uint32_t *__restrict__ Fn) {
+    constexpr int GPW = 32 / NW, kIds = 8 / NW;
     const uint32_t lane = threadIdx.x & 31, k = lane % NW;
+    const uint32_t alive = cnt->alive[k] & ms_valid(k, S);
     const uint32_t gmask = (NW == 32 ? 0xFFFFFFFFu : ((1u << NW) - 1u)) << (lane / NW * NW);
     const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarp = (gridDim.x * blockDim.x) >> 5;
@@ -96,26 +105,33 @@ __global__ void __launch_bounds__(kMsThreads)
         if (v < V) {
             b = poff[v];
             e = poff[v + 1];
-            need = ~seen[(size_t)v * NW + k] & ms_valid(k, S);
+            need = ~seen[(size_t)v * NW + k] & alive;
             if (e - b > kMsLight) e = b;  // heavy rows are worked by the chunk kernel
         }
         uint32_t acc = 0;
-        // group still searching: some lane of it has bits it needs and lacks
-        bool open = __ballot_sync(0xFFFFFFFFu, (need & ~acc) != 0 && b < e) & gmask;
+        // Eight in-edges per round: their ids, spread over the group's lanes
+        // and fetched a round ahead, then their mask words, all in flight
+        // together (the early exit checks once per round). open: some lane of
+        // the group has bits it needs and lacks.
+        bool open = __ballot_sync(0xFFFFFFFFu, need != 0 && b < e) & gmask;
         uint32_t j = b;
+        uint32_t ids[kIds];
+#pragma unroll
+        for (int i = 0; i < kIds; ++i) ids[i] = open && j + i * NW + k < e ? __ldg(psrc + j + i * NW + k) : 0u;
         while (__any_sync(0xFFFFFFFFu, open)) {
-            if (open) {
-                // four in-edges per round: their ids, then their mask words,
-                // in flight together (the early exit checks once per round)
-                uint32_t u[4];
+            uint32_t u[8];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) u[q] = j + q < e ? __ldg(psrc + j + q) : 0u;
+            for (int q = 0; q < 8; ++q) u[q] = __shfl_sync(0xFFFFFFFFu, ids[q / NW], q % NW, NW);
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (j + q < e) acc |= __ldg(F + (size_t)u[q] * NW + k);
-                j += 4;
-            }
-            open = __ballot_sync(0xFFFFFFFFu, (need & ~acc) != 0 && j < e) & gmask;
+            for (int i = 0; i < kIds; ++i)
+                ids[i] = open && j + 8 + i * NW + k < e ? __ldg(psrc + j + 8 + i * NW + k) : 0u;
+            uint32_t m[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) m[q] = open && j + q < e ? __ldg(F + (size_t)u[q] * NW + k) : 0u;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc |= m[q];
+            j += 8;
+            open = __ballot_sync(0xFFFFFFFFu, open && (need & ~acc) != 0 && j < e) & gmask;
         }
         if (v < V && acc) Fn[(size_t)v * NW + k] = acc;  // heavy rows leave acc 0 here
     }
@@ -129,27 +145,42 @@ struct MsChunk {
 template <int NW>
 __global__ void __launch_bounds__(kMsThreads)
     ms_pull_heavy_kernel(const MsChunk *__restrict__ chunks, uint32_t n_chunks, const uint32_t *__restrict__ psrc,
-                         uint32_t S, const uint32_t *__restrict__ F, const uint32_t *__restrict__ seen,
-                         uint32_t *__restrict__ Fn) {
+                         uint32_t S, const MsCounters *__restrict__ cnt, const uint32_t *__restrict__ F,
+                         const uint32_t *__restrict__ seen, uint32_t *__restrict__ Fn) {
     constexpr int GPW = 32 / NW;
+    constexpr int kPer = 8, kEdges = kPer * GPW;             // edges per group and per warp in a round
+    constexpr int kLoads = kEdges / 32 > 0 ? kEdges / 32 : 1;
     const uint32_t lane = threadIdx.x & 31, k = lane % NW, gi = lane / NW;
+    const uint32_t alive = cnt->alive[k] & ms_valid(k, S);
     const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarp = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t c = warp0; c < n_chunks; c += nwarp) {
         const MsChunk ck = chunks[c];
-        const uint32_t need = ~seen[(size_t)ck.row * NW + k] & ms_valid(k, S);
+        const uint32_t need = ~seen[(size_t)ck.row * NW + k] & alive;
+        if (!__any_sync(0xFFFFFFFFu, need)) continue;
         uint32_t acc = 0;
-        for (uint32_t j0 = ck.eb; j0 < ck.ee; j0 += 4 * GPW) {
-            // four edges per group per round, loads in flight together
-            uint32_t u[4];
+        // kEdges edges per round: 32 ids per load, fetched a round ahead, then
+        // each group's mask words in flight together
+        uint32_t ids[kLoads];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t j = j0 + q * GPW + gi;
-                u[q] = j < ck.ee ? __ldg(psrc + j) : 0u;
+        for (int i = 0; i < kLoads; ++i)
+            ids[i] = ck.eb + 32 * i + lane < ck.ee ? __ldg(psrc + ck.eb + 32 * i + lane) : 0u;
+        for (uint32_t j0 = ck.eb; j0 < ck.ee; j0 += kEdges) {
+            uint32_t u[kPer];
+#pragma unroll
+            for (int q = 0; q < kPer; ++q)
+                u[q] = __shfl_sync(0xFFFFFFFFu, ids[(q * GPW) / 32], (q * GPW) % 32 + gi);
+#pragma unroll
+            for (int i = 0; i < kLoads; ++i) {
+                const uint32_t j = j0 + kEdges + 32 * i + lane;
+                ids[i] = j < ck.ee ? __ldg(psrc + j) : 0u;
             }
+            uint32_t m[kPer];
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (j0 + q * GPW + gi < ck.ee) acc |= __ldg(F + (size_t)u[q] * NW + k);
+            for (int q = 0; q < kPer; ++q)
+                m[q] = j0 + q * GPW + gi < ck.ee ? __ldg(F + (size_t)u[q] * NW + k) : 0u;
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) acc |= m[q];
             // OR across the groups, then stop once every needed bit is present
             uint32_t all = acc;
 #pragma unroll
@@ -177,6 +208,10 @@ __global__ void __launch_bounds__(kMsThreads)
     // on the one length counter), the out-degree sum with one per warp
     constexpr uint32_t kCap = 128;
     __shared__ uint32_t s_q[kMsThreads / 32][kCap];
+    __shared__ uint32_t s_alive[NW];
+    if (threadIdx.x < NW) s_alive[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t alive = 0;
     constexpr int GPW = 32 / NW;
     const uint32_t lane = threadIdx.x & 31, k = lane % NW, gi = lane / NW;
     const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -200,6 +235,7 @@ __global__ void __launch_bounds__(kMsThreads)
             const size_t i = (size_t)v * NW + k;
             const uint32_t s0 = seen[i];
             nw = Fn[i] & ~s0;
+            alive |= nw;
             Fn[i] = nw;
             if (nw) {
                 seen[i] = s0 | nw;
@@ -222,6 +258,9 @@ __global__ void __launch_bounds__(kMsThreads)
     if (wn) flush();
     mf = warp_sum(mf);
     if (lane == 0 && mf) atomicAdd(&cnt->mf, mf);
+    if (alive) atomicOr(s_alive + k, alive);
+    __syncthreads();
+    if (threadIdx.x < NW && s_alive[threadIdx.x]) atomicOr(cnt->alive + threadIdx.x, s_alive[threadIdx.x]);
 }
 
 __global__ void ms_seed_kernel(const uint32_t *sources, uint32_t S, uint32_t NW, const uint32_t *off, uint32_t *seen,
@@ -232,6 +271,7 @@ __global__ void ms_seed_kernel(const uint32_t *sources, uint32_t S, uint32_t NW,
         atomicOr(F + (size_t)s * NW + i / 32, 1u << (i % 32));
         q[i] = s;  // a repeated source is pushed twice: OR makes that harmless
         atomicAdd(&cnt->mf, (unsigned long long)(off[s + 1] - off[s]));
+        atomicOr(cnt->alive + i / 32, 1u << (i % 32));
     }
     if (threadIdx.x == 0) cnt->qn = S;
 }
@@ -331,6 +371,143 @@ __global__ void __launch_bounds__(kMsThreads)
             atomicMax(s_depth + s0 + j, dm[j]);
         }
     }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < S; i += blockDim.x) {
+        // block 0 adds each source's own out-edges
+        const unsigned long long own = blockIdx.x == 0 ? __ldg(off + sources[i] + 1) - __ldg(off + sources[i]) : 0u;
+        if (s_cnt[i] || own) {
+            atomicAdd(cnt + i, s_cnt[i]);
+            atomicAdd(edges + i, s_edges[i] + own);
+            atomicMax(depth + i, s_depth[i]);
+        }
+    }
+}
+
+// The same for a traversal of up to 2^kPlanes levels, all of them kept (the
+// usual case). A lane first takes one mask word of one vertex and turns the
+// levels of its 32 sources into kPlanes bit planes of the level number --
+// GPW vertices per warp, loads coalesced, four instructions per level and
+// word. Then the warp goes through those vertices one by one: each lane gets
+// the planes' NW bits of its own sources by a shuffle, spreads them to bytes
+// with a multiplication, and writes its NW levels. The deepest level of a
+// source is kept as one word per level; counts as bytes that are emptied every
+// 255 vertices. Bound by the 4 V S bytes written: RMAT-20, 256 sources, 1.07 GB
+// in 286 us; a select per source and level, and 64-bit sums per source and
+// vertex, took 730 us.
+template <int NW, int kPlanes>
+__global__ void __launch_bounds__(kMsThreads)
+    ms_planes_kernel(MsLevels lv, uint32_t V, uint32_t S, const uint32_t *__restrict__ off,
+                     const uint32_t *__restrict__ sources, bool vec_rows, uint32_t *__restrict__ dist,
+                     uint32_t *__restrict__ cnt, unsigned long long *__restrict__ edges, uint32_t *__restrict__ depth) {
+    constexpr int GPW = 32 / NW, kLevels = 1 << kPlanes;
+    __shared__ uint32_t s_cnt[32 * NW], s_depth[32 * NW];
+    __shared__ unsigned long long s_edges[32 * NW];
+    for (uint32_t i = threadIdx.x; i < 32 * NW; i += blockDim.x) {
+        s_cnt[i] = 0;
+        s_depth[i] = 0;
+        s_edges[i] = 0;
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t s0 = lane * NW, word = s0 / 32, sh = s0 % 32;  // this lane's sources in the second half
+    constexpr uint32_t bmask = (1u << NW) - 1u;
+    uint32_t at_level[kLevels];  // first half: sources of this lane's word that reach anything at each level
+#pragma unroll
+    for (int L = 0; L < kLevels; ++L) at_level[L] = 0;
+    uint32_t c4[(NW + 3) / 4], ed[NW];  // reached: a byte per source; out-degree sums
+    unsigned long long held = 0;        // what ed may have grown to
+    uint32_t since = 0;
+#pragma unroll
+    for (int j = 0; j < (NW + 3) / 4; ++j) c4[j] = 0;
+#pragma unroll
+    for (int j = 0; j < NW; ++j) ed[j] = 0;
+    auto empty = [&]() {
+#pragma unroll
+        for (int j = 0; j < NW; ++j) {
+            const uint32_t n = (c4[j / 4] >> (8 * (j % 4))) & 0xFFu;
+            if (s0 + j < S && n) {
+                atomicAdd(s_cnt + s0 + j, n);
+                atomicAdd(s_edges + s0 + j, (unsigned long long)ed[j]);
+            }
+            ed[j] = 0;
+        }
+#pragma unroll
+        for (int j = 0; j < (NW + 3) / 4; ++j) c4[j] = 0;
+        since = 0;
+        held = 0;
+    };
+    const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarp = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t base = warp0 * GPW; base < V; base += nwarp * GPW) {
+        const uint32_t mine = base + lane / NW;
+        const bool in = mine < V;
+        const size_t w = (size_t)mine * NW + lane % NW;
+        uint32_t deg = in ? __ldg(off + mine + 1) - __ldg(off + mine) : 0u;
+        uint32_t found = 0, plane[kPlanes];
+#pragma unroll
+        for (int p = 0; p < kPlanes; ++p) plane[p] = 0;
+#pragma unroll
+        for (int L0 = 0; L0 < kLevels; L0 += 8) {
+            if (L0 && (uint32_t)L0 >= lv.n) break;
+            uint32_t m[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) m[q] = in && (uint32_t)(L0 + q) < lv.n ? __ldg(lv.m[L0 + q] + w) : 0u;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const uint32_t fresh = m[q] & ~found;
+                found |= m[q];
+                at_level[L0 + q] |= fresh;
+#pragma unroll
+                for (int p = 0; p < kPlanes; ++p)
+                    if (((L0 + q) >> p) & 1) plane[p] |= fresh;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < GPW; ++i) {
+            const uint32_t v = base + i;
+            if (v >= V) break;
+            const uint32_t d = __shfl_sync(0xffffffffu, deg, i * NW);
+            uint32_t bits[kPlanes], reached = 0;
+#pragma unroll
+            for (int p = 0; p < kPlanes; ++p) {
+                bits[p] = (__shfl_sync(0xffffffffu, plane[p], i * NW + word) >> sh) & bmask;
+                reached |= bits[p];  // level 1 or more
+            }
+            if (held + d > 0xFFFFFFFFull || since == 255) empty();
+            held += d;
+            ++since;
+            uint32_t lvl[NW];
+#pragma unroll
+            for (int j = 0; j < NW; j += 4) {
+                // four sources' bits to the low bits of four bytes
+                uint32_t bytes = 0;
+#pragma unroll
+                for (int p = 0; p < kPlanes; ++p)
+                    bytes |= ((((bits[p] >> j) & 15u) * 0x00204081u) & 0x01010101u) << p;
+                c4[j / 4] += (((reached >> j) & 15u) * 0x00204081u) & 0x01010101u;
+#pragma unroll
+                for (int q = 0; q < 4 && j + q < NW; ++q) lvl[j + q] = (bytes >> (8 * q)) & 0xFFu;
+            }
+#pragma unroll
+            for (int j = 0; j < NW; ++j) ed[j] += (reached >> j) & 1u ? d : 0u;
+            uint32_t *row = dist + (size_t)v * S + s0;
+            if (NW % 4 == 0 && vec_rows && s0 + NW <= S) {
+#pragma unroll
+                for (int q = 0; q < NW / 4; ++q)
+                    reinterpret_cast<uint4 *>(row)[q] =
+                        make_uint4(lvl[4 * q], lvl[(4 * q + 1) % NW], lvl[(4 * q + 2) % NW], lvl[(4 * q + 3) % NW]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < NW; ++j)
+                    if (s0 + j < S) row[j] = lvl[j];
+            }
+        }
+    }
+    empty();
+    // the deepest level that reached anything, per source
+#pragma unroll
+    for (int L = 1; L < kLevels; ++L)
+        for (uint32_t m = at_level[L]; m; m &= m - 1) atomicMax(s_depth + 32 * (lane % NW) + __ffs(m) - 1, (uint32_t)L);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < S; i += blockDim.x) {
         // block 0 adds each source's own out-edges
@@ -446,12 +623,12 @@ int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, 
             GBX_LAUNCH_CHECK();
             ++pushes;
         } else {
-            ms_pull_light_kernel<NW><<<grid, kMsThreads, 0, s>>>(g->pull_offsets(), g->pull_src(), V, S, F, seen.p,
-                                                                 Fn);
+            ms_pull_light_kernel<NW><<<grid, kMsThreads, 0, s>>>(g->pull_offsets(), g->pull_src(), V, S, cnt.p, F,
+                                                                 seen.p, Fn);
             GBX_LAUNCH_CHECK();
             if (plan->n_chunks) {
                 ms_pull_heavy_kernel<NW><<<grid, kMsThreads, 0, s>>>(plan->chunks, plan->n_chunks, g->pull_src(), S,
-                                                                     F, seen.p, Fn);
+                                                                     cnt.p, F, seen.p, Fn);
                 GBX_LAUNCH_CHECK();
             }
             ++pulls;
@@ -485,8 +662,14 @@ int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, 
     GBX_CUDA(cudaMemsetAsync(rd.p, 0, 4 * (size_t)S, s));
     GBX_CUDA(cudaMemsetAsync(re.p, 0, 8 * (size_t)S, s));
     const bool vec_rows = S % 4 == 0 && (reinterpret_cast<uintptr_t>(dist) & 15u) == 0;
-    ms_final_kernel<NW><<<(unsigned)num_sms() * 4, kMsThreads, 0, s>>>(lv, seen.p, V, S, g->offsets, src_d,
-                                                                       vec_rows, dist, rc.p, re.p, rd.p);
+    const unsigned fgrid = std::min<unsigned>((unsigned)num_sms() * 6, ceil_div((uint64_t)V * NW, kMsThreads));
+    if (stored == level + 1 && stored <= 8)
+        ms_planes_kernel<NW, 3><<<fgrid, kMsThreads, 0, s>>>(lv, V, S, g->offsets, src_d, vec_rows, dist, rc.p, re.p, rd.p);
+    else if (stored == level + 1 && stored <= 16)
+        ms_planes_kernel<NW, 4><<<fgrid, kMsThreads, 0, s>>>(lv, V, S, g->offsets, src_d, vec_rows, dist, rc.p, re.p, rd.p);
+    else
+        ms_final_kernel<NW><<<(unsigned)num_sms() * 4, kMsThreads, 0, s>>>(lv, seen.p, V, S, g->offsets, src_d,
+                                                                           vec_rows, dist, rc.p, re.p, rd.p);
     GBX_LAUNCH_CHECK();
     if (res_host) {
         std::vector<uint32_t> hc(S), hd(S);
