@@ -91,9 +91,9 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-__device__ __forceinline__ void trace_step(BfsState *st, unsigned kind, unsigned value,
+__device__ __forceinline__ void trace_step(Team team, BfsState *st, unsigned kind, unsigned value,
                                            const BfsStep *step = nullptr) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && st->ntrace < kTraceMax) {
+    if (team.leader() && st->ntrace < kTraceMax) {
         TraceRec &r = st->trace[st->ntrace++];
         r.kind = kind;
         r.value = value;
@@ -223,7 +223,7 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t r) {
     return pos;
 }
 
-__device__ void top_down_phase(const BfsArgs &a, const uint32_t *qin, uint32_t qn, const uint32_t *hvin,
+__device__ void top_down_phase(const BfsArgs &a, Team team, const uint32_t *qin, uint32_t qn, const uint32_t *hvin,
                                const uint32_t *hcin, uint32_t nh, uint32_t nc, BfsStep *cur, uint32_t *qout,
                                uint32_t *hvout, uint32_t *hcout, uint32_t lnext, uint32_t *fbm, uint32_t *clear_bm,
                                uint32_t *s_pre, uint32_t *s_base, uint32_t *s_v, uint32_t *s_wq) {
@@ -231,7 +231,7 @@ __device__ void top_down_phase(const BfsArgs &a, const uint32_t *qin, uint32_t q
     BusyClock clock(a.trace != 0);
     if (clear_bm) {
         // the bitmap the next top-down step fills (not read during this one)
-        for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < a.words; w += gridDim.x * blockDim.x)
+        for (uint32_t w = team.thread(); w < a.words; w += team.threads())
             clear_bm[w] = 0u;
     }
     Claimer claim(a, lnext, qout, hvout, hcout, fbm, cur, s_wq);
@@ -243,12 +243,12 @@ __device__ void top_down_phase(const BfsArgs &a, const uint32_t *qin, uint32_t q
     // then not one warp's serial chain); the group parts are dealt first,
     // the hub chunks after them.
     const uint32_t groups = (qn + 31) / 32;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t nwarps = team.threads() >> 5;
     const uint32_t split = groups ? max(1u, min(kTdMaxSplit, nwarps / groups)) : 1u;
     const uint32_t hsplit = nc ? max(1u, min(kHubChunk / 128, nwarps / nc)) : 1u;
     const uint32_t gunits = groups * split;
     const uint32_t units = gunits + nc * hsplit;
-    UnitDealer dealer(&cur->cursor);
+    UnitDealer dealer(&cur->cursor, team);
     for (;;) {
         const uint32_t unit = dealer.take(units);
         if (unit >= units) break;
@@ -368,7 +368,7 @@ __device__ __forceinline__ uint32_t bu_probe(const BfsArgs &a, const uint32_t *c
 // next-frontier word of every word of the unit (zero when nothing was
 // found). Found vertices are also appended to the next generation's queue /
 // hub list, so leaving bottom-up needs no bitmap-to-list pass.
-__device__ void bottom_up_phase(const BfsArgs &a, const uint32_t *cur_bm, uint32_t *next_bm, uint32_t lnext,
+__device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur_bm, uint32_t *next_bm, uint32_t lnext,
                                 BfsStep *cnt, uint32_t *qout, uint32_t *hvout, uint32_t *hcout, uint32_t *s_wq,
                                 uint32_t *s_found) {
     const uint32_t lane = threadIdx.x & 31;
@@ -377,7 +377,7 @@ __device__ void bottom_up_phase(const BfsArgs &a, const uint32_t *cur_bm, uint32
     unsigned long long edges = 0;
     WarpQueue wq(s_wq);
     const uint32_t units = (a.words + kBuWords - 1) / kBuWords;
-    UnitDealer dealer(&cnt->cursor);
+    UnitDealer dealer(&cnt->cursor, team);
     for (uint32_t unit = dealer.take(units); unit < units; unit = dealer.take(units)) {
         const uint32_t w0 = unit * kBuWords;
         const uint32_t nw = min(a.words - w0, kBuWords);
@@ -502,19 +502,19 @@ __device__ void bottom_up_phase(const BfsArgs &a, const uint32_t *cur_bm, uint32
 // bitmap that is still all zero: the queue and hub lists hold every frontier
 // vertex with out-degree > 0, and the caller checks that the others cannot
 // matter (no other frontier vertex, or no pull neighbour of out-degree 0).
-__device__ void lists_to_bitmap_phase(const uint32_t *qin, uint32_t qn, const uint32_t *hvin, uint32_t nh,
+__device__ void lists_to_bitmap_phase(Team team, const uint32_t *qin, uint32_t qn, const uint32_t *hvin, uint32_t nh,
                                       uint32_t *bm) {
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    const uint32_t tid = team.thread(), nt = team.threads();
     for (uint32_t i = tid; i < qn + nh; i += nt) {
         const uint32_t v = i < qn ? __ldcg(qin + i) : __ldcg(hvin + (i - qn));
         atomicOr(bm + (v >> 5), 1u << (v & 31));
     }
 }
 
-__device__ void level_to_bitmap_phase(const BfsArgs &a, uint32_t l, uint32_t *bm) {
+__device__ void level_to_bitmap_phase(const BfsArgs &a, Team team, uint32_t l, uint32_t *bm) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t gw = team.thread() >> 5;
+    const uint32_t nw = team.threads() >> 5;
     for (uint32_t w0 = gw; w0 < a.words; w0 += 4 * nw) {
         uint32_t lv[4];
 #pragma unroll
@@ -544,7 +544,59 @@ __device__ __forceinline__ void zero_step(BfsStep *s) {
     s->busy_max = 0;
 }
 
-__global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs a) {
+// Per traversal: levels, parents, visited and both frontier bitmaps, the
+// traversal state (zeroed as 32-bit words by the grid), and the generation-0
+// lists: the source alone, as a hub when its degree is large. The state
+// words that hold those lists are written only by thread 0, after its own
+// share of the zeroing.
+__device__ __forceinline__ void bfs_init(uint32_t *level, int32_t *parent, uint32_t *visited, uint32_t *bm0,
+                                         uint32_t *bm1, uint32_t V, uint32_t words, uint32_t source,
+                                         const uint32_t *outdeg, uint32_t *q0, uint32_t *hv0, uint32_t *hc0,
+                                         BfsState *st, Team team) {
+    const uint32_t tid = team.thread(), nt = team.threads();
+    for (uint32_t v = tid; v < V; v += nt) {
+        // the reference's values for unreached vertices (BFS.c:59-74); the
+        // traversal overwrites the reached ones
+        const uint32_t d = __ldg(outdeg + v);
+        level[v] = 0u;
+        parent[v] = v == source ? (int32_t)source : (d ? -(int32_t)d : -1);
+    }
+    for (uint32_t w = tid; w < words; w += nt) {
+        visited[w] = (w == (source >> 5)) ? (1u << (source & 31)) : 0u;
+        bm0[w] = 0;
+        bm1[w] = 0;
+    }
+    static_assert(sizeof(BfsState) % 4 == 0, "state is zeroed as words");
+    constexpr uint32_t kStateWords = sizeof(BfsState) / 4;
+    uint32_t *sw = reinterpret_cast<uint32_t *>(st);
+    const uint32_t conv_lo = (uint32_t)(offsetof(BfsState, conv) / 4);
+    const uint32_t conv_hi = conv_lo + (uint32_t)(sizeof(BfsStep) / 4);
+    for (uint32_t i = tid; i < kStateWords; i += nt)
+        if (i < conv_lo || i >= conv_hi) sw[i] = 0u;
+    if (tid == 0) {
+        const uint32_t d = outdeg[source];
+        BfsStep c = {};
+        if (d > kHubDeg) {
+            hv0[0] = source;
+            hc0[0] = 0;
+            c.hub = (1ull << 32) | hub_chunks(d);
+        } else if (d > 0) {
+            q0[0] = source;
+            c.qlen = 1;
+        }
+        st->conv = c;
+    }
+}
+
+__global__ void bfs_init_kernel(uint32_t *level, int32_t *parent, uint32_t *visited, uint32_t *bm0,
+                                uint32_t *bm1, uint32_t V, uint32_t words, uint32_t source,
+                                const uint32_t *outdeg, uint32_t *q0, uint32_t *hv0, uint32_t *hc0,
+                                BfsState *st) {
+    bfs_init(level, parent, visited, bm0, bm1, V, words, source, outdeg, q0, hv0, hc0, st, whole_grid());
+}
+
+// One traversal by a team, whose barrier is gs.
+__device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSync *gs) {
     __shared__ uint32_t s_pre[kBfsWarps][33];
     __shared__ uint32_t s_base[kBfsWarps][32];
     __shared__ uint32_t s_v[kBfsWarps][32];
@@ -553,7 +605,6 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
     __shared__ BfsStep s_cnt;  // the finished step's counters (fetch_counters)
     const uint32_t wid = threadIdx.x >> 5;
     BfsState *st = a.st;
-    grid_barrier_init();
     const uint32_t alpha = a.alpha, beta = a.beta;
     // DO bookkeeping, evaluated identically by every CTA
     uint32_t mu = a.E, mf = __ldg(a.outdeg + a.source), qsize = 1, nf_prev = 0, L = 0;
@@ -571,14 +622,14 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
     uint32_t qn = __ldcg(&st->conv.qlen);
     unsigned long long hub0 = __ldcg(&st->conv.hub);
     uint32_t nh = (uint32_t)(hub0 >> 32), nc = (uint32_t)hub0;
-    trace_step(st, kTrStart, 1);
+    trace_step(team, st, kTrStart, 1);
     for (uint32_t s = 0; !done; ++s) {
         if (s >= max_steps) {
             failed = true;
             break;
         }
         BfsStep *cur = &st->step[s % 3];
-        if (blockIdx.x == 0 && threadIdx.x == 0) zero_step(&st->step[(s + 1) % 3]);
+        if (team.leader()) zero_step(&st->step[(s + 1) % 3]);
         const uint32_t ib = s & 1, ob = ib ^ 1;
         bool use_bu;
         if (a.mode == 0) {
@@ -597,24 +648,24 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
                     // scattered from the lists when they hold the whole frontier
                     // and the bitmap is still clear, else from level[]
                     if (bm_clean[ib] && (a.pull_live || qsize == qn + nh))
-                        lists_to_bitmap_phase(a.q[ib], qn, a.hv[ib], nh, a.bm[ib]);
+                        lists_to_bitmap_phase(team, a.q[ib], qn, a.hv[ib], nh, a.bm[ib]);
                     else
-                        level_to_bitmap_phase(a, L, a.bm[ib]);
-                    if (!grid_barrier(&st->gs)) { failed = true; break; }
-                    trace_step(st, kTrToBitmap, qsize);
+                        level_to_bitmap_phase(a, team, L, a.bm[ib]);
+                    if (!grid_barrier(gs, team.ctas)) { failed = true; break; }
+                    trace_step(team, st, kTrToBitmap, qsize);
                 }
                 bm_clean[ib] = false;
                 bm_track = bm_ready = false;
                 nf_prev = qsize;
                 in_bu = true;
             }
-            bottom_up_phase(a, a.bm[ib], a.bm[ob], L + 1, cur, a.q[ob], a.hv[ob], a.hc[ob], s_wq[wid],
+            bottom_up_phase(a, team, a.bm[ib], a.bm[ob], L + 1, cur, a.q[ob], a.hv[ob], a.hc[ob], s_wq[wid],
                             s_found[wid]);
             bm_clean[ob] = false;
-            if (!grid_barrier(&st->gs)) { failed = true; break; }
+            if (!grid_barrier(gs, team.ctas)) { failed = true; break; }
             fetch_counters(cur, &s_cnt);
             const uint32_t nf = s_cnt.nf;
-            trace_step(st, kTrBottomUp, nf, cur);
+            trace_step(team, st, kTrBottomUp, nf, cur);
             processed += nf;
             iteration++;
             bu++;
@@ -641,7 +692,7 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
             mu -= mf;
             // bm[ob] is clear here while tracking: bfs_init_kernel cleared both
             // bitmaps, and each tracking step clears bm[ib] for the next one
-            top_down_phase(a, a.q[ib], qn, a.hv[ib], a.hc[ib], nh, nc, cur, a.q[ob], a.hv[ob], a.hc[ob], L + 1,
+            top_down_phase(a, team, a.q[ib], qn, a.hv[ib], a.hc[ib], nh, nc, cur, a.q[ob], a.hv[ob], a.hc[ob], L + 1,
                            bm_track ? a.bm[ob] : nullptr, bm_track && s > 0 ? a.bm[ib] : nullptr, s_pre[wid],
                            s_base[wid], s_v[wid], s_wq[wid]);
             if (bm_track) {
@@ -649,10 +700,10 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
                 bm_clean[ib] = true;
                 bm_ready = true;
             }
-            if (!grid_barrier(&st->gs)) { failed = true; break; }
+            if (!grid_barrier(gs, team.ctas)) { failed = true; break; }
             fetch_counters(cur, &s_cnt);
             const uint32_t nf = s_cnt.nf;
-            trace_step(st, kTrTopDown, nf, cur);
+            trace_step(team, st, kTrTopDown, nf, cur);
             mf = s_cnt.mf;
             qsize = nf;
             processed += nf;
@@ -667,7 +718,7 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
             if (qsize == 0) done = true;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (team.leader()) {
         st->processed = processed;
         st->iteration = iteration;
         st->td_steps = td;
@@ -684,8 +735,81 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
             o.depth = L;
             o.edges_total = edges_total;
             o.status = failed ? 1u : 0u;
-            o.timeout = ld_acquire_u32(&st->gs.error);
+            o.timeout = ld_acquire_u32(&gs->error);
         }
+    }
+}
+
+__global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs a) {
+    grid_barrier_init();
+    bfs_traverse(a, whole_grid(), &a.st->gs);
+}
+
+// ---- several traversals at once ----------------------------------------------
+// A traversal leaves most of the GPU waiting: with every SM on one RMAT-22
+// traversal DRAM runs at 14% and the issue slots at 22%, and what a step waits
+// for -- its barrier, the counters, dependent loads, its slowest unit -- does
+// not get shorter with more SMs. So trials with outputs of their own are taken
+// by teams of CTAs: one cooperative grid, a traversal per team with its own
+// working arrays and its own barrier, the next trial from a counter when one
+// is done. A team also writes its trial's initial state, which is a kernel of
+// its own otherwise. 8 trials: RMAT-22 (64M edges) 1,430 us one after the
+// other, 775 by eight teams; 250,000 vertices and 3M edges 543, 138.
+struct BfsTeams {
+    BfsArgs first;            // team 0's working arrays; level / parent: its own, unless given below
+    size_t pitch;             // bytes from one team's working arrays to the next's
+    uint32_t ctas;            // per team
+    uint32_t n;               // trials
+    const uint32_t *sources;  // device
+    uint32_t *level;          // trial i at level + i * stride, or null
+    int32_t *parent;
+    uint64_t stride;
+    BfsSlot *slots;
+    struct Control {
+        GridSync gs;
+        unsigned next;  // the team's next trial
+        unsigned pad[11];
+    } *teams;
+    unsigned *queue;  // trials taken after the teams' first ones
+};
+
+template <class T>
+__device__ __forceinline__ T *at_bytes(T *p, size_t bytes) {
+    return reinterpret_cast<T *>(reinterpret_cast<char *>(p) + bytes);
+}
+
+__global__ void __launch_bounds__(kBfsThreads, 1) bfs_teams_kernel(BfsTeams t) {
+    __shared__ BfsArgs a;
+    const uint32_t mine = blockIdx.x / t.ctas, count = gridDim.x / t.ctas;
+    const Team team{blockIdx.x - mine * t.ctas, t.ctas};
+    BfsTeams::Control *ctl = t.teams + mine;
+    grid_barrier_init();
+    for (uint32_t trial = mine; trial < t.n;) {
+        if (threadIdx.x == 0) {
+            const size_t skip = mine * t.pitch;
+            a = t.first;
+            a.source = __ldg(t.sources + trial);
+            a.level = t.level ? t.level + trial * t.stride : at_bytes(a.level, skip);
+            a.parent = t.parent ? t.parent + trial * t.stride : at_bytes(a.parent, skip);
+            a.visited = at_bytes(a.visited, skip);
+            for (int i = 0; i < 2; ++i) {
+                a.bm[i] = at_bytes(a.bm[i], skip);
+                a.q[i] = at_bytes(a.q[i], skip);
+                a.hv[i] = at_bytes(a.hv[i], skip);
+                a.hc[i] = at_bytes(a.hc[i], skip);
+            }
+            a.st = at_bytes(a.st, skip);
+            a.slot = t.slots + trial;
+        }
+        __syncthreads();
+        bfs_init(a.level, a.parent, a.visited, a.bm[0], a.bm[1], a.V, a.words, a.source, a.outdeg, a.q[0], a.hv[0],
+                 a.hc[0], a.st, team);
+        if (!grid_barrier(&ctl->gs, team.ctas)) return;
+        bfs_traverse(a, team, &ctl->gs);
+        // nobody writes the next trial's state before all have left this one's
+        if (team.leader()) ctl->next = count + atomicAdd(t.queue, 1u);
+        if (!grid_barrier(&ctl->gs, team.ctas)) return;
+        trial = __ldcg(&ctl->next);
     }
 }
 
@@ -913,50 +1037,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     }
 }
 
-// Per traversal: levels, parents, visited and both frontier bitmaps, the
-// traversal state (zeroed as 32-bit words by the grid), and the generation-0
-// lists: the source alone, as a hub when its degree is large. The state
-// words that hold those lists are written only by thread 0, after its own
-// share of the zeroing.
-__global__ void bfs_init_kernel(uint32_t *level, int32_t *parent, uint32_t *visited, uint32_t *bm0,
-                                uint32_t *bm1, uint32_t V, uint32_t words, uint32_t source,
-                                const uint32_t *outdeg, uint32_t *q0, uint32_t *hv0, uint32_t *hc0,
-                                BfsState *st) {
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-    for (uint32_t v = tid; v < V; v += nt) {
-        // the reference's values for unreached vertices (BFS.c:59-74); the
-        // traversal overwrites the reached ones
-        const uint32_t d = __ldg(outdeg + v);
-        level[v] = 0u;
-        parent[v] = v == source ? (int32_t)source : (d ? -(int32_t)d : -1);
-    }
-    for (uint32_t w = tid; w < words; w += nt) {
-        visited[w] = (w == (source >> 5)) ? (1u << (source & 31)) : 0u;
-        bm0[w] = 0;
-        bm1[w] = 0;
-    }
-    static_assert(sizeof(BfsState) % 4 == 0, "state is zeroed as words");
-    constexpr uint32_t kStateWords = sizeof(BfsState) / 4;
-    uint32_t *sw = reinterpret_cast<uint32_t *>(st);
-    const uint32_t conv_lo = (uint32_t)(offsetof(BfsState, conv) / 4);
-    const uint32_t conv_hi = conv_lo + (uint32_t)(sizeof(BfsStep) / 4);
-    for (uint32_t i = tid; i < kStateWords; i += nt)
-        if (i < conv_lo || i >= conv_hi) sw[i] = 0u;
-    if (tid == 0) {
-        const uint32_t d = outdeg[source];
-        BfsStep c = {};
-        if (d > kHubDeg) {
-            hv0[0] = source;
-            hc0[0] = 0;
-            c.hub = (1ull << 32) | hub_chunks(d);
-        } else if (d > 0) {
-            q0[0] = source;
-            c.qlen = 1;
-        }
-        st->conv = c;
-    }
-}
-
 // live[w] bit b: vertex 32w + b exists and has pull in-edges
 __global__ void live_bits_kernel(const uint32_t *poff, uint32_t V, uint32_t words, uint32_t *live) {
     const uint32_t lane = threadIdx.x & 31;
@@ -1071,9 +1151,33 @@ BfsArgs bfs_args(const gbx_graph *g, const BfsWork &w, int mode, uint32_t *lev, 
     return a;
 }
 
-// n traversals of g that may run at once are taken by bfs_small_kernel
+// n traversals of g that may run at once are taken by bfs_small_kernel. One CTA
+// per trial against teams, us for 8 R-MAT trials: 80k edges 75 / 108, 160k
+// 104 / 114, 320k 159 / 119; for 64: 192k 153 / 174; for 2: 96k 66 / 93.
 bool bfs_is_small(const gbx_graph *g, uint32_t n) {
-    return (g->V + 31) / 32 <= kSmallWords && g->E <= (uint64_t)kSmallEdges * std::min(n, 8u) && !trace_enabled();
+    return (g->V + 31) / 32 <= kSmallWords && g->E <= (uint64_t)kSmallEdges * std::min(n, 3u) && !trace_enabled();
+}
+
+// Teams for several traversals of g at once. More teams wait for less, until
+// their frontiers and outputs push one another out of the L2 or a step is too
+// much work for a team's few SMs: each factor of four in edges halves the
+// count. us for 8 (first four) or 64 R-MAT trials with 1 / 4 / 8 / 16 / 32 / 64 teams:
+//   edges 144M   2609 / 2240 / 2504
+//          96M   2049 / 1400 / 1553
+//          64M   1430 /  864 /  775
+//          12M    806 /  311 /  271
+//      64: 48M      - / 6053 / 5513 / 5804 / 7048 / 7852
+//          12M      - / 2031 / 1570 / 1471 / 1699 / 1870
+//           3M      - / 1233 /  788 /  595 /  537 /  538
+//         770K      - / 1014 /  575 /  374 /  284 /  246
+// The teams' working arrays are held to kTeamsBytes.
+constexpr uint32_t kMaxTeams = 64, kMinTeams = 4;
+constexpr uint64_t kMaxTeamsEdges = 1'250'000;
+constexpr size_t kTeamsBytes = size_t(4) << 30;
+uint32_t bfs_team_count(const gbx_graph *g, size_t pitch) {
+    uint32_t teams = kMaxTeams;
+    for (uint64_t e = kMaxTeamsEdges; teams > kMinTeams && std::max<uint64_t>(g->E, (uint64_t)g->V * 8) > e; e *= 4) teams /= 2;
+    return (uint32_t)std::min<size_t>(teams, kTeamsBytes / pitch);
 }
 
 // n <= kSmallBatch traversals, one CTA each, outputs `stride` entries apart
@@ -1103,6 +1207,53 @@ int bfs_enqueue(gbx_graph *g, const BfsWork &w, uint32_t source, int mode, uint3
     void *args[] = {&a};
     GBX_CUDA(cudaLaunchCooperativeKernel((const void *)bfs_persistent_kernel, grid, kBfsThreads, args, 0, s));
     GBX_LAUNCH_CHECK();
+    return GBX_OK;
+}
+
+// n traversals by teams of CTAs, each trial writing outputs of its own (or none).
+// *done stays false where there is no memory for the teams' working arrays.
+int bfs_enqueue_teams(gbx_graph *g, const uint32_t *sources, uint32_t n, int mode, uint32_t *distances,
+                      int32_t *parents, uint64_t stride, BfsSlot *slots, cudaStream_t s, bool *done) {
+    int grid = 0;
+    static int grid_cache[64] = {0};
+    GBX_TRY(coop_grid(bfs_teams_kernel, kBfsThreads, 0, &grid, &grid_cache));
+    const size_t pitch = BfsWork::bytes(g->V, false);
+    const uint32_t teams = std::min(std::min(n, (uint32_t)grid), bfs_team_count(g, pitch));
+    if (teams < 2) return GBX_OK;
+    DevBuf<char> work;
+    DevBuf<uint32_t> src;
+    DevBuf<BfsTeams::Control> ctl;  // the last one's first word: the queue
+    if (work.alloc(teams * pitch, s) != GBX_OK) {
+        clear_error();
+        return GBX_OK;
+    }
+    GBX_TRY(src.alloc(n, s));
+    GBX_TRY(ctl.alloc(teams + 1, s));
+    GBX_CUDA(cudaMemsetAsync(ctl.p, 0, (teams + 1) * sizeof(BfsTeams::Control), s));
+    GBX_CUDA(cudaMemsetAsync(slots, 0xff, n * sizeof(BfsSlot), s));  // a trial that is never reached counts as timed out
+    GBX_CUDA(cudaMemcpyAsync(src.p, sources, (size_t)n * 4, cudaMemcpyHostToDevice, s));
+    Scratch carve;  // over the first team's part
+    carve.base = work.p;
+    carve.cap = pitch;
+    BfsWork w;
+    GBX_TRY(w.carve(carve, g->V, false));
+    BfsTeams t{};
+    t.first = bfs_args(g, w, mode, w.level, w.parent, nullptr);
+    t.pitch = pitch;
+    t.ctas = (uint32_t)grid / teams;
+    t.n = n;
+    t.sources = src.p;
+    t.level = distances;
+    t.parent = parents;
+    t.stride = stride;
+    t.slots = slots;
+    t.teams = ctl.p;
+    t.queue = reinterpret_cast<unsigned *>(ctl.p + teams);
+    void *args[] = {&t};
+    GBX_CUDA(cudaLaunchCooperativeKernel((const void *)bfs_teams_kernel, dim3(t.ctas * teams), dim3(kBfsThreads), args, 0,
+                                         s));
+    GBX_LAUNCH_CHECK();
+    *done = true;
     return GBX_OK;
 }
 
@@ -1239,9 +1390,12 @@ extern "C" int gbx_bfs_trials(gbx_graph *g, const uint32_t *sources, uint32_t nu
                              slots.p + i);
         GBX_TRY(bfs_enqueue_small(a, sources + i, std::min(kSmallBatch, num_sources - i), out_stride, s));
     }
+    bool by_teams = false;
+    if (!at_once && !copies.cs && num_sources > 1 && (out_stride || (!distances && !parents)) && !trace_enabled())
+        GBX_TRY(bfs_enqueue_teams(g, sources, num_sources, mode, distances, parents, out_stride, slots.p, s, &by_teams));
     // every traversal re-initialises the shared work arrays on the stream, so
     // the traversals run back to back without the host in between
-    for (uint32_t i = 0; !at_once && i < num_sources; ++i) {
+    for (uint32_t i = 0; !at_once && !by_teams && i < num_sources; ++i) {
         const uint32_t b = i & 1;
         const size_t off = (size_t)i * out_stride;
         uint32_t *lev = dist_host ? dstage.p + (size_t)b * V : distances ? distances + off : w.level;

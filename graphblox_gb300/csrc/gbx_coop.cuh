@@ -48,12 +48,23 @@ __device__ __forceinline__ void grid_barrier_init() {
     if (threadIdx.x == 0) s_grid_target = 0;
 }
 
-// Returns false when the grid must stop (a wait expired somewhere).
-__device__ __forceinline__ bool grid_barrier(GridSync *gs) {
+// The CTAs that work on one thing: the whole grid, or one of several equal
+// teams of a cooperative grid, each with a GridSync of its own (all CTAs are
+// resident, so a team's wait ends like the grid's).
+struct Team {
+    uint32_t cta, ctas;
+    __device__ __forceinline__ uint32_t thread() const { return cta * blockDim.x + threadIdx.x; }
+    __device__ __forceinline__ uint32_t threads() const { return ctas * blockDim.x; }
+    __device__ __forceinline__ bool leader() const { return cta == 0 && threadIdx.x == 0; }
+};
+__device__ __forceinline__ Team whole_grid() { return Team{blockIdx.x, gridDim.x}; }
+
+// Returns false when the team must stop (a wait expired somewhere).
+__device__ __forceinline__ bool grid_barrier(GridSync *gs, uint32_t ctas = gridDim.x) {
     __shared__ unsigned s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned long long target = s_grid_target + gridDim.x;
+        const unsigned long long target = s_grid_target + ctas;
         s_grid_target = target;
         asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&gs->arrived) : "memory");
         unsigned ok = 1, spins = 0;
@@ -126,14 +137,14 @@ struct WarpQueue {
 struct UnitDealer {
     unsigned *cursor;
     uint32_t ticket;  // lane 0: reply of the increment in flight
-    uint32_t nwarps;
+    uint32_t nwarps, warp;
     bool first;
-    __device__ __forceinline__ UnitDealer(unsigned *c)
-        : cursor(c), ticket(0), nwarps((gridDim.x * blockDim.x) >> 5), first(true) {}
+    __device__ __forceinline__ UnitDealer(unsigned *c, Team t = whole_grid())
+        : cursor(c), ticket(0), nwarps(t.threads() >> 5), warp(t.thread() >> 5), first(true) {}
     __device__ __forceinline__ uint32_t take(uint32_t units) {
         uint32_t u;
         if (first) {
-            u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+            u = warp;
             first = false;
         } else {
             u = nwarps + __shfl_sync(0xffffffffu, ticket, 0);
