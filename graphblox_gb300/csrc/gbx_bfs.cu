@@ -749,19 +749,19 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
 // A traversal leaves most of the GPU waiting: with every SM on one RMAT-22
 // traversal DRAM runs at 14% and the issue slots at 22%, and what a step waits
 // for -- its barrier, the counters, dependent loads, its slowest unit -- does
-// not get shorter with more SMs. So trials with outputs of their own are taken
-// by teams of CTAs: one cooperative grid, a traversal per team with its own
+// not get shorter with more SMs. So trials that leave their outputs on the
+// device are taken by teams of CTAs: one cooperative grid, a traversal per team with its own
 // working arrays and its own barrier, the next trial from a counter when one
 // is done. A team also writes its trial's initial state, which is a kernel of
 // its own otherwise. 8 trials: RMAT-22 (64M edges) 1,430 us one after the
 // other, 775 by eight teams; 250,000 vertices and 3M edges 543, 138.
 struct BfsTeams {
-    BfsArgs first;            // team 0's working arrays; level / parent: its own, unless given below
+    BfsArgs first;            // team 0's working arrays; level / parent: its own, for trials without outputs
     size_t pitch;             // bytes from one team's working arrays to the next's
     uint32_t ctas;            // per team
     uint32_t n;               // trials
     const uint32_t *sources;  // device
-    uint32_t *level;          // trial i at level + i * stride, or null
+    uint32_t *level;          // trial i at level + i * stride (stride 0: the last trial's), or null
     int32_t *parent;
     uint64_t stride;
     BfsSlot *slots;
@@ -789,8 +789,9 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_teams_kernel(BfsTeams t) {
             const size_t skip = mine * t.pitch;
             a = t.first;
             a.source = __ldg(t.sources + trial);
-            a.level = t.level ? t.level + trial * t.stride : at_bytes(a.level, skip);
-            a.parent = t.parent ? t.parent + trial * t.stride : at_bytes(a.parent, skip);
+            const bool out = t.stride || trial == t.n - 1;
+            a.level = t.level && out ? t.level + trial * t.stride : at_bytes(a.level, skip);
+            a.parent = t.parent && out ? t.parent + trial * t.stride : at_bytes(a.parent, skip);
             a.visited = at_bytes(a.visited, skip);
             for (int i = 0; i < 2; ++i) {
                 a.bm[i] = at_bytes(a.bm[i], skip);
@@ -1210,7 +1211,7 @@ int bfs_enqueue(gbx_graph *g, const BfsWork &w, uint32_t source, int mode, uint3
     return GBX_OK;
 }
 
-// n traversals by teams of CTAs, each trial writing outputs of its own (or none).
+// n traversals by teams of CTAs, outputs (if any) in device memory.
 // *done stays false where there is no memory for the teams' working arrays.
 int bfs_enqueue_teams(gbx_graph *g, const uint32_t *sources, uint32_t n, int mode, uint32_t *distances,
                       int32_t *parents, uint64_t stride, BfsSlot *slots, cudaStream_t s, bool *done) {
@@ -1390,8 +1391,10 @@ extern "C" int gbx_bfs_trials(gbx_graph *g, const uint32_t *sources, uint32_t nu
                              slots.p + i);
         GBX_TRY(bfs_enqueue_small(a, sources + i, std::min(kSmallBatch, num_sources - i), out_stride, s));
     }
+    // (2 or 3 trials of a small graph into shared outputs: one CTA after the
+    // other is still faster than teams, 33 us a trial against 95 in all)
     bool by_teams = false;
-    if (!at_once && !copies.cs && num_sources > 1 && (out_stride || (!distances && !parents)) && !trace_enabled())
+    if (!at_once && !copies.cs && num_sources > (bfs_is_small(g, 1) ? 3u : 1u) && !trace_enabled())
         GBX_TRY(bfs_enqueue_teams(g, sources, num_sources, mode, distances, parents, out_stride, slots.p, s, &by_teams));
     // every traversal re-initialises the shared work arrays on the stream, so
     // the traversals run back to back without the host in between

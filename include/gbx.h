@@ -156,8 +156,8 @@ int gbx_bfs(gbx_graph *g, uint32_t source, int mode, uint32_t *distances, int32_
 /* The BFS trials of the reference's benchmark loop (runGraphAlgorithms,
  * graphRun.c:463-595: one breadthFirstSearchGraphCSR per trial, each from a
  * new root): one gbx_bfs traversal per source, enqueued back to back on
- * `stream` with a single host synchronisation after the last; trials that
- * write device memory of their own (or nothing) run several at once. sources and
+ * `stream` with a single host synchronisation after the last; without host
+ * outputs several trials run at once. sources and
  * results are host arrays of num_sources entries; results[i] is what gbx_bfs
  * returns for sources[i]. distances / parents: NULL, or device or host
  * arrays; with out_stride 0 every trial writes the same V entries (the last

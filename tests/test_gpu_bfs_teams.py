@@ -52,6 +52,9 @@ def test_trials_by_teams(gbx, cuda_device, name, n):
             levels_only = gbx.breadth_first_search_trials(dg, roots, mode, distances=only, out_stride=stride)
             bare = gbx.breadth_first_search_trials(dg, roots, mode)
             assert torch.equal(dist, only)
+            last = torch.full((V,), -7, dtype=torch.int32, device=cuda_device)
+            gbx.breadth_first_search_trials(dg, roots[::-1], mode, distances=last)
+            assert torch.equal(last, dist[:V])
             d_all, p_all = dist.cpu().numpy().reshape(n, stride), par.cpu().numpy().reshape(n, stride)
             assert np.all(d_all[:, V:] == -7) and np.all(p_all[:, V:] == -7)
             for i in sorted({0, 1, n // 2, n - 1}):
