@@ -11,7 +11,7 @@
 // generations of frontier lists: a queue of vertices with out-degree in
 // (0, kHubDeg] and a hub list for larger ones.
 //
-//  top-down  : warps take work units from an atomic cursor. A unit is either
+//  top-down  : warps take their CTA's work units in turn. A unit is either
 //              kHubChunk edges of one hub (hubs are cut so no warp serialises
 //              a hub's row) or 32 queued vertices whose edges the warp
 //              flattens (warp scan of degrees, consecutive lanes on
@@ -48,10 +48,10 @@ constexpr uint32_t kBuProbe = 64;     // bottom-up: in-edges a lane probes alone
 constexpr uint32_t kTdMaxSplit = 64;  // top-down: most warps sharing one 32-vertex group's edges
 constexpr uint32_t kBuWords = 8;      // bottom-up: frontier-bitmap words (32 vertices each) per work unit
 constexpr int kBfsThreads = 768;
+constexpr uint32_t kBfsQueueCap = 256;  // entries a warp stages (128: 171 us a traversal of RMAT-22, 256: 167)
 constexpr int kBfsWarps = kBfsThreads / 32;
 
 struct BfsStep {
-    unsigned cursor;          // work-unit cursor
     unsigned nf;              // vertices claimed
     unsigned mf;              // sum over claimed of max(out_degree, 1) (BFS.c:537)
     unsigned qlen;            // next queue length
@@ -138,6 +138,35 @@ struct BfsArgs {
 
 __device__ __forceinline__ uint32_t hub_chunks(uint32_t d) { return (d + kHubChunk - 1) / kHubChunk; }
 
+// End of a step's phase, all threads of the CTA: its warps' queues and sums
+// go out as one set of atomics per CTA (per warp they were up to 14,600 on one
+// sector, some 15 us of a step).
+__device__ __forceinline__ void step_flush(const WarpQueue &wq, uint32_t *qout, BfsStep *cnt, unsigned nf, unsigned mf,
+                                           unsigned long long edges) {
+    __shared__ unsigned s_nf, s_mf;
+    __shared__ unsigned long long s_edges;
+    if (threadIdx.x == 0) {
+        s_nf = s_mf = 0;
+        s_edges = 0;
+    }
+    __syncthreads();
+    nf = warp_sum(nf);
+    mf = warp_sum(mf);
+    edges = warp_sum(edges);
+    if ((threadIdx.x & 31) == 0 && nf) {
+        atomicAdd(&s_nf, nf);
+        atomicAdd(&s_mf, mf);
+        atomicAdd(&s_edges, edges);
+    }
+    const WarpQueue none(nullptr);
+    cta_flush(wq, qout, &cnt->qlen, none, nullptr, nullptr);
+    if (threadIdx.x == 0 && s_nf) {
+        atomicAdd(&cnt->nf, s_nf);
+        atomicAdd(&cnt->mf, s_mf);
+        atomicAdd(&cnt->edges, s_edges);
+    }
+}
+
 // Claim u (reached from v) at level lnext; all lanes call together.
 struct Claimer {
     const BfsArgs &a;
@@ -150,7 +179,7 @@ struct Claimer {
     unsigned long long edges = 0;
     __device__ __forceinline__ Claimer(const BfsArgs &a_, uint32_t l, uint32_t *q, uint32_t *hv, uint32_t *hc,
                                        uint32_t *f, BfsStep *c, uint32_t *wbuf)
-        : a(a_), lnext(l), qout(q), hvout(hv), hcout(hc), fbm(f), cnt(c), wq(wbuf) {}
+        : a(a_), lnext(l), qout(q), hvout(hv), hcout(hc), fbm(f), cnt(c), wq(wbuf, kBfsQueueCap) {}
     // Four candidate edges per lane: the visited-word loads and the
     // targets' out-degrees (needed only by the winners, but loading them
     // here takes them off the claim's dependent chain), then the atomicOr
@@ -180,33 +209,17 @@ struct Claimer {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const bool won = !(old[q] & (1u << (u[q] & 31)));
-            bool push = false;
             if (won) {
                 nf += 1;
                 mf += du[q] ? du[q] : 1u;
                 edges += du[q];
-                if (du[q] > kHubDeg) {
-                    unsigned long long h = atomicAdd(&cnt->hub, (1ull << 32) | hub_chunks(du[q]));
-                    uint32_t slot = (uint32_t)(h >> 32);
-                    hvout[slot] = u[q];
-                    hcout[slot] = (uint32_t)h;
-                } else {
-                    push = du[q] > 0;
-                }
             }
-            wq.push(u[q], push, qout, &cnt->qlen);
+            push_hubs(u[q], hub_chunks(du[q]), du[q] > kHubDeg, hvout, hcout, &cnt->hub);
+            wq.push(u[q], du[q] > 0 && du[q] <= kHubDeg, qout, &cnt->qlen);
         }
     }
-    __device__ __forceinline__ void flush() {
-        wq.flush(qout, &cnt->qlen);
-        unsigned n = warp_sum(nf), f = warp_sum(mf);
-        unsigned long long e = warp_sum(edges);
-        if ((threadIdx.x & 31) == 0 && n) {
-            atomicAdd(&cnt->nf, n);
-            atomicAdd(&cnt->mf, f);
-            atomicAdd(&cnt->edges, e);
-        }
-    }
+    // all threads of the CTA
+    __device__ __forceinline__ void flush() { step_flush(wq, qout, cnt, nf, mf, edges); }
 };
 
 // Position of the r-th set bit (from 0) of m; m has more than r set bits.
@@ -248,9 +261,9 @@ __device__ void top_down_phase(const BfsArgs &a, Team team, const uint32_t *qin,
     const uint32_t hsplit = nc ? max(1u, min(kHubChunk / 128, nwarps / nc)) : 1u;
     const uint32_t gunits = groups * split;
     const uint32_t units = gunits + nc * hsplit;
-    UnitDealer dealer(&cur->cursor, team);
+    UnitDealer dealer(team);
     for (;;) {
-        const uint32_t unit = dealer.take(units);
+        const uint32_t unit = dealer.take();
         if (unit >= units) break;
         if (unit >= gunits) {
             // kHubChunk edges of one hub (every hsplit-th batch of them)
@@ -375,10 +388,10 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
     BusyClock clock(a.trace != 0);
     unsigned nf = 0;
     unsigned long long edges = 0;
-    WarpQueue wq(s_wq);
+    WarpQueue wq(s_wq, kBfsQueueCap);
     const uint32_t units = (a.words + kBuWords - 1) / kBuWords;
-    UnitDealer dealer(&cnt->cursor, team);
-    for (uint32_t unit = dealer.take(units); unit < units; unit = dealer.take(units)) {
+    UnitDealer dealer(team);
+    for (uint32_t unit = dealer.take(); unit < units; unit = dealer.take()) {
         const uint32_t w0 = unit * kBuWords;
         const uint32_t nw = min(a.words - w0, kBuWords);
         // lane k < nw holds word w0 + k (only this warp writes these words in the step)
@@ -468,13 +481,8 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
             if (found) {
                 atomicOr(s_found + k, 1u << (v & 31));
                 edges += dv;
-                if (dv > kHubDeg) {
-                    const unsigned long long h = atomicAdd(&cnt->hub, (1ull << 32) | hub_chunks(dv));
-                    const uint32_t slot = (uint32_t)(h >> 32);
-                    hvout[slot] = v;
-                    hcout[slot] = (uint32_t)h;
-                }
             }
+            push_hubs(v, hub_chunks(dv), found && dv > kHubDeg, hvout, hcout, &cnt->hub);
             // the vertices found also form the next step's lists, in case the
             // traversal returns to top-down after this step (bitmapToArrayQueue)
             wq.push(v, found && dv > 0 && dv <= kHubDeg, qout, &cnt->qlen);
@@ -488,13 +496,7 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
         }
         __syncwarp();
     }
-    wq.flush(qout, &cnt->qlen);
-    nf = warp_sum(nf);
-    edges = warp_sum(edges);
-    if (lane == 0 && (nf || edges)) {
-        atomicAdd(&cnt->nf, nf);
-        atomicAdd(&cnt->edges, edges);
-    }
+    step_flush(wq, qout, cnt, nf, 0, edges);
     clock.stop(cnt);
 }
 
@@ -534,7 +536,6 @@ __device__ void level_to_bitmap_phase(const BfsArgs &a, Team team, uint32_t l, u
 }
 
 __device__ __forceinline__ void zero_step(BfsStep *s) {
-    s->cursor = 0;
     s->nf = 0;
     s->mf = 0;
     s->qlen = 0;
@@ -600,7 +601,7 @@ __device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSy
     __shared__ uint32_t s_pre[kBfsWarps][33];
     __shared__ uint32_t s_base[kBfsWarps][32];
     __shared__ uint32_t s_v[kBfsWarps][32];
-    __shared__ uint32_t s_wq[kBfsWarps][kWarpQueueCap];
+    __shared__ uint32_t s_wq[kBfsWarps][kBfsQueueCap];
     __shared__ uint32_t s_found[kBfsWarps][kBuWords];
     __shared__ BfsStep s_cnt;  // the finished step's counters (fetch_counters)
     const uint32_t wid = threadIdx.x >> 5;

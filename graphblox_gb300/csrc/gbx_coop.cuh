@@ -29,6 +29,8 @@ constexpr unsigned kBarrierSpinLimit = 1u << 22;
 
 // this CTA's arrival target for its next barrier (set by grid_barrier_init)
 __shared__ unsigned long long s_grid_target;
+// units of the current phase taken by this CTA's warps after their first ones (UnitDealer)
+__shared__ unsigned s_units_dealt;
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
     unsigned v;
@@ -42,10 +44,13 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
     return v;
 }
 
-// Once at kernel start, before the first grid_barrier (whose leading
-// __syncthreads orders it).
+// Once at kernel start, by all threads.
 __device__ __forceinline__ void grid_barrier_init() {
-    if (threadIdx.x == 0) s_grid_target = 0;
+    if (threadIdx.x == 0) {
+        s_grid_target = 0;
+        s_units_dealt = 0;
+    }
+    __syncthreads();
 }
 
 // The CTAs that work on one thing: the whole grid, or one of several equal
@@ -66,6 +71,7 @@ __device__ __forceinline__ bool grid_barrier(GridSync *gs, uint32_t ctas = gridD
     if (threadIdx.x == 0) {
         const unsigned long long target = s_grid_target + ctas;
         s_grid_target = target;
+        s_units_dealt = 0;
         asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&gs->arrived) : "memory");
         unsigned ok = 1, spins = 0;
         while (ld_acquire_u64(&gs->arrived) < target) {
@@ -106,7 +112,8 @@ constexpr uint32_t kWarpQueueCap = 128;
 struct WarpQueue {
     uint32_t *buf;  // kWarpQueueCap entries of shared memory owned by this warp
     uint32_t n;     // fill, identical in all lanes
-    __device__ __forceinline__ explicit WarpQueue(uint32_t *b) : buf(b), n(0) {}
+    uint32_t cap;
+    __device__ __forceinline__ explicit WarpQueue(uint32_t *b, uint32_t c = kWarpQueueCap) : buf(b), n(0), cap(c) {}
     __device__ __forceinline__ void flush(uint32_t *queue, unsigned *len) {
         if (n == 0) return;
         __syncwarp();
@@ -125,32 +132,84 @@ struct WarpQueue {
         const uint32_t lane = threadIdx.x & 31;
         if (p) buf[n + __popc(m & ((1u << lane) - 1u))] = x;
         n += __popc(m);
-        if (n > kWarpQueueCap - 32) flush(queue, len);
+        if (n > cap - 32) flush(queue, len);
     }
 };
 
-// Work-unit dealer: a warp's first unit is its global warp index (no atomic),
-// later ones come from the cursor, offset by the number of warps, so steps
-// with little work cost no atomics at all. The cursor increment for the next
-// unit is issued when a unit is handed out and its reply is only read at the
-// next take(), so its latency overlaps the unit's work.
-struct UnitDealer {
-    unsigned *cursor;
-    uint32_t ticket;  // lane 0: reply of the increment in flight
-    uint32_t nwarps, warp;
-    bool first;
-    __device__ __forceinline__ UnitDealer(unsigned *c, Team t = whole_grid())
-        : cursor(c), ticket(0), nwarps(t.threads() >> 5), warp(t.thread() >> 5), first(true) {}
-    __device__ __forceinline__ uint32_t take(uint32_t units) {
-        uint32_t u;
-        if (first) {
-            u = warp;
-            first = false;
-        } else {
-            u = nwarps + __shfl_sync(0xffffffffu, ticket, 0);
+// The warp's hubs (lanes with hub set, of `chunks` work chunks each) into a
+// hub list behind one atomic: *len holds (hubs << 32) | chunks, and the list
+// stays sorted by first chunk.
+__device__ __forceinline__ void push_hubs(uint32_t v, uint32_t chunks, bool hub, uint32_t *hv, uint32_t *hc,
+                                          unsigned long long *len) {
+    const unsigned m = __ballot_sync(0xffffffffu, hub);
+    if (!m) return;
+    const uint32_t lane = threadIdx.x & 31, mine = hub ? chunks : 0u;
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += t;
+    }
+    unsigned long long h = 0;
+    if (lane == 31) h = atomicAdd(len, ((unsigned long long)__popc(m) << 32) | incl);
+    h = __shfl_sync(0xffffffffu, h, 31);
+    if (hub) {
+        const uint32_t slot = (uint32_t)(h >> 32) + __popc(m & ((1u << lane) - 1u));
+        hv[slot] = v;
+        hc[slot] = (uint32_t)h + incl - mine;
+    }
+}
+
+// End of a phase, all threads of the CTA: what its warps still hold of two
+// queues goes out behind one reservation per queue and CTA. A reservation per
+// warp would be 4,864 atomics on one address, which L2 takes one by one, about
+// a nanosecond each.
+__device__ __forceinline__ void cta_flush(const WarpQueue &a, uint32_t *qa, unsigned *la, const WarpQueue &b,
+                                          uint32_t *qb, unsigned *lb) {
+    __shared__ uint32_t s_fill[2][32], s_at[2][32];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) {
+        s_fill[0][wid] = a.n;
+        s_fill[1][wid] = b.n;
+    }
+    __syncthreads();
+    if (wid < 2) {
+        const uint32_t n = lane < blockDim.x >> 5 ? s_fill[wid][lane] : 0u;
+        uint32_t incl = n, at = 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += t;
         }
-        if (u < units && (threadIdx.x & 31) == 0) ticket = atomicAdd(cursor, 1u);
-        return u;
+        if (lane == 31 && incl) at = atomicAdd(wid ? lb : la, incl);
+        s_at[wid][lane] = __shfl_sync(0xffffffffu, at, 31) + incl - n;
+    }
+    __syncthreads();
+    for (uint32_t i = lane; i < a.n; i += 32) qa[s_at[0][wid] + i] = a.buf[i];
+    for (uint32_t i = lane; i < b.n; i += 32) qb[s_at[1][wid] + i] = b.buf[i];
+}
+
+// Work-unit dealer: unit u belongs to CTA u mod ctas. A CTA's warps take its
+// units in turn -- the first by their index, later ones from a counter in
+// shared memory, which grid_barrier clears, so every phase between two
+// barriers deals anew. One counter for the grid would be an atomic per unit on
+// one address, about a nanosecond each one after the other: 20,000 units are
+// 20 us however they are spread (SSSP on RMAT-22 1,812 -> 1,525 us, on 16M
+// edges 1,003 -> 763). What the CTAs lose by not helping one another is less,
+// as long as a CTA has several units a warp (with the last quarter of the
+// units from a common counter: 1,680 and 871).
+struct UnitDealer {
+    uint32_t cta, ctas, k;
+    bool first;
+    __device__ __forceinline__ explicit UnitDealer(Team t = whole_grid())
+        : cta(t.cta), ctas(t.ctas), k(threadIdx.x >> 5), first(true) {}
+    __device__ __forceinline__ uint32_t take() {
+        if (!first) {
+            if ((threadIdx.x & 31) == 0) k = (blockDim.x >> 5) + atomicAdd(&s_units_dealt, 1u);
+            k = __shfl_sync(0xffffffffu, k, 0);
+        }
+        first = false;
+        return k * ctas + cta;
     }
 };
 

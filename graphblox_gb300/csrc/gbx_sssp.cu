@@ -35,15 +35,20 @@
 
 namespace gbx {
 
-constexpr uint32_t kSsspHubDeg = 1024;
-constexpr uint32_t kSsspHubChunk = 2048;
+// A group of 32 near vertices is one unit of up to 32 * kSsspHubDeg edges, so
+// the hub line bounds a round's slowest warp. R-MAT of 64M / 16M edges and a
+// crawl of 20M, us: 1024 1513 / 767 / 1280, 512 1488 / 649 / 1108, 256 with
+// chunks of 512 1363 / 633 / 991, of 1024 1342 / 634 / 983, 128 1459 / 642 /
+// 921 (more hub units to look up on the largest graph).
+constexpr uint32_t kSsspHubDeg = 256;
+constexpr uint32_t kSsspHubChunk = 1024;
+constexpr uint32_t kScanPerChunk = 16;  // near vertices that a hub chunk counts for in scan_min
 constexpr uint32_t kSsspMaxSplit = 64;  // most warps sharing one 32-vertex group's edges
 constexpr uint32_t kStaleRow = 0xFFFFFFFFu;  // snapshot marker of a near row skipped this round
 constexpr int kSsspThreads = 1024;
 constexpr int kSsspWarps = kSsspThreads / 32;
 
 struct SsspRound {
-    unsigned cursor;
     unsigned near_len;          // next near queue (degree in (0, hub])
     unsigned far_len;           // far pile length (carried across rounds)
     unsigned far_min;           // smallest distance pushed at or past the threshold
@@ -89,7 +94,7 @@ struct SsspArgs {
     uint32_t *dist, *settled, *stamp, *in_far;
     uint32_t *touched;  // bit v: dist[v] lowered in this (scan-mode) round; all zero between rounds
     uint32_t words;     // (V + 31) / 32
-    uint32_t scan_min;  // near vertices (+32 per hub chunk) from which a round runs in scan mode
+    uint32_t scan_min;  // near vertices (+kScanPerChunk per hub chunk) from which a round runs in scan mode
     uint32_t *q[2], *hv[2], *hc[2];
     uint32_t *far[2];
     SsspState *st;
@@ -146,19 +151,11 @@ struct Relaxer {
         for (int q = 0; q < 4; ++q) {
             const bool to_near = below[q] && stamp_old[q] != round;
             const bool to_far = far_cl[q] && far_old[q] == 0u;
-            bool hub = false;
-            if (du[q] == 0) {
-                // nothing to expand: its snapshot is simply its distance, so
-                // a far entry it left behind is dropped, not re-bucketed
-                atomicMin(a.settled + u[q], nd[q]);
-                hub = true;
-            } else if (to_near && du[q] > kSsspHubDeg) {
-                hub = true;
-                unsigned long long h = atomicAdd(&cnt->near_hub, (1ull << 32) | sssp_chunks(du[q]));
-                uint32_t slot = (uint32_t)(h >> 32);
-                hvout[slot] = u[q];
-                hcout[slot] = (uint32_t)h;
-            }
+            // nothing to expand: its snapshot is simply its distance, so a far
+            // entry it left behind is dropped, not re-bucketed
+            if (du[q] == 0) atomicMin(a.settled + u[q], nd[q]);
+            push_hubs(u[q], sssp_chunks(du[q]), to_near && du[q] > kSsspHubDeg, hvout, hcout, &cnt->near_hub);
+            const bool hub = du[q] == 0 || du[q] > kSsspHubDeg;
             wnear.push(u[q], to_near && !hub, qout, &cnt->near_len);
             wfar.push(u[q], to_far, far, &cnt->far_len);
         }
@@ -179,24 +176,33 @@ struct Relaxer {
         for (int q = 0; q < 4; ++q) {
             const float wt = (act[q] && a.w) ? __ldcs(a.w + e[q]) : 1.0f;
             nd[q] = sssp_add(d[q], wt);
+            relaxed += act[q] ? 1u : 0u;
             cur[q] = act[q] ? __ldca(a.dist + u[q]) : 0u;
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            relaxed += act[q] ? 1u : 0u;
-            if (act[q] && nd[q] < cur[q]) {
+            if (nd[q] < cur[q]) {
                 atomicMin(a.dist + u[q], nd[q]);
                 atomicOr(a.touched + (u[q] >> 5), 1u << (u[q] & 31));
             }
         }
     }
+    // all threads of the CTA
     __device__ __forceinline__ void flush() {
-        wnear.flush(qout, &cnt->near_len);
-        wfar.flush(far, &cnt->far_len);
-        unsigned long long r = warp_sum(relaxed);
-        if ((threadIdx.x & 31) == 0 && r) atomicAdd(&cnt->relaxed, r);
+        __shared__ unsigned long long s_relaxed;
+        __shared__ uint32_t s_far_min;
+        if (threadIdx.x == 0) {
+            s_relaxed = 0;
+            s_far_min = 0xFFFFFFFFu;
+        }
+        __syncthreads();
+        const unsigned long long r = warp_sum(relaxed);
         const uint32_t m = warp_min(far_min);
-        if ((threadIdx.x & 31) == 0 && m != 0xFFFFFFFFu) atomicMin(&cnt->far_min, m);
+        if ((threadIdx.x & 31) == 0 && r) atomicAdd(&s_relaxed, r);
+        if ((threadIdx.x & 31) == 0 && m != 0xFFFFFFFFu) atomicMin(&s_far_min, m);
+        cta_flush(wnear, qout, &cnt->near_len, wfar, far, &cnt->far_len);
+        if (threadIdx.x == 0 && s_relaxed) atomicAdd(&cnt->relaxed, s_relaxed);
+        if (threadIdx.x == 32 && s_far_min != 0xFFFFFFFFu) atomicMin(&cnt->far_min, s_far_min);
     }
 };
 
@@ -223,9 +229,9 @@ __device__ void relax_phase(const SsspArgs &a, const uint32_t *qin, uint32_t qn,
     const uint32_t hsplit = nc ? max(1u, min(kSsspHubChunk / 128, kUnitsPerWarp * nwarps / nc)) : 1u;
     const uint32_t gunits = groups * split;
     const uint32_t units = gunits + nc * hsplit;
-    UnitDealer dealer(&cur->cursor);
+    UnitDealer dealer;
     for (;;) {
-        const uint32_t unit = dealer.take(units);
+        const uint32_t unit = dealer.take();
         if (unit >= units) break;
         if (unit >= gunits) {
             const uint32_t chunk = (unit - gunits) / hsplit, hpart = (unit - gunits) % hsplit;
@@ -319,62 +325,90 @@ __device__ void relax_phase(const SsspArgs &a, const uint32_t *qin, uint32_t qn,
 // below the threshold into the next near list (hubs into the hub list,
 // vertices without out-edges settled on the spot), else into the far pile
 // once. A warp takes 32 consecutive vertices (one bitmap word) at a time.
+constexpr uint32_t kScanWords = 4;  // words a warp has in flight: 1 29 to 47 us a pass on RMAT-22, 4 15 to 34, 8 the same
 __device__ void scan_phase(const SsspArgs &a, uint32_t thr, SsspRound *cnt, uint32_t *qout, uint32_t *hvout,
-                           uint32_t *hcout, uint32_t *far, uint32_t *bn, uint32_t *bf) {
+                           uint32_t *hcout, uint32_t *far, uint32_t *bn, uint32_t *bf,
+                           uint32_t *bh, uint32_t *bc) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    uint32_t staged = 0;  // hubs in bh / bc (vertex, chunks), at most 32
+    auto flush_hubs = [&] {
+        __syncwarp();
+        push_hubs(bh[lane], bc[lane], lane < staged, hvout, hcout, &cnt->near_hub);
+        __syncwarp();
+        staged = 0;
+    };
     WarpQueue wnear(bn), wfar(bf);
     uint32_t far_min = 0xFFFFFFFFu;
-    for (uint32_t w = gw; w < a.words; w += nw) {
-        // lane 0 reads and clears the word (one thread: the read is ordered
-        // before the clear), the warp gets it by a shuffle
+    // one lane reads and clears its word: the read is ordered before the clear
+    auto take = [&](uint32_t w0) {
         uint32_t m = 0;
-        if (lane == 0) {
+        const uint32_t w = w0 + lane * nw;
+        if (lane < kScanWords && w < a.words) {
             m = __ldcg(a.touched + w);
             if (m) a.touched[w] = 0u;
         }
-        m = __shfl_sync(0xffffffffu, m, 0);
-        if (!m) continue;
-        const uint32_t u = w * 32 + lane;
-        const bool t = (m >> lane) & 1u;
-        uint32_t d = 0, du = 0, inf = 1;
-        if (t) {
-            d = __ldcg(a.dist + u);
-            du = __ldg(a.outdeg + u);
-            inf = __ldcg(a.in_far + u);
-        }
-        const bool below = t && d < thr;
-        bool to_near = false, to_far = false;
-        if (below) {
-            if (du == 0) {
-                a.settled[u] = d;  // nothing to expand
-            } else if (du > kSsspHubDeg) {
-                const unsigned long long h = atomicAdd(&cnt->near_hub, (1ull << 32) | sssp_chunks(du));
-                const uint32_t slot = (uint32_t)(h >> 32);
-                hvout[slot] = u;
-                hcout[slot] = (uint32_t)h;
-            } else {
-                to_near = true;
+        return m;
+    };
+    uint32_t mine = take(gw);
+    for (uint32_t w0 = gw; w0 < a.words;) {
+        const uint32_t next = w0 + nw * kScanWords;
+        const uint32_t words = mine;
+        mine = next < a.words ? take(next) : 0u;
+        if (__any_sync(0xffffffffu, words != 0)) {
+            uint32_t d[kScanWords], du[kScanWords], inf[kScanWords];
+#pragma unroll
+            for (uint32_t q = 0; q < kScanWords; ++q) {
+                const uint32_t u = (w0 + q * nw) * 32 + lane;
+                const bool t = (__shfl_sync(0xffffffffu, words, q) >> lane) & 1u;
+                d[q] = t ? __ldcg(a.dist + u) : 0xFFFFFFFFu;
+                du[q] = t ? __ldg(a.outdeg + u) : 0u;
+                inf[q] = t ? __ldcg(a.in_far + u) : 1u;
             }
-        } else if (t) {
-            far_min = min(far_min, d);
-            if (!inf) {
-                a.in_far[u] = 1u;
-                to_far = true;
+#pragma unroll
+            for (uint32_t q = 0; q < kScanWords; ++q) {
+                const uint32_t u = (w0 + q * nw) * 32 + lane;
+                const bool t = (__shfl_sync(0xffffffffu, words, q) >> lane) & 1u;
+                const bool below = t && d[q] < thr;
+                const bool hub = below && du[q] > kSsspHubDeg;
+                const bool to_near = below && du[q] != 0 && !hub;
+                bool to_far = false;
+                if (const unsigned hubs = __ballot_sync(0xffffffffu, hub)) {
+                    if (staged + __popc(hubs) > 32) flush_hubs();
+                    if (hub) {
+                        const uint32_t at = staged + __popc(hubs & ((1u << lane) - 1u));
+                        bh[at] = u;
+                        bc[at] = sssp_chunks(du[q]);
+                    }
+                    staged += __popc(hubs);
+                }
+                if (below) {
+                    if (du[q] == 0) a.settled[u] = d[q];  // nothing to expand
+                } else if (t) {
+                    far_min = min(far_min, d[q]);
+                    if (!inf[q]) {
+                        a.in_far[u] = 1u;
+                        to_far = true;
+                    }
+                }
+                wnear.push(u, to_near, qout, &cnt->near_len);
+                wfar.push(u, to_far, far, &cnt->far_len);
             }
         }
-        wnear.push(u, to_near, qout, &cnt->near_len);
-        wfar.push(u, to_far, far, &cnt->far_len);
+        w0 = next;
     }
-    wnear.flush(qout, &cnt->near_len);
-    wfar.flush(far, &cnt->far_len);
+    if (staged) flush_hubs();
+    __shared__ uint32_t s_far_min;
+    if (threadIdx.x == 0) s_far_min = 0xFFFFFFFFu;
+    __syncthreads();
     const uint32_t fm = warp_min(far_min);
-    if (lane == 0 && fm != 0xFFFFFFFFu) atomicMin(&cnt->far_min, fm);
+    if (lane == 0 && fm != 0xFFFFFFFFu) atomicMin(&s_far_min, fm);
+    cta_flush(wnear, qout, &cnt->near_len, wfar, far, &cnt->far_len);
+    if (threadIdx.x == 0 && s_far_min != 0xFFFFFFFFu) atomicMin(&cnt->far_min, s_far_min);
 }
 
 __device__ __forceinline__ void zero_round(SsspRound *r, uint32_t far_len) {
-    r->cursor = 0;
     r->near_len = 0;
     r->far_len = far_len;
     r->far_min = 0xFFFFFFFFu;
@@ -427,14 +461,14 @@ __global__ void __launch_bounds__(kSsspThreads, 1) sssp_persistent_kernel(SsspAr
             // a large round relaxes with reductions and queues what it
             // lowered in a scan pass after one more barrier; a small one
             // queues each improvement as it happens
-            const bool scan = (uint64_t)qn + 32ull * nc >= a.scan_min;
+            const bool scan = (uint64_t)qn + kScanPerChunk * nc >= a.scan_min;
             if (scan) {
                 relax_phase<true>(a, a.q[ib], qn, a.hv[ib], a.hc[ib], nh, nc, rx, cur, s_pre[wid], s_base[wid],
                                   s_d[wid]);
                 rx.flush();
                 if (!grid_barrier(&st->gs)) { failed = true; break; }
                 scan_phase(a, thr, cur, a.q[ib ^ 1], a.hv[ib ^ 1], a.hc[ib ^ 1], a.far[fb] + far_len, s_wn[wid],
-                           s_wf[wid]);
+                           s_wf[wid], s_base[wid], s_d[wid]);
             } else {
                 relax_phase<false>(a, a.q[ib], qn, a.hv[ib], a.hc[ib], nh, nc, rx, cur, s_pre[wid], s_base[wid],
                                    s_d[wid]);
@@ -514,28 +548,16 @@ __global__ void __launch_bounds__(kSsspThreads, 1) sssp_persistent_kernel(SsspAr
                 }
 #pragma unroll
                 for (uint32_t q = 0; q < kSplitIlp; ++q) {
-                    if (to_near[q]) {
-                        if (du[q] > kSsspHubDeg) {
-                            hub[q] = true;
-                            const unsigned long long h =
-                                atomicAdd(&cur->near_hub, (1ull << 32) | sssp_chunks(du[q]));
-                            const uint32_t slot = (uint32_t)(h >> 32);
-                            a.hv[ib][slot] = u[q];
-                            a.hc[ib][slot] = (uint32_t)h;
-                        } else if (du[q] == 0) {
-                            // nothing to relax: settled right here
-                            hub[q] = true;
-                            a.settled[u[q]] = d[q];
-                        }
-                    }
+                    push_hubs(u[q], sssp_chunks(du[q]), to_near[q] && du[q] > kSsspHubDeg, a.hv[ib], a.hc[ib], &cur->near_hub);
+                    if (to_near[q] && du[q] == 0) a.settled[u[q]] = d[q];  // nothing to relax
+                    hub[q] = du[q] > kSsspHubDeg || du[q] == 0;
                     wnear.push(u[q], to_near[q] && !hub[q], a.q[ib], &cur->near_len);
                     wfar.push(u[q], keep[q], a.far[fb ^ 1], &cur->far_len);
                 }
             }
-            wnear.flush(a.q[ib], &cur->near_len);
-            wfar.flush(a.far[fb ^ 1], &cur->far_len);
             kmin = warp_min(kmin);
             if (lane == 0 && kmin != 0xFFFFFFFFu) atomicMin(&cur->kept_min, kmin);
+            cta_flush(wnear, a.q[ib], &cur->near_len, wfar, a.far[fb ^ 1], &cur->far_len);
         }
         if (!grid_barrier(&st->gs)) { failed = true; break; }
         fetch_counters(cur, &s_cnt);
@@ -760,10 +782,10 @@ extern "C" int gbx_sssp(gbx_graph *g, uint32_t source, uint32_t delta, uint32_t 
     const uint32_t V = g->V;
     if (V <= kSsspSmallV && g->E <= kSsspSmallE && !trace_enabled()) return sssp_small(g, source, distances, result, s);
     // Bucket width where neither the caller nor the graph's tuning gives one:
-    // up to a few million edges a round is mostly latency, so fewer, wider
-    // buckets (R-MAT of 250,000 vertices and 2.5M edges: 535 us with 256, 472
-    // with 1024; crawl of 1M edges: 711, 581; R-MAT of 8M edges: 1226, 1301)
-    if (delta == 0) delta = g->sssp_delta ? g->sssp_delta : !g->weight ? 1u : g->E <= 6'000'000u ? 1024u : 256u;
+    // up to some ten million edges a round is mostly latency, so fewer, wider
+    // buckets. us with 256 / 1024: R-MAT of 2.5M edges 365 / 334, 8M 686 / 666,
+    // 16M 556 / 559, 64M 1,227 / 1,292; crawl of 1M edges 537 / 436, 20M 931 / 870.
+    if (delta == 0) delta = g->sssp_delta ? g->sssp_delta : !g->weight ? 1u : g->E <= 32'000'000u ? 1024u : 256u;
     // working arrays from the graph's scratch arena (plus staging for a
     // host-memory result)
     const int out_dev = is_device_ptr(distances) ? 1 : 0;
@@ -804,7 +826,8 @@ extern "C" int gbx_sssp(gbx_graph *g, uint32_t source, uint32_t delta, uint32_t 
     a.in_far = in_far;
     a.touched = touched;
     a.words = words;
-    a.scan_min = std::max<uint32_t>(4096u, V / 256);
+        // (V / 1024: 1,239 us on RMAT-22, V / 256: 1,229, V / 64: 1,221)
+    a.scan_min = std::max<uint32_t>(8192u, V / 64);
     a.q[0] = q0;
     a.q[1] = q1;
     a.hv[0] = hv0;
