@@ -46,7 +46,6 @@ constexpr uint32_t kHubDeg = 1024;    // out-degree above which a vertex is a hu
 constexpr uint32_t kHubChunk = 1024;  // edges per hub work unit
 constexpr uint32_t kBuProbe = 64;     // bottom-up: in-edges a lane probes alone before the warp helps
 constexpr uint32_t kTdMaxSplit = 64;  // top-down: most warps sharing one 32-vertex group's edges
-constexpr uint32_t kBuWords = 8;      // bottom-up: frontier-bitmap words (32 vertices each) per work unit
 constexpr int kBfsThreads = 768;
 constexpr uint32_t kBfsQueueCap = 256;  // entries a warp stages (128: 171 us a traversal of RMAT-22, 256: 167)
 constexpr int kBfsWarps = kBfsThreads / 32;
@@ -370,7 +369,7 @@ __device__ __forceinline__ uint32_t bu_probe(const BfsArgs &a, const uint32_t *c
     return pick;
 }
 
-// One bottom-up step. A work unit is kBuWords frontier-bitmap words; its
+// One bottom-up step. A work unit is a few frontier-bitmap words; its
 // candidates -- vertices not yet visited that have pull in-edges (the live
 // bitmap), the only ones a bottom-up step can find -- are numbered word by
 // word and dealt to the lanes 32 at a time, so a lane never idles on a
@@ -389,11 +388,17 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
     unsigned nf = 0;
     unsigned long long edges = 0;
     WarpQueue wq(s_wq, kBfsQueueCap);
-    const uint32_t units = (a.words + kBuWords - 1) / kBuWords;
+    // Words per unit: many candidates per unit keep the lanes full (a unit of
+    // n words ends with a part round), two units per warp even the warps out.
+    // us with 4 / 8 / 16 / 32 words: RMAT-22, eight teams 903 / 770 / 718 /
+    // 695; one traversal 183 / 167 / 167 / 176; 100,000 vertices 73 / 78 / 84.
+    uint32_t bw = 2;
+    while (bw < 32 && a.words >= 4 * bw * (team.threads() >> 5)) bw *= 2;
+    const uint32_t units = (a.words + bw - 1) / bw;
     UnitDealer dealer(team);
     for (uint32_t unit = dealer.take(); unit < units; unit = dealer.take()) {
-        const uint32_t w0 = unit * kBuWords;
-        const uint32_t nw = min(a.words - w0, kBuWords);
+        const uint32_t w0 = unit * bw;
+        const uint32_t nw = min(a.words - w0, bw);
         // lane k < nw holds word w0 + k (only this warp writes these words in the step)
         const uint32_t vis = lane < nw ? __ldcg(a.visited + w0 + lane) : 0xFFFFFFFFu;
         const uint32_t cand = lane < nw ? (~vis & __ldg(a.live + w0 + lane)) : 0u;
@@ -405,7 +410,7 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
             if (lane >= (uint32_t)o) incl += t;
         }
         const uint32_t excl = incl - c, total = __shfl_sync(0xffffffffu, incl, 31);
-        if (lane < kBuWords) s_found[lane] = 0u;
+        s_found[lane] = 0u;
         __syncwarp();
         // candidate i -> (its word k, its vertex, that vertex's row bounds and
         // out-degree); the next round's rows are loaded while this round probes
@@ -602,7 +607,7 @@ __device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSy
     __shared__ uint32_t s_base[kBfsWarps][32];
     __shared__ uint32_t s_v[kBfsWarps][32];
     __shared__ uint32_t s_wq[kBfsWarps][kBfsQueueCap];
-    __shared__ uint32_t s_found[kBfsWarps][kBuWords];
+    __shared__ uint32_t s_found[kBfsWarps][32];
     __shared__ BfsStep s_cnt;  // the finished step's counters (fetch_counters)
     const uint32_t wid = threadIdx.x >> 5;
     BfsState *st = a.st;
@@ -755,7 +760,7 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
 // working arrays and its own barrier, the next trial from a counter when one
 // is done. A team also writes its trial's initial state, which is a kernel of
 // its own otherwise. 8 trials: RMAT-22 (64M edges) 1,430 us one after the
-// other, 775 by eight teams; 250,000 vertices and 3M edges 543, 138.
+// other, 695 by eight teams; 250,000 vertices and 3M edges 543, 137.
 struct BfsTeams {
     BfsArgs first;            // team 0's working arrays; level / parent: its own, for trials without outputs
     size_t pitch;             // bytes from one team's working arrays to the next's
