@@ -24,7 +24,7 @@
 // with many upper neighbours is cut into units of kUpperChunk of them, dealt
 // to warps by an atomic cursor, so hubs are spread over the GPU; the rest
 // are one warp per v. A v whose N+(v) is
-// longer than the per-warp table (up to 16384 ids) goes to tc_wide_kernel:
+// longer than the per-warp tests take (up to 16384 ids) goes to tc_wide_kernel:
 // one CTA per unit of its upper neighbours, N+(v) in a CTA-wide table, so no
 // element is searched in global memory. The prefixes are read as aligned
 // 16-byte quads.
@@ -49,6 +49,11 @@ namespace gbx {
 constexpr int kTcThreads = 256;
 constexpr int kTcWarps = kTcThreads / 32;
 constexpr uint32_t kTcTableMax = 512;   // |N+(v)| that fits a per-warp table
+// |N+(v)| up to which a warp's bitmap (v below its range, or few ids of the
+// list above it) takes v instead of a CTA; every unit builds it anew, which
+// costs less than the CTA's waits. RMAT of 16M / 64M edges, us: 512 982 /
+// 7,684, 1024 929 / 7,125, 2048 926 / 7,137, 16384 923 / 7,145.
+constexpr uint32_t kTcBitsMax = 2048;
 constexpr uint32_t kTcWarpSlots = 1024;  // hash slots per warp
 constexpr uint32_t kUpperChunk = 256;   // upper neighbours per work unit
 constexpr uint32_t kEmptySlot = 0xFFFFFFFFu;
@@ -58,6 +63,11 @@ constexpr uint32_t kEmptySlot = 0xFFFFFFFFu;
 // second per-warp hash table of at most kHybridSlots slots
 constexpr uint32_t kHybridSplit = kTcWarpSlots * 32;
 constexpr uint32_t kHybridSlots = 256;
+
+// whether the sorted list N+(v) fits the hybrid test: at most kHybridSlots / 2 ids at or above kHybridSplit
+__device__ __forceinline__ bool hybrid_fits(const uint32_t *nv, uint32_t pv) {
+    return pv <= kHybridSlots / 2 || __ldg(nv + pv - 1 - kHybridSlots / 2) < kHybridSplit;
+}
 
 // number of elements <= x (or < x) in sorted a[0..n)
 __device__ __forceinline__ uint32_t count_le(const uint32_t *a, uint32_t n, uint32_t x) {
@@ -263,74 +273,78 @@ __device__ __forceinline__ unsigned long long count_flat(const uint32_t *__restr
 // Same count with 16-byte loads: each lane's list [base, base+len) is read as
 // the aligned quads that cover it (the neighbour array is 16-byte aligned and
 // padded by four ids), four quads per lane per step, and the elements of a
-// quad outside the list are masked. Four times fewer load instructions and
-// four times the bytes in flight of count_flat.
+// quad outside the list are masked. Issue slots bound it (65% busy, LSU 51%),
+// so a quad costs as few instructions as it can: a list is one 16-byte record
+// that stays in registers until the lane's quads leave the list, the masks of
+// its first and last quad are shifts kept in the record, and the four
+// membership words meet as bytes of one word. RMAT of 16M edges: 764 us -> 662.
+struct QuadList {
+    uint32_t pre, next;  // the list's quads are [pre, next) of the warp's
+    uint32_t shift;      // quad index - position among the warp's quads
+    uint32_t cut;        // 8 * (elements of the first quad before the list) | 8 * (of the last one after it) << 8
+};
+
 template <class Member>
-__device__ __forceinline__ unsigned long long count_flat4(const uint32_t *__restrict__ dest, uint32_t base,
-                                                         uint32_t len, uint32_t *s_pre, uint32_t *s_base,
-                                                         uint32_t *s_end, const Member &member) {
+__device__ __forceinline__ uint32_t count_flat4(const uint32_t *__restrict__ dest, uint32_t base, uint32_t len,
+                                                QuadList *s_list, const Member &member) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t q0 = base >> 2;
-    const uint32_t nq = len ? ((base + len + 3) >> 2) - q0 : 0u;
+    const uint32_t end = base + len, q0 = base >> 2;
+    const uint32_t nq = len ? ((end + 3) >> 2) - q0 : 0u;
     uint32_t incl = nq;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= (uint32_t)o) incl += t;
     }
-    s_pre[lane] = incl - nq;
-    s_base[lane] = base;
-    s_end[lane] = base + len;
-    if (lane == 31) s_pre[32] = incl;
+    const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
+    *reinterpret_cast<uint4 *>(s_list + lane) =
+        make_uint4(incl - nq, incl, q0 - (incl - nq), 8 * (base & 3) | (8 * (3 - ((end - 1) & 3))) << 8);
     __syncwarp();
-    const uint32_t tot = s_pre[32];
     const uint4 *d4 = reinterpret_cast<const uint4 *>(dest);
-    unsigned long long count = 0;
-    uint32_t k = 0;  // owner lane of this lane's current quad, advanced monotonically
+    uint32_t count = 0;
+    const uint4 *at = reinterpret_cast<const uint4 *>(s_list);  // the list of this lane's current quad
+    uint4 l = *at;
     for (uint32_t i0 = 0; i0 < tot; i0 += 128) {
         uint4 w[4];
-        uint32_t e0[4], lo[4], hi[4];
+        uint32_t valid[4];  // byte j: 1 where the quad's element j is in the list
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const uint32_t i = i0 + q * 32 + lane;
-            lo[q] = hi[q] = e0[q] = 0;
+            valid[q] = 0;
             w[q] = make_uint4(0u, 0u, 0u, 0u);
             if (i < tot) {
-                while (s_pre[k + 1] <= i) ++k;
-                const uint32_t qa = (s_base[k] >> 2) + (i - s_pre[k]);
-                w[q] = __ldg(d4 + qa);
-                e0[q] = qa * 4;
-                lo[q] = s_base[k];
-                hi[q] = s_end[k];
+                while (l.y <= i) l = *++at;
+                w[q] = __ldg(d4 + (l.z + i));
+                const uint32_t from = i == l.x ? l.w & 31u : 0u, to = i + 1 == l.y ? l.w >> 8 : 0u;
+                valid[q] = (0x01010101u << from) & (0x01010101u >> to);
             }
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            // the quad's elements inside [lo, hi) as a 4-bit mask; the
-            // membership bits of all four, then one popcount
-            const uint32_t x[4] = {w[q].x, w[q].y, w[q].z, w[q].w};
-            const uint32_t from = lo[q] > e0[q] ? min(lo[q] - e0[q], 4u) : 0u;
-            const uint32_t to = hi[q] > e0[q] ? min(hi[q] - e0[q], 4u) : 0u;
-            const uint32_t valid = (0xFu >> (4u - to)) & (0xFu << from) & 0xFu;
-            uint32_t hit = 0;
+            if (Member::kProbeAll) {
+                // reading a bitmap word is cheaper than branching around it
+                const uint32_t lo = __byte_perm(member.word(w[q].x), member.word(w[q].y), 0x0040);
+                const uint32_t hi = __byte_perm(member.word(w[q].z), member.word(w[q].w), 0x4000);
+                count += __popc(__byte_perm(lo, hi, 0x7610) & valid[q]);
+            } else {
+                const uint32_t x[4] = {w[q].x, w[q].y, w[q].z, w[q].w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                // a bitmap bit is cheaper to read than to branch around
-                if (Member::kProbeAll || ((valid >> j) & 1u)) hit |= member.bit(x[j]) << j;
+                for (int j = 0; j < 4; ++j)
+                    if ((valid[q] >> (8 * j)) & 1u) count += member.word(x[j]);
             }
-            count += __popc(hit & valid);
         }
     }
     __syncwarp();
     return count;
 }
 
+// Membership tests: bit 0 of word(w) says whether w is in the list (the other
+// bits are 0 unless kProbeAll).
 struct HashMember {
     static constexpr bool kProbeAll = false;
     const uint32_t *table;
     uint32_t mask;
-    __device__ __forceinline__ bool operator()(uint32_t w) const { return hash_contains(table, mask, w); }
-    __device__ __forceinline__ uint32_t bit(uint32_t w) const { return hash_contains(table, mask, w) ? 1u : 0u; }
+    __device__ __forceinline__ uint32_t word(uint32_t w) const { return hash_contains(table, mask, w) ? 1u : 0u; }
 };
 
 // Exact bitmap over [0, nbits) with nbits a power of two. Ids are masked
@@ -342,22 +356,21 @@ struct HybridMember {
     const uint32_t *bits;   // ids below kHybridSplit
     const uint32_t *table;  // the others
     uint32_t mask;
-    __device__ __forceinline__ uint32_t bit(uint32_t w) const {
-        if (w < kHybridSplit) return (bits[w >> 5] >> (w & 31)) & 1u;
+    __device__ __forceinline__ uint32_t word(uint32_t w) const {
+        if (w < kHybridSplit) return bits[w >> 5] >> (w & 31);
         return hash_contains(table, mask, w) ? 1u : 0u;
     }
-    __device__ __forceinline__ bool operator()(uint32_t w) const { return bit(w) != 0u; }
 };
 
 struct BitmapMember {
     static constexpr bool kProbeAll = true;
     const uint32_t *bits;
     uint32_t id_mask;  // nbits - 1
-    __device__ __forceinline__ uint32_t bit(uint32_t w) const {
-        const uint32_t x = w & id_mask;
-        return (bits[x >> 5] >> (x & 31)) & 1u;
+    __device__ __forceinline__ uint32_t word(uint32_t w) const {
+        // byte offset of id w's word, masked into the bitmap
+        const uint32_t at = (w >> 3) & (id_mask >> 3 & ~3u);
+        return *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(bits) + at) >> (w & 31);
     }
-    __device__ __forceinline__ bool operator()(uint32_t w) const { return bit(w) != 0u; }
 };
 
 // For the upper neighbours u in [ub, ue) of v's row nv, 32 at a time: the
@@ -368,8 +381,7 @@ template <class Member>
 __device__ __forceinline__ unsigned long long stream_pairs(const uint32_t *__restrict__ off,
                                                           const uint32_t *__restrict__ dest, const uint32_t *nv,
                                                           const uint32_t *pl, uint32_t v, uint32_t ub, uint32_t ue,
-                                                          uint32_t *s_pre, uint32_t *s_base, uint32_t *s_end,
-                                                          const Member &m) {
+                                                          QuadList *s_list, const Member &m) {
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long count = 0;
     for (uint32_t a0 = ub; a0 < ue; a0 += 32) {
@@ -379,7 +391,7 @@ __device__ __forceinline__ unsigned long long stream_pairs(const uint32_t *__res
             base = __ldg(off + u);
             len = pl ? __ldg(pl + a0 + lane) : count_le(dest + base, __ldg(off + u + 1) - base, v);
         }
-        count += count_flat4(dest, base, len, s_pre, s_base, s_end, m);
+        count += count_flat4(dest, base, len, s_list, m);
     }
     return count;
 }
@@ -392,9 +404,7 @@ template <class Member>
 __device__ __forceinline__ unsigned long long stream_pairs_dealt(const uint32_t *__restrict__ off,
                                                                 const uint32_t *__restrict__ dest,
                                                                 const uint32_t *nv, const uint32_t *pl, uint32_t v,
-                                                                uint32_t ub, uint32_t ue, uint32_t *s_pre,
-                                                                uint32_t *s_base,
-                                                                uint32_t *s_end, const Member &m,
+                                                                uint32_t ub, uint32_t ue, QuadList *s_list, const Member &m,
                                                                 unsigned *s_next) {
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long count = 0;
@@ -409,7 +419,7 @@ __device__ __forceinline__ unsigned long long stream_pairs_dealt(const uint32_t 
             base = __ldg(off + u);
             len = pl ? __ldg(pl + a0 + lane) : count_le_front(dest + base, __ldg(off + u + 1) - base, v);
         }
-        count += count_flat4(dest, base, len, s_pre, s_base, s_end, m);
+        count += count_flat4(dest, base, len, s_list, m);
     }
     return count;
 }
@@ -419,7 +429,7 @@ struct SortedMember {
     const uint32_t *list;
     uint32_t n;
     __device__ __forceinline__ bool operator()(uint32_t w) const { return sorted_contains(list, n, w); }
-    __device__ __forceinline__ uint32_t bit(uint32_t w) const { return sorted_contains(list, n, w) ? 1u : 0u; }
+    __device__ __forceinline__ uint32_t word(uint32_t w) const { return sorted_contains(list, n, w) ? 1u : 0u; }
 };
 
 // One v, upper neighbours [ub, ue) of its row: build the membership test of
@@ -428,7 +438,7 @@ __device__ __forceinline__ unsigned long long v_unit(const uint32_t *__restrict_
                                                     const uint32_t *__restrict__ dest,
                                                     const uint32_t *__restrict__ pre_len, uint32_t v, uint32_t pv,
                                                     uint32_t ub, uint32_t ue, uint32_t *table, uint32_t *htable,
-                                                    uint32_t *s_pre, uint32_t *s_base, uint32_t *s_end) {
+                                                    QuadList *s_list) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t row = __ldg(off + v);
     const uint32_t *nv = dest + row, *pl = pre_len ? pre_len + row : nullptr;
@@ -441,47 +451,44 @@ __device__ __forceinline__ unsigned long long v_unit(const uint32_t *__restrict_
             atomicOr(table + (w >> 5), 1u << (w & 31));
         }
         __syncwarp();
-        count = stream_pairs(off, dest, nv, pl, v, ub, ue, s_pre, s_base, s_end,
+        count = stream_pairs(off, dest, nv, pl, v, ub, ue, s_list,
                              BitmapMember{table, kTcWarpSlots * 32 - 1});
         __syncwarp();
         for (uint32_t i = lane; i < pv; i += 32) table[__ldg(nv + i) >> 5] = 0u;
         __syncwarp();
-    } else if (pv <= kTcTableMax) {
-        uint32_t nh = 0;  // ids of N+(v) at or above kHybridSplit
-        for (uint32_t i = lane; i < pv; i += 32) nh += __ldg(nv + i) >= kHybridSplit ? 1u : 0u;
+    } else if (hybrid_fits(nv, pv)) {
+        uint32_t nh = 0;  // ids of N+(v) at or above kHybridSplit: among the last kHybridSlots / 2
+        for (uint32_t i = lane; i < min(pv, kHybridSlots / 2); i += 32) nh += __ldg(nv + pv - 1 - i) >= kHybridSplit ? 1u : 0u;
         nh = warp_sum(nh);
-        if (2 * nh <= kHybridSlots) {
-            uint32_t hmask = 31;
-            while (hmask + 1 < 2 * nh) hmask = 2 * hmask + 1;
-            for (uint32_t i = lane; i <= hmask; i += 32) htable[i] = kEmptySlot;
-            __syncwarp();
-            for (uint32_t i = lane; i < pv; i += 32) {
-                const uint32_t w = __ldg(nv + i);
-                if (w < kHybridSplit) atomicOr(table + (w >> 5), 1u << (w & 31));
-                else hash_insert(htable, hmask, w);
-            }
-            __syncwarp();
-            count = stream_pairs(off, dest, nv, pl, v, ub, ue, s_pre, s_base, s_end,
-                                 HybridMember{table, htable, hmask});
-            __syncwarp();
-            for (uint32_t i = lane; i < pv; i += 32) {
-                const uint32_t w = __ldg(nv + i);
-                if (w < kHybridSplit) table[w >> 5] = 0u;
-            }
-            __syncwarp();
-            return count;
+        uint32_t hmask = 31;
+        while (hmask + 1 < 2 * nh) hmask = 2 * hmask + 1;
+        for (uint32_t i = lane; i <= hmask; i += 32) htable[i] = kEmptySlot;
+        __syncwarp();
+        for (uint32_t i = lane; i < pv; i += 32) {
+            const uint32_t w = __ldg(nv + i);
+            if (w < kHybridSplit) atomicOr(table + (w >> 5), 1u << (w & 31));
+            else hash_insert(htable, hmask, w);
         }
+        __syncwarp();
+        count = stream_pairs(off, dest, nv, pl, v, ub, ue, s_list, HybridMember{table, htable, hmask});
+        __syncwarp();
+        for (uint32_t i = lane; i < pv; i += 32) {
+            const uint32_t w = __ldg(nv + i);
+            if (w < kHybridSplit) table[w >> 5] = 0u;
+        }
+        __syncwarp();
+    } else if (pv <= kTcTableMax) {
         const uint32_t mask = table_mask(pv);
         for (uint32_t i = lane; i <= mask; i += 32) table[i] = kEmptySlot;
         __syncwarp();
         for (uint32_t i = lane; i < pv; i += 32) hash_insert(table, mask, __ldg(nv + i));
         __syncwarp();
-        count = stream_pairs(off, dest, nv, pl, v, ub, ue, s_pre, s_base, s_end, HashMember{table, mask});
+        count = stream_pairs(off, dest, nv, pl, v, ub, ue, s_list, HashMember{table, mask});
         __syncwarp();
         for (uint32_t i = lane; i <= mask; i += 32) table[i] = 0u;
         __syncwarp();
     } else {
-        count = stream_pairs(off, dest, nv, pl, v, ub, ue, s_pre, s_base, s_end, SortedMember{nv, pv});
+        count = stream_pairs(off, dest, nv, pl, v, ub, ue, s_list, SortedMember{nv, pv});
     }
     return count;
 }
@@ -608,9 +615,7 @@ __global__ void __launch_bounds__(kTcThreads, 4)
                        unsigned long long *total) {
     __shared__ uint32_t tables[kTcWarps][kTcWarpSlots];
     __shared__ uint32_t htables[kTcWarps][kHybridSlots];
-    __shared__ uint32_t s_pre[kTcWarps][33];
-    __shared__ uint32_t s_base[kTcWarps][32];
-    __shared__ uint32_t s_end[kTcWarps][32];
+    __shared__ __align__(16) QuadList s_list[kTcWarps][32];
     __shared__ unsigned long long sred[32];
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned long long count = 0;
@@ -631,7 +636,7 @@ __global__ void __launch_bounds__(kTcThreads, 4)
         const uint32_t ub = bg.ub + (unit - bg.first_unit) * kUpperChunk;
         const uint32_t ue = min(ub + kUpperChunk, bg.ue);
         count += v_unit(off, dest, pre_len, bg.v, __ldg(low + bg.v), ub, ue, tables[wid], htables[wid],
-                        s_pre[wid], s_base[wid], s_end[wid]);
+                        s_list[wid]);
     }
     // the other pivots with work (the plan's compact list, with the first
     // upper neighbour precomputed): one warp each
@@ -640,7 +645,7 @@ __global__ void __launch_bounds__(kTcThreads, 4)
     for (uint32_t i = gw; i < n_small; i += nw) {
         const TcBig sm = small[i];
         count += v_unit(off, dest, pre_len, sm.v, __ldg(low + sm.v), sm.ub, sm.ue, tables[wid], htables[wid],
-                        s_pre[wid], s_base[wid], s_end[wid]);
+                        s_list[wid]);
     }
     count = block_sum(count, sred);
     if (threadIdx.x == 0 && count) atomicAdd(total, count);
@@ -693,9 +698,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                    const TcBig *__restrict__ wide, uint32_t n_wide,
                    uint32_t n_units, uint32_t slots, unsigned *cursor, unsigned long long *total) {
     extern __shared__ uint32_t s_table[];
-    __shared__ uint32_t s_pre[kWideThreads / 32][33];
-    __shared__ uint32_t s_base[kWideThreads / 32][32];
-    __shared__ uint32_t s_end[kWideThreads / 32][32];
+    __shared__ __align__(16) QuadList s_list[kWideThreads / 32][32];
     __shared__ uint32_t s_unit;
     __shared__ unsigned s_next;
     __shared__ unsigned long long sred[32];
@@ -727,7 +730,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                 atomicOr(s_table + (w >> 5), 1u << (w & 31));
             }
             __syncthreads();
-            count += stream_pairs_dealt(off, dest, nv, pl, v, ub, ue, s_pre[wid], s_base[wid], s_end[wid],
+            count += stream_pairs_dealt(off, dest, nv, pl, v, ub, ue, s_list[wid],
                                         BitmapMember{s_table, slots * 32 - 1}, &s_next);
             __syncthreads();
             for (uint32_t i = threadIdx.x; i < pv; i += blockDim.x) s_table[__ldg(nv + i) >> 5] = 0u;
@@ -738,7 +741,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
             __syncthreads();
             for (uint32_t i = threadIdx.x; i < pv; i += blockDim.x) hash_insert(s_table, mask, __ldg(nv + i));
             __syncthreads();
-            count += stream_pairs_dealt(off, dest, nv, pl, v, ub, ue, s_pre[wid], s_base[wid], s_end[wid],
+            count += stream_pairs_dealt(off, dest, nv, pl, v, ub, ue, s_list[wid],
                                         HashMember{s_table, mask}, &s_next);
             __syncthreads();
             for (uint32_t i = threadIdx.x; i <= mask; i += blockDim.x) s_table[i] = 0u;
@@ -751,8 +754,8 @@ __global__ void __launch_bounds__(kWideThreads, 1)
 // Work lists of the v-centric count. kind 3: v's below the hub range H with
 // pairs (units of hub_uppers_per_unit(v), tc_hub_kernel); for the others,
 // kind 0: v's with more than kUpperChunk upper neighbours and |N+(v)| within
-// the warp table (units of kUpperChunk); kind 1: v's with |N+(v)| above the
-// warp table and within the CTA table (units of kWideChunk, for
+// what a warp takes (units of kUpperChunk); kind 1: v's with |N+(v)| above
+// that and within the CTA table (units of kWideChunk, for
 // tc_wide_kernel); kind 2: every other v with N+(v) and an upper neighbour
 // (one warp each). v's without both have no pairs and are in no list.
 __global__ void tc_plan_flags_kernel(const uint32_t *off, const uint32_t *dest, const uint32_t *low, uint32_t V,
@@ -764,7 +767,8 @@ __global__ void tc_plan_flags_kernel(const uint32_t *off, const uint32_t *dest, 
         const uint32_t up = d - ub, pv = low[v];
         const bool pairs = pv > 0 && up > 0;
         const bool hub = v < H;
-        const bool wide = !hub && pv > kTcTableMax && pv <= kWideSlotsMax / 2;
+        const uint32_t warp_max = v < kTcWarpSlots * 32 || hybrid_fits(dest + b, pv) ? kTcBitsMax : kTcTableMax;
+        const bool wide = !hub && pv > warp_max && pv <= kWideSlotsMax / 2;
         const bool big = !hub && !wide && (up > kUpperChunk || pv > kTcTableMax);
         flag[v] = pairs && big ? 1u : 0u;
         flag[(size_t)V + v] = pairs && wide ? 1u : 0u;
@@ -931,12 +935,10 @@ extern "C" int gbx_tc(gbx_graph *g, uint64_t *total, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t V = g->V;
     GBX_TRY(tc_prepare(g, s));
-    DevBuf<unsigned long long> d;
-    DevBuf<unsigned> cursor;
-    GBX_TRY(d.alloc(1, s));
-    GBX_TRY(cursor.alloc(3, s));
-    GBX_CUDA(cudaMemsetAsync(d.p, 0, 8, s));
-    GBX_CUDA(cudaMemsetAsync(cursor.p, 0, 12, s));
+    DevBuf<unsigned long long> d;  // the total, then the kernels' cursors
+    GBX_TRY(d.alloc(3, s));
+    GBX_CUDA(cudaMemsetAsync(d.p, 0, 24, s));
+    unsigned *const cursor = reinterpret_cast<unsigned *>(d.p + 1);
     if (g->tc_plan) {
         int per_sm = 0;
         GBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_vcentric_kernel, kTcThreads, 0));
@@ -944,7 +946,7 @@ extern "C" int gbx_tc(gbx_graph *g, uint64_t *total, void *stream) {
         const gbx_tc_plan *p = g->tc_plan;
         tc_vcentric_kernel<<<grid, kTcThreads, 0, s>>>(g->offsets, g->dest, g->low_count, p->pre_len, p->big,
                                                        p->n_big, p->n_big ? p->n_units : 0u, p->small, p->n_small,
-                                                       cursor.p, d.p);
+                                                       cursor, d.p);
         GBX_LAUNCH_CHECK();
         if (p->n_wide) {
             const size_t smem = (size_t)kWideSlotsMax * 4;
@@ -954,7 +956,7 @@ extern "C" int gbx_tc(gbx_graph *g, uint64_t *total, void *stream) {
             const unsigned wgrid = std::min<unsigned>((unsigned)std::max(1, wper) * (unsigned)num_sms(), p->n_wunits);
             tc_wide_kernel<<<wgrid, kWideThreads, smem, s>>>(g->offsets, g->dest, g->low_count, p->pre_len,
                                                               p->wide, p->n_wide, p->n_wunits, kWideSlotsMax,
-                                                              cursor.p + 1, d.p);
+                                                              cursor + 1, d.p);
         }
         if (p->n_hub) {
             GBX_LAUNCH_CHECK();
@@ -963,7 +965,7 @@ extern "C" int gbx_tc(gbx_graph *g, uint64_t *total, void *stream) {
             const unsigned hgrid = std::min<unsigned>((unsigned)std::max(1, hper) * (unsigned)num_sms(),
                                                       ceil_div(p->n_hunits, kTcWarps));
             tc_hub_kernel<<<hgrid, kTcThreads, 0, s>>>(g->offsets, g->dest, p->hub_bits, p->hub_words, p->hub,
-                                                       p->n_hub, p->n_hunits, cursor.p + 2, d.p);
+                                                       p->n_hub, p->n_hunits, cursor + 2, d.p);
         }
     } else {
         const unsigned wgrid = std::min<unsigned>(ceil_div((uint64_t)V * 32, kTcThreads), (unsigned)num_sms() * 8);
