@@ -103,10 +103,17 @@ __global__ void pull_units_kernel(const uint32_t *off, const uint32_t *row_pos, 
 
 // Sweeps after which a layout has paid for itself.
 constexpr uint32_t kLayoutSweeps = 4;
-// Below this many edges a sweep is a chain of latencies, and a launch per
-// sweep of the row engine is shorter than this engine's with its grid barrier
-// (20 PageRank iterations, 36k edges: 118 against 175 us; 150k: 217 against 170).
+// Below kLayoutEdges edges a sweep is a chain of latencies, and a launch per
+// sweep of the row engine is shorter than this engine's with its grid barrier.
+// Up to kLayoutLocalEdges that holds as well for graphs without long rows,
+// which the row engine cuts into pieces and joins. 20 PageRank iterations, us,
+// row engine / this one: R-MAT of 36k edges 118 / 175, 200k (longest row 4,254)
+// 219 / 176, 400k 354 / 185, 4M 595 / 396; local graphs of 400k edges (longest
+// row 224) 144 / 161, 4M (875) 402 / 419, 8M (1,250) 657 / 715, 16M (1,968)
+// 1,020 / 944, 32M 2,307 / 1,864.
 constexpr uint32_t kLayoutEdges = 65536;
+constexpr uint32_t kLayoutLocalEdges = 12'000'000;
+constexpr uint32_t kLayoutLongRow = 3072;
 
 int build_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout *l) {
     const uint32_t V = g->V, E = g->E;
@@ -184,6 +191,8 @@ int get_pull_layout(gbx_graph *g, uint32_t sweeps, cudaStream_t s, gbx_pull_layo
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     GBX_CUDA(cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone || g->E < kLayoutEdges || g->E > 0x7FFFFFFFu || g->V > kIdMask) return GBX_OK;
+    const uint32_t longest = g->in_offsets ? g->max_in_degree : g->max_out_degree;
+    if (g->E < kLayoutLocalEdges && longest < kLayoutLongRow) return GBX_OK;
     std::lock_guard<std::mutex> lock(g_layout_mutex);
     if (!g->pull_layout && g->pull_layout_tries < 2) {
         g->pull_sweeps += std::min(sweeps, kLayoutSweeps);
