@@ -49,9 +49,9 @@ N_ROOTS = 64
 N_SSSP_ROOTS = 4
 PR_ITERS = 20
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of each
-# kernel, from ncu captures of this workload on a GB300 (profiles/): bfs and
-# sssp one source (--set full), pr one iteration, spmv one launch.
-NCU_TRAFFIC_PER_LAUNCH = {"pr": 0.4006e9, "bfs": 0.1688e9, "sssp": 1.946e9, "spmv": 0.6775e9}
+# kernel, from ncu captures of this workload on a GB300 (profiles/): bfs the 64
+# roots, sssp the mean of the 4 sources, pr the 20 iterations, spmv one sweep.
+NCU_TRAFFIC_PER_LAUNCH = {"pr": 5.664e9, "bfs": 14.48e9, "sssp": 1.706e9, "spmv": 0.5826e9}
 W_LO, W_HI = 1, 255
 # differentiable personalised PageRank: RMAT-20, 2^24 edges as generated,
 # lognormal(0,1) weights, 64 teleport columns of 32 seeds, d 0.85 to 1e-7 L1
@@ -341,8 +341,8 @@ def run_gpu(args):
     def kernels():
         """(name, fn) -> fn returns (traversed edges, algorithmic bytes)"""
         def bfs():
-            # the reference's trial loop: one traversal per root, enqueued
-            # back to back (gbx_bfs_trials), one host synchronisation
+            # the reference's trial loop: one traversal per root, several at
+            # once (gbx_bfs_trials), one host synchronisation
             te = tb = 0
             for st in gbx.breadth_first_search_trials(dg, roots, 2, distances=dist_d, parents=par_d, stream=sp):
                 te += st.edges_traversed
@@ -434,7 +434,7 @@ def run_gpu(args):
                   "frac": round(tb / (ms * 1e-3) / 1e9 / peak, 3), "edges": int(te), "alg_bytes": int(tb)}
         if n in NCU_TRAFFIC_PER_LAUNCH:
             # DRAM bytes one launch moved under ncu, over this run's time per launch
-            per_step = {"bfs": len(roots), "sssp": len(sssp_roots), "pr": PR_ITERS}.get(n, 1)
+            per_step = {"sssp": len(sssp_roots)}.get(n, 1)
             per[n]["dram_frac"] = round(NCU_TRAFFIC_PER_LAUNCH[n] * per_step / (ms * 1e-3) / 1e9 / peak, 3)
         if n == "tc":
             per[n]["merge_bytes"] = int(tc_merge_bytes)
