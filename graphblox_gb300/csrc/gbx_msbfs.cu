@@ -48,12 +48,21 @@ struct MsCounters {
     uint32_t alive[8];          // sources whose next frontier holds any vertex
 };
 
+// Whether the step from the frontier *cur is a push (few out-edges) or a pull.
+// Steps are enqueued before the host knows their frontiers, so the kernels of
+// both kinds look here whether the step is theirs.
+__host__ __device__ __forceinline__ bool ms_pushes(const MsCounters &cur, uint32_t E) {
+    return cur.mf * 16 < E;
+}
+
 // ---- expansion: push ----------------------------------------------------------
 template <int NW>
 __global__ void __launch_bounds__(kMsThreads)
     ms_push_kernel(const uint32_t *__restrict__ off, const uint32_t *__restrict__ dest, const uint32_t *__restrict__ q,
-                   uint32_t qn, const uint32_t *__restrict__ F, const uint32_t *__restrict__ seen,
-                   uint32_t *__restrict__ Fn) {
+                   const MsCounters *__restrict__ cur, uint32_t E, const uint32_t *__restrict__ F,
+                   const uint32_t *__restrict__ seen, uint32_t *__restrict__ Fn) {
+    const uint32_t qn = cur->qn;
+    if (qn == 0 || !ms_pushes(*cur, E)) return;
     constexpr int GPW = 32 / NW;  // groups per warp
     const uint32_t lane = threadIdx.x & 31, k = lane % NW;
     const uint32_t grp = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * GPW + lane / NW;
@@ -91,8 +100,9 @@ __global__ void __launch_bounds__(kMsThreads)
 template <int NW>
 __global__ void __launch_bounds__(kMsThreads)
     ms_pull_light_kernel(const uint32_t *__restrict__ poff, const uint32_t *__restrict__ psrc, uint32_t V, uint32_t S,
-                         const MsCounters *__restrict__ cnt, const uint32_t *__restrict__ F,
+                         const MsCounters *__restrict__ cnt, uint32_t E, const uint32_t *__restrict__ F,
                          const uint32_t *__restrict__ seen, uint32_t *__restrict__ Fn) {
+    if (cnt->qn == 0 || ms_pushes(*cnt, E)) return;
     constexpr int GPW = 32 / NW, kIds = 8 / NW;
     const uint32_t lane = threadIdx.x & 31, k = lane % NW;
     const uint32_t alive = cnt->alive[k] & ms_valid(k, S);
@@ -145,8 +155,9 @@ struct MsChunk {
 template <int NW>
 __global__ void __launch_bounds__(kMsThreads)
     ms_pull_heavy_kernel(const MsChunk *__restrict__ chunks, uint32_t n_chunks, const uint32_t *__restrict__ psrc,
-                         uint32_t S, const MsCounters *__restrict__ cnt, const uint32_t *__restrict__ F,
+                         uint32_t S, const MsCounters *__restrict__ cnt, uint32_t E, const uint32_t *__restrict__ F,
                          const uint32_t *__restrict__ seen, uint32_t *__restrict__ Fn) {
+    if (cnt->qn == 0 || ms_pushes(*cnt, E)) return;
     constexpr int GPW = 32 / NW;
     constexpr int kPer = 8, kEdges = kPer * GPW;             // edges per group and per warp in a round
     constexpr int kLoads = kEdges / 32 > 0 ? kEdges / 32 : 1;
@@ -197,12 +208,15 @@ __global__ void __launch_bounds__(kMsThreads)
 // new = Fn & ~seen; seen |= new; F_next = new (written into Fn, which is kept
 // as this level's mask while levels are stored); v appended to the next
 // frontier list when any bit is new. Past the stored levels (kWriteDist) the
-// distances of the new bits are written here, one by one.
+// distances of the new bits are written here, one by one. Fz is the mask that
+// the step after this one fills, zeroed on the way (or null).
 template <int NW, bool kWriteDist>
 __global__ void __launch_bounds__(kMsThreads)
     ms_update_kernel(uint32_t V, uint32_t S, uint32_t level, const uint32_t *__restrict__ off,
-                     uint32_t *__restrict__ seen, uint32_t *__restrict__ Fn, uint32_t *__restrict__ dist,
-                     uint32_t *__restrict__ qnext, MsCounters *cnt) {
+                     uint32_t *__restrict__ seen, uint32_t *__restrict__ Fn, uint32_t *__restrict__ Fz,
+                     uint32_t *__restrict__ dist, uint32_t *__restrict__ qnext, const MsCounters *cur,
+                     MsCounters *cnt) {
+    if (cur->qn == 0) return;  // the sweep ended before this step
     // next-frontier appends are staged per warp in shared memory; what the
     // warps hold at the end and the out-degree sum go out once per CTA, since
     // atomics on one address take about a nanosecond each, one after the other
@@ -229,6 +243,7 @@ __global__ void __launch_bounds__(kMsThreads)
             nw = Fn[i] & ~s0;
             alive |= nw;
             Fn[i] = nw;
+            if (Fz) Fz[i] = 0;
             if (nw) {
                 seen[i] = s0 | nw;
                 if (kWriteDist) {
@@ -562,6 +577,15 @@ int ms_plan(gbx_graph *g, cudaStream_t s, gbx_ms_plan **out) {
     return GBX_OK;
 }
 
+// Steps enqueued before the host looks: as many as most graphs have levels at
+// first, then fewer, since those past a sweep's end are empty launches. us for
+// 100 sources, one at a time / 2 / 4 / 8: R-MAT of 1,000 vertices 481 / 405 /
+// 376 / 358, 250,000 613 / 543 / 515 / 495; local graph of 30,000 842 / 706 /
+// 684 / 728; RMAT-20 with 256 sources 1,622 / 1,543 / 1,519 / 1,494. Masks above
+// kAheadBytes are not allocated ahead.
+constexpr uint32_t kAhead = 8, kAheadLater = 4;
+constexpr size_t kAheadBytes = size_t(64) << 20;
+
 template <int NW>
 int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, gbx_bfs_result *res_host,
                cudaStream_t s) {
@@ -575,99 +599,126 @@ int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, 
     const uint32_t max_stored = (uint32_t)std::max<size_t>(
         2, std::min<size_t>(kMsMaxStoredLevels, (8ull << 30) / std::max<size_t>(1, words * 4)));
     std::vector<DevBuf<uint32_t>> lvbuf(max_stored);
-    DevBuf<uint32_t> seen, deep[2], q0, q1, rc, rd;
-    DevBuf<unsigned long long> re;
+    DevBuf<uint32_t> seen, deep[2], q0, q1;
+    DevBuf<unsigned long long> per_source;  // edges, then reached vertices and depths, S of each
+    // Steps go out kAhead at a time where a mask is small: a step that is short
+    // against the host's round trip does not wait for one. cnt[j]: the
+    // frontier of the j-th step of a batch.
+    uint32_t ahead = words * 4 <= kAheadBytes ? kAhead : 1;
     DevBuf<MsCounters> cnt;
     GBX_TRY(seen.alloc(words, s));
     GBX_TRY(lvbuf[0].alloc(words, s));
     GBX_TRY(q0.alloc(std::max(V, S), s));
     GBX_TRY(q1.alloc(std::max(V, S), s));
-    GBX_TRY(cnt.alloc(1, s));
+    GBX_TRY(cnt.alloc(ahead + 1, s));
     GBX_CUDA(cudaMemsetAsync(seen.p, 0, words * 4, s));
     GBX_CUDA(cudaMemsetAsync(lvbuf[0].p, 0, words * 4, s));
-    GBX_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(MsCounters), s));
+    GBX_CUDA(cudaMemsetAsync(cnt.p, 0, (ahead + 1) * sizeof(MsCounters), s));
     ms_seed_kernel<<<1, 256, 0, s>>>(src_d, S, NW, g->offsets, seen.p, lvbuf[0].p, q0.p, cnt.p);
     GBX_LAUNCH_CHECK();
-    MsCounters h{};
-    GBX_CUDA(cudaMemcpyAsync(&h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-    GBX_CUDA(cudaStreamSynchronize(s));
-    uint32_t *F = lvbuf[0].p, *q = q0.p, *qn = q1.p;
-    const unsigned grid = (unsigned)num_sms() * 8;
-    const unsigned long long E = g->E;
-    uint32_t level = 0, pushes = 0, pulls = 0, stored = 1;
-    while (h.qn > 0 && level <= V) {
-        const uint32_t next = level + 1;
-        const bool keep = next < max_stored;
-        uint32_t *Fn;
-        if (keep) {
-            GBX_TRY(lvbuf[next].alloc(words, s));
-            Fn = lvbuf[next].p;
-        } else {
-            DevBuf<uint32_t> &d = deep[next & 1];
-            if (!d.p) GBX_TRY(d.alloc(words, s));
-            Fn = d.p;
-        }
+    MsCounters h[kAhead + 1] = {};
+    h[0].qn = S;
+    bool known = ahead == 1;  // the host has read the batch's first frontier
+    if (known) {
+        GBX_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h[0]), cudaMemcpyDeviceToHost, s));
+        GBX_CUDA(cudaStreamSynchronize(s));
+    }
+    // the mask of a level: kept while it fits, else one of two in turn
+    auto mask_of = [&](uint32_t l, uint32_t **out) -> int {
+        DevBuf<uint32_t> &d = l < max_stored ? lvbuf[l] : deep[l & 1];
+        if (!d.p) GBX_TRY(d.alloc(words, s));
+        *out = d.p;
+        return GBX_OK;
+    };
+    uint32_t *F = lvbuf[0].p, *Fn = nullptr, *q = q0.p, *qn = q1.p;
+    if (ahead > 1) {
+        GBX_TRY(mask_of(1, &Fn));
         GBX_CUDA(cudaMemsetAsync(Fn, 0, words * 4, s));
-        if (h.mf * 16 < E) {
-            ms_push_kernel<NW><<<grid, kMsThreads, 0, s>>>(g->offsets, g->dest, q, h.qn, F, seen.p, Fn);
-            GBX_LAUNCH_CHECK();
-            ++pushes;
-        } else {
-            ms_pull_light_kernel<NW><<<grid, kMsThreads, 0, s>>>(g->pull_offsets(), g->pull_src(), V, S, cnt.p, F,
-                                                                 seen.p, Fn);
-            GBX_LAUNCH_CHECK();
-            if (plan->n_chunks) {
-                ms_pull_heavy_kernel<NW><<<grid, kMsThreads, 0, s>>>(plan->chunks, plan->n_chunks, g->pull_src(), S,
-                                                                     cnt.p, F, seen.p, Fn);
+    }
+    // no more CTAs than a small graph's words give work to
+    const unsigned grid = (unsigned)std::min<size_t>((size_t)num_sms() * 8, std::max<size_t>(num_sms(), ceil_div(words, kMsThreads)));
+    const uint32_t E = g->E;
+    uint32_t level = 0, pushes = 0, pulls = 0, stored = 1;
+    while (h[0].qn > 0 && level <= V) {
+        for (uint32_t j = 0; j < ahead; ++j) {
+            const uint32_t next = level + 1 + j;
+            const bool keep = next < max_stored;
+            uint32_t *Fz = nullptr;
+            if (ahead > 1) {
+                GBX_TRY(mask_of(next + 1, &Fz));
+            } else {
+                // large masks: none before it is needed
+                GBX_TRY(mask_of(next, &Fn));
+                GBX_CUDA(cudaMemsetAsync(Fn, 0, words * 4, s));
+            }
+            const MsCounters *cur = cnt.p + j;
+            const bool push = !(known && j == 0) || ms_pushes(h[0], E), pull = !(known && j == 0) || !push;
+            if (push) {
+                ms_push_kernel<NW><<<grid, kMsThreads, 0, s>>>(g->offsets, g->dest, q, cur, E, F, seen.p, Fn);
                 GBX_LAUNCH_CHECK();
             }
-            ++pulls;
+            if (pull) {
+                ms_pull_light_kernel<NW><<<grid, kMsThreads, 0, s>>>(g->pull_offsets(), g->pull_src(), V, S, cur, E, F,
+                                                                     seen.p, Fn);
+                GBX_LAUNCH_CHECK();
+                if (plan->n_chunks) {
+                    ms_pull_heavy_kernel<NW><<<grid, kMsThreads, 0, s>>>(plan->chunks, plan->n_chunks, g->pull_src(),
+                                                                         S, cur, E, F, seen.p, Fn);
+                    GBX_LAUNCH_CHECK();
+                }
+            }
+            if (keep)
+                ms_update_kernel<NW, false><<<grid, kMsThreads, 0, s>>>(V, S, next, g->offsets, seen.p, Fn, Fz, dist,
+                                                                        qn, cur, cnt.p + j + 1);
+            else
+                ms_update_kernel<NW, true><<<grid, kMsThreads, 0, s>>>(V, S, next, g->offsets, seen.p, Fn, Fz, dist,
+                                                                       qn, cur, cnt.p + j + 1);
+            GBX_LAUNCH_CHECK();
+            F = Fn;
+            Fn = Fz;
+            std::swap(q, qn);
         }
-        level = next;
-        GBX_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(MsCounters), s));
-        if (keep) {
-            ms_update_kernel<NW, false><<<grid, kMsThreads, 0, s>>>(V, S, level, g->offsets, seen.p, Fn, dist, qn,
-                                                                    cnt.p);
-            stored = next + 1;
-        } else {
-            ms_update_kernel<NW, true><<<grid, kMsThreads, 0, s>>>(V, S, level, g->offsets, seen.p, Fn, dist, qn,
-                                                                   cnt.p);
-        }
-        GBX_LAUNCH_CHECK();
-        GBX_CUDA(cudaMemcpyAsync(&h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+        GBX_CUDA(cudaMemcpyAsync(h, cnt.p, (ahead + 1) * sizeof(MsCounters), cudaMemcpyDeviceToHost, s));
         GBX_CUDA(cudaStreamSynchronize(s));
-        F = Fn;
-        std::swap(q, qn);
+        uint32_t j = 0;
+        for (; j < ahead && h[j].qn > 0; ++j) {
+            ++(ms_pushes(h[j], E) ? pushes : pulls);
+            ++level;
+            if (level < max_stored) stored = level + 1;
+        }
+        h[0] = h[j];
+        if (h[0].qn > 0) {
+            GBX_CUDA(cudaMemcpyAsync(cnt.p, cnt.p + ahead, sizeof(MsCounters), cudaMemcpyDeviceToDevice, s));
+            GBX_CUDA(cudaMemsetAsync(cnt.p + 1, 0, ahead * sizeof(MsCounters), s));
+        }
+        known = true;
+        ahead = std::min(ahead, kAheadLater);
     }
-    GBX_REQUIRE(h.qn == 0, GBX_ERR_ITER_CAP, "multi-source BFS level cap reached");
+    GBX_REQUIRE(h[0].qn == 0, GBX_ERR_ITER_CAP, "multi-source BFS level cap reached");
     // distances of the stored levels, zeros for unreached pairs, and the
     // per-source results, in one pass
     MsLevels lv{};
     lv.n = stored;
     for (uint32_t L = 0; L < stored; ++L) lv.m[L] = lvbuf[L].p;
-    GBX_TRY(rc.alloc(S, s));
-    GBX_TRY(rd.alloc(S, s));
-    GBX_TRY(re.alloc(S, s));
-    GBX_CUDA(cudaMemsetAsync(rc.p, 0, 4 * (size_t)S, s));
-    GBX_CUDA(cudaMemsetAsync(rd.p, 0, 4 * (size_t)S, s));
-    GBX_CUDA(cudaMemsetAsync(re.p, 0, 8 * (size_t)S, s));
+    GBX_TRY(per_source.alloc(2 * (size_t)S, s));
+    GBX_CUDA(cudaMemsetAsync(per_source.p, 0, 16 * (size_t)S, s));
+    unsigned long long *const re = per_source.p;
+    uint32_t *const rc = reinterpret_cast<uint32_t *>(re + S), *const rd = rc + S;
     const bool vec_rows = S % 4 == 0 && (reinterpret_cast<uintptr_t>(dist) & 15u) == 0;
     const unsigned fgrid = std::min<unsigned>((unsigned)num_sms() * 6, ceil_div((uint64_t)V * NW, kMsThreads));
     if (stored == level + 1 && stored <= 8)
-        ms_planes_kernel<NW, 3><<<fgrid, kMsThreads, 0, s>>>(lv, V, S, g->offsets, src_d, vec_rows, dist, rc.p, re.p, rd.p);
+        ms_planes_kernel<NW, 3><<<fgrid, kMsThreads, 0, s>>>(lv, V, S, g->offsets, src_d, vec_rows, dist, rc, re, rd);
     else if (stored == level + 1 && stored <= 16)
-        ms_planes_kernel<NW, 4><<<fgrid, kMsThreads, 0, s>>>(lv, V, S, g->offsets, src_d, vec_rows, dist, rc.p, re.p, rd.p);
+        ms_planes_kernel<NW, 4><<<fgrid, kMsThreads, 0, s>>>(lv, V, S, g->offsets, src_d, vec_rows, dist, rc, re, rd);
     else
         ms_final_kernel<NW><<<(unsigned)num_sms() * 4, kMsThreads, 0, s>>>(lv, seen.p, V, S, g->offsets, src_d,
-                                                                           vec_rows, dist, rc.p, re.p, rd.p);
+                                                                           vec_rows, dist, rc, re, rd);
     GBX_LAUNCH_CHECK();
     if (res_host) {
-        std::vector<uint32_t> hc(S), hd(S);
-        std::vector<unsigned long long> he(S);
-        GBX_CUDA(cudaMemcpyAsync(hc.data(), rc.p, 4 * (size_t)S, cudaMemcpyDeviceToHost, s));
-        GBX_CUDA(cudaMemcpyAsync(hd.data(), rd.p, 4 * (size_t)S, cudaMemcpyDeviceToHost, s));
-        GBX_CUDA(cudaMemcpyAsync(he.data(), re.p, 8 * (size_t)S, cudaMemcpyDeviceToHost, s));
+        std::vector<unsigned long long> he(2 * (size_t)S);
+        GBX_CUDA(cudaMemcpyAsync(he.data(), re, 16 * (size_t)S, cudaMemcpyDeviceToHost, s));
         GBX_CUDA(cudaStreamSynchronize(s));
+        const uint32_t *hc = reinterpret_cast<const uint32_t *>(he.data() + S), *hd = hc + S;
         for (uint32_t i = 0; i < S; ++i) {
             gbx_bfs_result r{};
             r.processed_nodes = hc[i] + 1;
