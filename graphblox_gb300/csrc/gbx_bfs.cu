@@ -832,8 +832,9 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_teams_kernel(BfsTeams t) {
 // too). Above kSmallEdges one SM's throughput loses against 152.
 constexpr int kSmallThreads = 1024;
 constexpr uint32_t kSmallWords = 2048;  // V <= 65,536
-// 8,000-vertex R-MAT graph, 80k edges: 38 us against 54 for one traversal;
-// 16,000 and 160k: 62 against 58; crawl graph of 80k edges: 138 against 136.
+// A call, us, persistent kernel / this one: R-MAT of 10k edges 62 / 37, 60k
+// 62 / 46; local graphs of 10k edges 61 / 34, 60k 90 / 65. At 160k edges this
+// kernel took 62, the other 58.
 constexpr uint32_t kSmallEdges = 65536;
 constexpr uint32_t kSmallBatch = 64;  // traversals per launch, one CTA each
 constexpr uint32_t kSmallHub = 128;   // out-degree above which the whole CTA takes a row

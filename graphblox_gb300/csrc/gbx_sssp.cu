@@ -617,7 +617,7 @@ __global__ void sssp_finish_kernel(const uint32_t *dist, const uint32_t *outdeg,
 }
 
 // ---- small graphs: one CTA ---------------------------------------------------
-// As for BFS (gbx_bfs.cu): a round of the persistent kernel costs 10 to 12 us
+// As for BFS (gbx_bfs.cu): a round of the persistent kernel costs 5 to 12 us
 // however little it holds. One CTA keeps distances and frontier bitmaps in
 // shared memory and relaxes the whole frontier every round (no buckets: a
 // small graph has few rounds, and a vertex relaxed early is relaxed again),
@@ -625,7 +625,8 @@ __global__ void sssp_finish_kernel(const uint32_t *dist, const uint32_t *outdeg,
 // The distances are the same fixed point.
 constexpr int kSsspSmallThreads = 1024;
 constexpr uint32_t kSsspSmallV = 24576;  // 96 KB of distances
-// R-MAT, 1,000 vertices, 10k edges: 172 -> 72 us; 4,000 and 40k: 175 -> 184.
+// A call, us, persistent kernel / this one: R-MAT of 10k edges 148 / 72, 24k 148 / 95; local graphs 159 / 98, 186 / 156.
+// At 40k edges this one took 184, the persistent one takes 149.
 constexpr uint32_t kSsspSmallE = 24576;
 constexpr uint32_t kSsspSmallHub = 128;  // out-degree above which the whole CTA takes a row
 constexpr uint32_t kSsspSmallHubs = 1024;
