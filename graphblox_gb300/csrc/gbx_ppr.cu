@@ -20,7 +20,7 @@
 // Layout: R, Lam, T, W are [V][K] row-major, K = 32*KPL (32..256), so one
 // gathered neighbour row is K*4 contiguous bytes read by one warp with a
 // KPL-float vector load per lane. Rows are dealt as chunks of at most
-// kPprChunk edges, one warp per chunk (a per-direction chunk table); a row
+// ppr_chunk(E) edges, one warp per chunk (a per-direction chunk table); a row
 // cut into several chunks writes K-wide partial sums that a second kernel
 // adds in chunk order, so every result is deterministic. The iteration loop
 // runs without host round trips: a one-block check kernel turns the
@@ -42,7 +42,15 @@
 
 namespace gbx {
 
-constexpr uint32_t kPprChunk = 256;
+// Edges to a chunk: a chunk is one warp's chain of neighbour rows, eight at a
+// time, so short chunks shorten a sweep; shorter ones yet put more partial sums
+// through memory. ms a training pass with 256 / 128 / 64 / 32, R-MAT, 64 columns:
+// 10k edges 4.4 / 3.6 / 3.2 / 2.8, 160k 7.3 / 5.3 / 4.7 / 4.9, 540k 10.5 / 8.0 /
+// 7.0 / 7.4, 2.5M 24.6 / 21.7 / 22.6 / 27.5, 16M 104.7 / 101.2 / 103.4 / 112.2;
+// local graphs: 180k 5.2 / 5.0 / 4.5 / 4.6, 3M with 32 columns 16.7 / 17.1 / 17.6.
+constexpr uint32_t kPprChunk = 128, kPprChunkSmall = 64;
+constexpr uint32_t kPprSmallEdges = 1'000'000;
+inline uint32_t ppr_chunk(uint32_t E) { return E <= kPprSmallEdges ? kPprChunkSmall : kPprChunk; }
 constexpr int kPprThreads = 256;
 constexpr int kPprWarps = kPprThreads / 32;
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
@@ -52,8 +60,8 @@ struct PprChunk {
     uint32_t row, eb, ee, slot;  // slot: partial-sum slot, kNoSlot when the chunk is the whole row
 };
 
-// Chunk table of one CSR direction: whole rows up to kPprChunk edges, longer
-// rows cut into kPprChunk pieces with one partial slot each.
+// Chunk table of one CSR direction: whole rows up to ppr_chunk(E) edges, longer
+// rows cut into pieces of as many, with one partial slot each.
 struct PprPlan {
     PprChunk *chunks = nullptr;       // device
     uint32_t *split_rows = nullptr;   // device: rows cut into several chunks
@@ -81,16 +89,17 @@ static int build_ppr_plan(const uint32_t *d_off, uint32_t V, cudaStream_t s, Ppr
     GBX_CUDA(cudaStreamSynchronize(s));
     std::vector<PprChunk> ch;
     std::vector<uint32_t> srows, sfirst;
-    ch.reserve(V + off[V] / kPprChunk + 1);
+    const uint32_t chunk = ppr_chunk(off[V]);
+    ch.reserve(V + off[V] / chunk + 1);
     uint32_t slot = 0;
     for (uint32_t v = 0; v < V; ++v) {
         const uint32_t b = off[v], e = off[v + 1];
-        if (e - b <= kPprChunk) {
+        if (e - b <= chunk) {
             ch.push_back({v, b, e, kNoSlot});
         } else {
             srows.push_back(v);
             sfirst.push_back(slot);
-            for (uint32_t c = b; c < e; c += kPprChunk) ch.push_back({v, c, std::min(c + kPprChunk, e), slot++});
+            for (uint32_t c = b; c < e; c += chunk) ch.push_back({v, c, std::min(c + chunk, e), slot++});
         }
     }
     sfirst.push_back(slot);
