@@ -39,7 +39,6 @@ struct gbx_batch {
     uint32_t *in_src = nullptr;      // E or null
     uint32_t *order = nullptr;       // G, graph ids by descending edge count
     std::vector<uint32_t> h_vbase;   // host copy of vbase
-    std::vector<uint32_t> h_edges;   // edges per graph
     // PageRank's in-edge words (built by its first call): graph g's start
     // wbase[g] units of 16 bytes into words, its rows with edges at rows + vbase[g]
     uint4 *words = nullptr;
@@ -618,6 +617,12 @@ __global__ void __launch_bounds__(kBpThreads, 1) pr_batched_kernel(BpArgs a) {
     }
 }
 
+// first_edge[g]: graph g's first in-edge; first_edge[G]: past the last graph's
+__global__ void bp_bounds_kernel(const uint32_t *vbase, uint32_t G, const uint32_t *poff, uint32_t *first_edge) {
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g <= G; g += gridDim.x * blockDim.x)
+        first_edge[g] = poff[vbase[g]];
+}
+
 // One CTA lays a graph's words out.
 __global__ void __launch_bounds__(kBpThreads)
     bp_layout_kernel(uint32_t G, const uint32_t *order, const uint32_t *vbase, const uint32_t *off, const uint32_t *poff, const uint32_t *psrc,
@@ -750,8 +755,7 @@ int batch_create(gbx_batch *b, uint32_t G, const uint32_t *vertex_base, const ui
     std::vector<uint32_t> order(G);
     std::vector<uint64_t> eg(G);
     for (uint32_t g = 0; g < G; ++g) {
-        b->h_edges.push_back(off[vb[g + 1]] - off[vb[g]]);
-        eg[g] = (uint64_t)b->h_edges[g] + (vb[g + 1] - vb[g]);
+        eg[g] = (uint64_t)(off[vb[g + 1]] - off[vb[g]]) + (vb[g + 1] - vb[g]);
         b->max_v = std::max(b->max_v, vb[g + 1] - vb[g]);
     }
     std::iota(order.begin(), order.end(), 0u);
@@ -811,12 +815,22 @@ int bp_layout(gbx_batch *b, cudaStream_t s) {
     std::lock_guard<std::mutex> lock(b->words_mutex);
     if (b->starts) return GBX_OK;
     const uint32_t smem_v = bp_smem_v(b);
+    // The words are the in-edges, which a graph may have more or fewer of than
+    // out-edges: a caller's in-edge CSR need not be the forward one's transpose.
+    std::vector<uint32_t> first_edge((size_t)b->G + 1);
+    DevBuf<uint32_t> bounds;
+    GBX_TRY(bounds.alloc(first_edge.size(), s));
+    bp_bounds_kernel<<<std::min<unsigned>(ceil_div(first_edge.size(), 256), (unsigned)num_sms() * 8), 256, 0, s>>>(
+        b->vbase, b->G, b->poff(), bounds.p);
+    GBX_LAUNCH_CHECK();
+    GBX_CUDA(cudaMemcpyAsync(first_edge.data(), bounds.p, first_edge.size() * 4, cudaMemcpyDeviceToHost, s));
+    GBX_CUDA(cudaStreamSynchronize(s));
     std::vector<uint32_t> wbase(b->G);
     uint64_t at = 0;
     for (uint32_t g = 0; g < b->G; ++g) {
-        const uint32_t v = b->h_vbase[g + 1] - b->h_vbase[g];
+        const uint32_t v = b->h_vbase[g + 1] - b->h_vbase[g], edges = first_edge[g + 1] - first_edge[g];
         wbase[g] = (uint32_t)at;
-        at += ((uint64_t)b->h_edges[g] + 255) / 256 * (v <= kBpShortV && ((v + 31) & ~31u) <= smem_v ? 32 : 64);
+        at += ((uint64_t)edges + 255) / 256 * (v <= kBpShortV && ((v + 31) & ~31u) <= smem_v ? 32 : 64);
     }
     auto build = [&]() -> int {
         GBX_TRY(dev_alloc((void **)&b->words, std::max<uint64_t>(at, 1) * sizeof(uint4), s));
