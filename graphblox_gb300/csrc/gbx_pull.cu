@@ -167,6 +167,7 @@ int build_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout *l) {
     GBX_TRY(dev_alloc((void **)&l->hot_ids, (size_t)std::max(l->hot, 1u) * 4, s));
     GBX_TRY(dev_alloc((void **)&l->rows, (size_t)std::max(l->n_rows, 1u) * sizeof(uint2), s));
     GBX_TRY(dev_alloc((void **)&l->units, ((size_t)l->n_units + 1) * sizeof(uint4), s));
+    GBX_TRY(dev_alloc((void **)&l->work, pull_work_words(*l) * 4, s));
     GBX_CUDA(cudaMemsetAsync(l->edges + E, 0, kPullPad * 4, s));
     if (l->hot) GBX_CUDA(cudaMemsetAsync(l->hot_ids, 0xFF, (size_t)l->hot * 4, s));
     pull_rows_kernel<<<grid, 256, 0, s>>>(has.p, row_pos.p, hot.p, slot_pos.p, V, l->rows, l->hot_ids, word.p);
@@ -188,13 +189,13 @@ std::mutex g_layout_mutex;
 
 int get_pull_layout(gbx_graph *g, uint32_t sweeps, cudaStream_t s, gbx_pull_layout **out) {
     *out = nullptr;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    GBX_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (cap != cudaStreamCaptureStatusNone || g->E < kLayoutEdges || g->E > 0x7FFFFFFFu || g->V > kIdMask) return GBX_OK;
+    if (g->E < kLayoutEdges || g->E > 0x7FFFFFFFu || g->V > kIdMask) return GBX_OK;
     const uint32_t longest = g->in_offsets ? g->max_in_degree : g->max_out_degree;
     if (g->E < kLayoutLocalEdges && longest < kLayoutLongRow) return GBX_OK;
+    bool captured = false;
+    GBX_TRY(is_capturing(s, &captured));
     std::lock_guard<std::mutex> lock(g_layout_mutex);
-    if (!g->pull_layout && g->pull_layout_tries < 2) {
+    if (!g->pull_layout && !captured && g->pull_layout_tries < 2) {
         g->pull_sweeps += std::min(sweeps, kLayoutSweeps);
         if (g->pull_sweeps < kLayoutSweeps) return GBX_OK;
         gbx_pull_layout *l = new gbx_pull_layout();
@@ -223,5 +224,6 @@ void gbx_free_pull_layout(gbx_pull_layout *l) {
     gbx::dev_free(l->hot_ids);
     gbx::dev_free(l->rows);
     gbx::dev_free(l->units);
+    gbx::dev_free(l->work);
     delete l;
 }

@@ -37,6 +37,8 @@
 // us, SpMV 427 -> 209 us; SpMV over 150M crawl edges 640 -> 425 us.
 #pragma once
 
+#include <algorithm>
+
 #include "gbx_coop.cuh"
 #include "gbx_gather.cuh"
 
@@ -56,6 +58,9 @@ struct gbx_pull_layout {
     // device [n_units + 1]: {first edge, row of that edge, the unit where that
     // row begins when it is cut (else ~0), units of the cut row}
     uint4 *units = nullptr;
+    // device [pull_work_words]: working memory of captured SpMV calls (the
+    // graph that a capture makes outlives any allocation of the call)
+    float *work = nullptr;
 };
 
 __host__ __device__ inline uint32_t pull_unit_edge(const gbx_pull_layout &l, uint32_t t) {
@@ -88,6 +93,13 @@ struct PullPieces {
     float *sums;
     unsigned *tickets;
 };
+
+// Working memory of SpMV sweeps, one run of words: the slots' values, piece
+// sums, then tickets and cursors (zeroed by the call).
+constexpr uint32_t kPullCursors = 64;
+inline size_t pull_work_words(const gbx_pull_layout &l) {
+    return (size_t)std::max(l.hot, 4u) + 3 * (size_t)l.n_units + kPullCursors;
+}
 
 // Term:  const float *cold            values by vertex
 //        struct Factors; void factors(uint32_t e, uint32_t e0, uint32_t e1, Factors &)   of edges e..e+3
@@ -323,7 +335,15 @@ __device__ __forceinline__ void load_hot(const float *values, uint32_t hot, floa
 }
 
 // The layout of g's pull CSR when `sweeps` more sweeps make it worth having
-// (or it is there already); *out null: use the row engine of gbx_gather.cuh.
+// (or it is there already; nothing is built while s captures); *out null: use
+// the row engine of gbx_gather.cuh.
 int get_pull_layout(gbx_graph *g, uint32_t sweeps, cudaStream_t s, gbx_pull_layout **out);
+
+inline int is_capturing(cudaStream_t s, bool *yes) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GBX_CUDA(cudaStreamIsCapturing(s, &cap));
+    *yes = cap != cudaStreamCaptureStatusNone;
+    return GBX_OK;
+}
 
 }  // namespace gbx

@@ -81,24 +81,29 @@ __global__ void __launch_bounds__(kPullThreads, 1)
     deal_units(sweep, cursor, first);
 }
 
-// Working memory is the call's own: calls on one graph may overlap.
+// Working memory is the call's own, so that sweeps of one graph on several
+// streams do not meet; a captured call's is the layout's.
 static int spmv_run_hot(const gbx_pull_layout &l, SpmvHotTerm term, float *y, uint32_t iterations, cudaStream_t s) {
-    DevBuf<float> hot_x, sums;
-    DevBuf<unsigned> tickets;  // then one cursor per iteration
-    GBX_TRY(hot_x.alloc(std::max(l.hot, 4u), s));
-    GBX_TRY(sums.alloc(2 * (size_t)l.n_units, s));
-    GBX_TRY(tickets.alloc((size_t)l.n_units + iterations, s));
-    GBX_CUDA(cudaMemsetAsync(tickets.p, 0, ((size_t)l.n_units + iterations) * sizeof(unsigned), s));
+    bool captured = false;
+    GBX_TRY(is_capturing(s, &captured));
+    DevBuf<float> own;
+    if (!captured) GBX_TRY(own.alloc(pull_work_words(l), s));
+    float *const hot_x = captured ? l.work : own.p, *const sums = hot_x + std::max(l.hot, 4u);
+    unsigned *const tickets = reinterpret_cast<unsigned *>(sums + 2 * (size_t)l.n_units);
+    unsigned *const cursors = tickets + l.n_units;
+    GBX_CUDA(cudaMemsetAsync(tickets, 0, ((size_t)l.n_units + kPullCursors) * sizeof(unsigned), s));
     if (l.hot) {
-        spmv_hot_values_kernel<<<ceil_div(l.hot, 256), 256, 0, s>>>(term.cold, l.hot_ids, l.hot, l.V, hot_x.p);
+        spmv_hot_values_kernel<<<ceil_div(l.hot, 256), 256, 0, s>>>(term.cold, l.hot_ids, l.hot, l.V, hot_x);
         GBX_LAUNCH_CHECK();
     }
     const size_t smem = pull_smem(l);
     GBX_CUDA(cudaFuncSetAttribute(spmv_hot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned ctas = std::min<unsigned>((unsigned)num_sms(), ceil_div(l.n_units, kPullWarps));
     for (uint32_t it = 0; it < iterations; ++it) {
-        spmv_hot_kernel<<<ctas, kPullThreads, smem, s>>>(l, hot_x.p, term, SpmvHotEpi{y},
-                                                         PullPieces{sums.p, tickets.p}, tickets.p + l.n_units + it);
+        const uint32_t at = it % kPullCursors;
+        if (it && at == 0) GBX_CUDA(cudaMemsetAsync(cursors, 0, kPullCursors * sizeof(unsigned), s));
+        spmv_hot_kernel<<<ctas, kPullThreads, smem, s>>>(l, hot_x, term, SpmvHotEpi{y}, PullPieces{sums, tickets},
+                                                         cursors + at);
         GBX_LAUNCH_CHECK();
     }
     return GBX_OK;
