@@ -238,10 +238,10 @@ struct gbx_graph {
     struct gbx_ms_plan *ms_plan = nullptr;
     // PageRank working memory (gbx_pagerank.cu)
     struct gbx_pr_cache *pr_cache = nullptr;
-    // hot-table pull engine (gbx_pull.cu): its layout, the sweeps asked for
-    // before it was built, and attempts that found no memory for it
+    // hot-table pull engine (gbx_pull.cu): its layout, and attempts that found
+    // no memory for it
     struct gbx_pull_layout *pull_layout = nullptr;
-    uint32_t pull_sweeps = 0, pull_layout_tries = 0;
+    uint32_t pull_layout_tries = 0;
     // betweenness centrality: successor CSR with ascending rows (gbx_bc.cu)
     struct gbx_bc_cache *bc_cache = nullptr;
     // device scratch lent to one synchronous call at a time (gbx::Scratch)
@@ -332,6 +332,9 @@ struct Scratch {
 // plan for the pull CSR of g (built on first use, cached on the graph)
 int get_pull_plan(gbx_graph *g, cudaStream_t s, gbx_gather_plan **plan);
 void free_plan(gbx_gather_plan *p);
+// gbx_pagerank_pull's work; by_rows: on the row engine whatever the graph
+int pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon, float *ranks, gbx_pr_result *result,
+                  cudaStream_t s, bool by_rows);
 // device-wide exclusive scans (gbx_scan.cu); temp storage is internal
 int exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint32_t n, cudaStream_t s,
                        uint32_t *total_dev /* may be null */);

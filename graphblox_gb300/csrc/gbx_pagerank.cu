@@ -11,11 +11,10 @@
 // reproduces the reference's early exit (stats->iterations = the index of the
 // iteration with no active vertex). A final kernel divides by N (:344-350).
 //
-// From kLayoutSweeps iterations on (over all calls on the graph) the sweeps
-// run on the hot-table engine (gbx_pull.cuh) in one persistent kernel, one
-// CTA per SM: each iteration loads the hot sources' contributions into shared
-// memory, deals the edge units and ends at a grid barrier. Fewer iterations,
-// and those of small graphs, run as one launch each on the row engine
+// The sweeps run on the hot-table engine (gbx_pull.cuh) in one persistent
+// kernel, one CTA per SM: each iteration loads the hot sources' contributions
+// into shared memory, deals the edge units and ends at a grid barrier. Those
+// of small and some local graphs run as one launch each on the row engine
 // (gbx_gather.cuh), which needs no layout; that loop (state reset, initial
 // ranks, the iterations) is captured once per graph and (max_iterations,
 // epsilon) as a CUDA graph and replayed by every later call. With epsilon = 0 no iteration's residual but the last is asked for,
@@ -404,17 +403,11 @@ int pr_run_hot(gbx_graph *g, const gbx_pull_layout &l, uint32_t max_it, double e
 
 }  // namespace
 
-extern "C" int gbx_pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon,
-                                 float *ranks, gbx_pr_result *result, void *stream) {
-    clear_error();
-    GBX_REQUIRE(g && ranks, GBX_ERR_INVALID, "graph or ranks is NULL");
-    GBX_REQUIRE(epsilon >= 0.0, GBX_ERR_INVALID, "epsilon must be >= 0");
-    GBX_TRY(ensure_device());
-    cudaStream_t s = (cudaStream_t)stream;
+int gbx::pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon, float *ranks, gbx_pr_result *result,
+                       cudaStream_t s, bool by_rows) {
     const uint32_t V = g->V;
     gbx_pull_layout *layout = nullptr;
-    GBX_TRY(get_pull_layout(g, max_iterations, s, &layout));
-    if (max_iterations == 0) layout = nullptr;
+    if (max_iterations && !by_rows) GBX_TRY(get_pull_layout(g, s, &layout));
     gbx_gather_plan *plan = nullptr;
     if (!layout) GBX_TRY(get_pull_plan(g, s, &plan));
     OutArray<float> out;
@@ -442,4 +435,13 @@ extern "C" int gbx_pagerank_pull(gbx_graph *g, uint32_t max_iterations, double e
     }
     if (result) *result = h.res;
     return GBX_OK;
+}
+
+extern "C" int gbx_pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon,
+                                 float *ranks, gbx_pr_result *result, void *stream) {
+    clear_error();
+    GBX_REQUIRE(g && ranks, GBX_ERR_INVALID, "graph or ranks is NULL");
+    GBX_REQUIRE(epsilon >= 0.0, GBX_ERR_INVALID, "epsilon must be >= 0");
+    GBX_TRY(ensure_device());
+    return pagerank_pull(g, max_iterations, epsilon, ranks, result, (cudaStream_t)stream, false);
 }

@@ -4,8 +4,9 @@
 // CSR, exactly so with an inverse CSR or a symmetric graph and a fair guess
 // otherwise -- gives the degree from which on vertices get a slot; slots and
 // rows with edges are numbered by prefix sums, and one pass rewrites the edge
-// ids as words. That pass is a gather per edge, so building costs about 1.3
-// sweeps of the row engine, and a sweep then saves almost half of one.
+// ids as words: it looks every source up in a bitmap of V / 8 bytes, which L1
+// serves far better than a word per vertex, and only sources with a slot in
+// their slot's number.
 #include <algorithm>
 #include <mutex>
 #include <vector>
@@ -39,33 +40,44 @@ __global__ void degree_bins_kernel(const uint32_t *deg, uint32_t V, uint32_t *bi
 }
 
 __global__ void pull_flags_kernel(const uint32_t *off, const uint32_t *deg, uint32_t V, uint32_t hot_bin,
-                                  uint32_t *has_edges, uint32_t *is_hot) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-        has_edges[v] = off[v + 1] != off[v];
-        is_hot[v] = degree_bin(deg[v]) >= hot_bin;
+                                  uint32_t *has_edges, uint32_t *is_hot, uint32_t *hot_bits) {
+    const uint32_t step = gridDim.x * blockDim.x;  // a multiple of 32: a warp's lanes hold a word's 32 vertices
+    for (uint64_t v0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; v0 < V; v0 += step) {
+        const uint64_t v = v0 + (threadIdx.x & 31);
+        const bool hot = v < V && degree_bin(deg[v]) >= hot_bin;
+        if (v < V) {
+            has_edges[v] = off[v + 1] != off[v];
+            is_hot[v] = hot;
+        }
+        const unsigned bits = __ballot_sync(0xffffffffu, hot);
+        if ((threadIdx.x & 31) == 0) hot_bits[v0 / 32] = bits;
     }
 }
 
-// rows and slots; word[v] = what an edge from v carries
+// rows and slots
 __global__ void pull_rows_kernel(const uint32_t *has_edges, const uint32_t *row_pos, const uint32_t *is_hot,
-                                 const uint32_t *slot_pos, uint32_t V, uint2 *rows, uint32_t *hot_ids, uint32_t *word) {
+                                 const uint32_t *slot_pos, uint32_t V, uint2 *rows, uint32_t *hot_ids) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
         const bool hot = is_hot[v];
         const uint32_t slot = hot ? slot_pos[v] : ~0u;
         if (has_edges[v]) rows[row_pos[v]] = make_uint2(v, slot);
         if (hot) hot_ids[slot] = v;
-        word[v] = hot ? slot | kPullHot : v;
     }
 }
 
-__global__ void pull_words_kernel(const uint32_t *src, uint32_t E, const uint32_t *word, uint32_t *edges) {
+// what an edge carries: its source, or its source's slot
+__global__ void pull_words_kernel(const uint32_t *src, uint32_t E, const uint32_t *hot_bits, const uint32_t *slot_pos,
+                                  uint32_t *edges) {
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += 8 * step) {
-        uint32_t u[8];
+        uint32_t u[8], bits[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) u[q] = i + q * step < E ? __ldcs(src + i + q * step) : 0u;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) u[q] = __ldg(word + u[q]);
+        for (int q = 0; q < 8; ++q) bits[q] = __ldg(hot_bits + (u[q] >> 5));
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if ((bits[q] >> (u[q] & 31)) & 1u) u[q] = __ldg(slot_pos + u[q]) | kPullHot;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
             if (i + q * step < E) __stcs(edges + i + q * step, u[q]);
@@ -101,8 +113,6 @@ __global__ void pull_units_kernel(const uint32_t *off, const uint32_t *row_pos, 
     }
 }
 
-// Sweeps after which a layout has paid for itself.
-constexpr uint32_t kLayoutSweeps = 4;
 // Below kLayoutEdges edges a sweep is a chain of latencies, and a launch per
 // sweep of the row engine is shorter than this engine's with its grid barrier.
 // Up to kLayoutLocalEdges that holds as well for graphs without long rows,
@@ -110,7 +120,10 @@ constexpr uint32_t kLayoutSweeps = 4;
 // row engine / this one: R-MAT of 36k edges 118 / 175, 200k (longest row 4,254)
 // 219 / 176, 400k 354 / 185, 4M 595 / 396; local graphs of 400k edges (longest
 // row 224) 144 / 161, 4M (875) 402 / 419, 8M (1,250) 657 / 715, 16M (1,968)
-// 1,020 / 944, 32M 2,307 / 1,864.
+// 1,020 / 944, 32M 2,307 / 1,864. A graph's first SpMV, us, with the row plan
+// and a row sweep / with the layout and its sweep: R-MAT of 400k edges 255 / 193,
+// 3M 295 / 199, 16M 409 / 287, 64M 775 / 676; crawl of 16M edges 335 / 278, 48M
+// 516 / 520, 142M 1,030 / 1,084 (the second call: 661 / 452).
 constexpr uint32_t kLayoutEdges = 65536;
 constexpr uint32_t kLayoutLocalEdges = 12'000'000;
 constexpr uint32_t kLayoutLongRow = 3072;
@@ -121,14 +134,14 @@ int build_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout *l) {
     l->V = V;
     l->E = E;
     const int grid = (int)std::min<uint64_t>((V + 255) / 256, (uint64_t)num_sms() * 8);
-    DevBuf<uint32_t> bins, has, hot, row_pos, slot_pos, tot, word;
+    DevBuf<uint32_t> bins, has, hot, hot_bits, row_pos, slot_pos, tot;
     GBX_TRY(bins.alloc(kDegreeBins, s));
     GBX_TRY(has.alloc(V, s));
     GBX_TRY(hot.alloc(V, s));
     GBX_TRY(row_pos.alloc(V, s));
     GBX_TRY(slot_pos.alloc(V, s));
     GBX_TRY(tot.alloc(2, s));
-    GBX_TRY(word.alloc(V, s));
+    GBX_TRY(hot_bits.alloc(ceil_div(V, 32), s));
     GBX_CUDA(cudaMemsetAsync(bins.p, 0, kDegreeBins * 4, s));
     degree_bins_kernel<<<std::min(grid, num_sms() * 2), 256, 0, s>>>(g->out_degree, V, bins.p);
     GBX_LAUNCH_CHECK();
@@ -142,7 +155,7 @@ int build_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout *l) {
     uint32_t bin = kDegreeBins, slots = 0;
     while (bin > 1 && slots + count[bin - 1] <= most) slots += count[--bin];
     l->hot = (slots + 3) & ~3u;
-    pull_flags_kernel<<<grid, 256, 0, s>>>(off, g->out_degree, V, bin, has.p, hot.p);
+    pull_flags_kernel<<<grid, 256, 0, s>>>(off, g->out_degree, V, bin, has.p, hot.p, hot_bits.p);
     GBX_LAUNCH_CHECK();
     GBX_TRY(exclusive_scan_u32(has.p, row_pos.p, V, s, tot.p));
     GBX_TRY(exclusive_scan_u32(hot.p, slot_pos.p, V, s, tot.p + 1));
@@ -170,10 +183,10 @@ int build_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout *l) {
     GBX_TRY(dev_alloc((void **)&l->work, pull_work_words(*l) * 4, s));
     GBX_CUDA(cudaMemsetAsync(l->edges + E, 0, kPullPad * 4, s));
     if (l->hot) GBX_CUDA(cudaMemsetAsync(l->hot_ids, 0xFF, (size_t)l->hot * 4, s));
-    pull_rows_kernel<<<grid, 256, 0, s>>>(has.p, row_pos.p, hot.p, slot_pos.p, V, l->rows, l->hot_ids, word.p);
+    pull_rows_kernel<<<grid, 256, 0, s>>>(has.p, row_pos.p, hot.p, slot_pos.p, V, l->rows, l->hot_ids);
     GBX_LAUNCH_CHECK();
     const int egrid = (int)std::min<uint64_t>((E + 2047ull) / 2048, (uint64_t)num_sms() * 8);
-    pull_words_kernel<<<egrid, 256, 0, s>>>(g->pull_src(), E, word.p, l->edges);
+    pull_words_kernel<<<egrid, 256, 0, s>>>(g->pull_src(), E, hot_bits.p, slot_pos.p, l->edges);
     GBX_LAUNCH_CHECK();
     pull_ends_kernel<<<grid, 256, 0, s>>>(off, V, l->edges);
     GBX_LAUNCH_CHECK();
@@ -187,7 +200,7 @@ std::mutex g_layout_mutex;
 
 }  // namespace
 
-int get_pull_layout(gbx_graph *g, uint32_t sweeps, cudaStream_t s, gbx_pull_layout **out) {
+int get_pull_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout **out) {
     *out = nullptr;
     if (g->E < kLayoutEdges || g->E > 0x7FFFFFFFu || g->V > kIdMask) return GBX_OK;
     const uint32_t longest = g->in_offsets ? g->max_in_degree : g->max_out_degree;
@@ -196,8 +209,6 @@ int get_pull_layout(gbx_graph *g, uint32_t sweeps, cudaStream_t s, gbx_pull_layo
     GBX_TRY(is_capturing(s, &captured));
     std::lock_guard<std::mutex> lock(g_layout_mutex);
     if (!g->pull_layout && !captured && g->pull_layout_tries < 2) {
-        g->pull_sweeps += std::min(sweeps, kLayoutSweeps);
-        if (g->pull_sweeps < kLayoutSweeps) return GBX_OK;
         gbx_pull_layout *l = new gbx_pull_layout();
         const int st = build_layout(g, s, l);
         if (st == GBX_OK) {

@@ -1,6 +1,7 @@
 // Hot-table pull engine: the repeated form of the pull sweep of
-// gbx_gather.cuh, for graphs that are swept more than a few times (PageRank's
-// iterations, repeated SpMV).
+// gbx_gather.cuh. Which of the two a graph gets depends on the graph alone
+// (get_pull_layout), so that equal calls give equal bits whatever was called
+// before them.
 //
 // What bounds a pull sweep is the gather of one 4-byte value per edge. An
 // access that misses L1 costs one 32-byte sector from L2, and an SM gets one
@@ -334,10 +335,9 @@ __device__ __forceinline__ void load_hot(const float *values, uint32_t hot, floa
     __syncthreads();
 }
 
-// The layout of g's pull CSR when `sweeps` more sweeps make it worth having
-// (or it is there already; nothing is built while s captures); *out null: use
-// the row engine of gbx_gather.cuh.
-int get_pull_layout(gbx_graph *g, uint32_t sweeps, cudaStream_t s, gbx_pull_layout **out);
+// The layout of g's pull CSR, built on first use (not while s captures); *out
+// null: the graph's sweeps run on the row engine of gbx_gather.cuh.
+int get_pull_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout **out);
 
 inline int is_capturing(cudaStream_t s, bool *yes) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;

@@ -1,9 +1,8 @@
 // SpMV pull (the reference's SPMVPullGraphCSR, SPMV.c:117-215):
 // y[v] += sum over pull edges (u->v) of w_uv * x[u], repeated `iterations`
-// times with y never reset. The pull engine (gbx_gather.cuh) computes each
-// row's sum (Kahan-compensated on medium and heavy rows) and adds it to y;
-// from the fourth sweep of a graph on the hot-table engine (gbx_pull.cuh) does,
-// with the hot vertices' x gathered once per call.
+// times with y never reset. The hot-table engine (gbx_pull.cuh), with the hot
+// vertices' x gathered once per call, or for small and some local graphs the
+// row engine (gbx_gather.cuh) computes each row's sum and adds it to y.
 #include <algorithm>
 
 #include "gbx_pull.cuh"
@@ -121,7 +120,7 @@ extern "C" int gbx_spmv(gbx_graph *g, const float *values, float default_value, 
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t V = g->V;
     gbx_pull_layout *layout = nullptr;
-    GBX_TRY(get_pull_layout(g, iterations, s, &layout));
+    if (iterations) GBX_TRY(get_pull_layout(g, s, &layout));
     gbx_gather_plan *plan = nullptr;
     if (!layout) GBX_TRY(get_pull_plan(g, s, &plan));
     InArray<float> xin, vin;

@@ -5,8 +5,9 @@
 //               unexplored edges / alpha (the reference fixes 15, BFS.c:374)
 //   bfs_beta    stay bottom-up while the frontier exceeds V / beta (18)
 //   sssp_delta  bucket width of the near/far schedule
-//   pull_heavy_min  in-degree above which the pull engine (PR, SpMV) cuts a
-//               row into CTA-sized chunks (rows of 33 up to it get a warp)
+//   pull_heavy_min  in-degree above which the row engine (PR and SpMV of small
+//               and some local graphs, gbx_pull.cu) cuts a row into CTA-sized
+//               chunks (rows of 33 up to it get a warp)
 // SSSP distances are the same for every setting, and PR/SpMV sums only change
 // their FP32 summation order (within the 1e-6 relative L1 bound). BFS levels,
 // processed_nodes and iteration are the same for every bfs_alpha / bfs_beta
@@ -170,21 +171,7 @@ extern "C" int gbx_autotune(gbx_graph *g, uint32_t flags, uint32_t num_samples, 
         g->sssp_delta = best_d;
     }
     if (flags & 4u) {
-        // row classes of the row engine, timed on pull PageRank iterations
-        // with the hot-table engine (which has none) held off
-        struct RowsOnly {
-            gbx_graph *g;
-            gbx_pull_layout *layout;
-            uint32_t tries;
-            explicit RowsOnly(gbx_graph *gr) : g(gr), layout(gr->pull_layout), tries(gr->pull_layout_tries) {
-                g->pull_layout = nullptr;
-                g->pull_layout_tries = ~0u;
-            }
-            ~RowsOnly() {
-                g->pull_layout = layout;
-                g->pull_layout_tries = tries;
-            }
-        } rows_only(g);
+        // row classes of the row engine, timed on its PageRank iterations
         const uint32_t cands[] = {1024, 4096, 16384};
         DevBuf<float> ranks;
         GBX_TRY(ranks.alloc(g->V, s));
@@ -192,9 +179,9 @@ extern "C" int gbx_autotune(gbx_graph *g, uint32_t flags, uint32_t num_samples, 
         uint32_t best_h = g->pull_heavy_min;
         for (uint32_t c : cands) {
             GBX_TRY(gbx_graph_set_tuning(g, "pull_heavy_min", c));
-            GBX_TRY(gbx_pagerank_pull(g, 5, 0.0, ranks.p, nullptr, stream));  // builds the plan
+            GBX_TRY(pagerank_pull(g, 5, 0.0, ranks.p, nullptr, s, true));  // builds the plan, captures
             float ms = 0.f;
-            GBX_TRY(time_ms([&]() { return gbx_pagerank_pull(g, 5, 0.0, ranks.p, nullptr, stream); }, s, &ms));
+            GBX_TRY(time_ms([&]() { return pagerank_pull(g, 5, 0.0, ranks.p, nullptr, s, true); }, s, &ms));
             if (trace_enabled()) fprintf(stderr, "| autotune pull_heavy_min %-5u | %9.3f ms |\n", c, ms);
             if (ms < best) {
                 best = ms;

@@ -119,8 +119,8 @@ int gbx_graph_device_arrays(const gbx_graph *g, const uint32_t **offsets, const 
  * exceed unexplored edges / alpha; the reference fixes 15), "bfs_beta" (stay
  * bottom-up while the frontier exceeds V / beta; 18), "sssp_delta" (bucket
  * width, 0 = default), "pull_heavy_min" (in-degree above which PR/SpMV cut a
- * row into CTA-sized chunks; 4096; sweeps of small graphs and a graph's first
- * three only: later ones are cut by edges). SSSP distances never change; PR and SpMV
+ * row into CTA-sized chunks; 4096; without effect on graphs whose sweeps are
+ * cut by edges, see gbx_pagerank_pull). SSSP distances never change; PR and SpMV
  * sums may change their FP32 summation order only. BFS results do not depend
  * on alpha/beta when the graph has an inverse CSR or is symmetric; without an
  * inverse CSR the reference pulls over out-edges, and on an asymmetric graph
@@ -131,7 +131,7 @@ int gbx_graph_get_tuning(const gbx_graph *g, const char *key, double *value);
 /* Time candidate settings on num_samples sources of this graph (CUDA
  * events) and keep the fastest: flags bit 0 BFS direction threshold (graphs
  * with an inverse CSR only), bit 1 SSSP bucket width, bit 2 the pull engine's
- * heavy-row threshold (timed on PageRank iterations). */
+ * heavy-row threshold (timed on PageRank iterations of that engine). */
 int gbx_autotune(gbx_graph *g, uint32_t flags, uint32_t num_samples, void *stream);
 
 /* ---- BFS --------------------------------------------------------------- */
@@ -202,8 +202,13 @@ int gbx_bfs_bottom_up_step(gbx_graph *g, const uint32_t *bitmap_curr, uint32_t *
 /* Pull PageRank with the reference's recurrence (damping 0.85f, ranks start
  * at 1-d, dangling mass dropped, stop when no vertex moves by >= epsilon,
  * final ranks divided by N). epsilon = 0 runs exactly max_iterations. FP32
- * ranks; high-degree pull sums use compensated (Kahan) accumulation;
- * the convergence residual is reduced in FP64. */
+ * ranks; pull sums use compensated accumulation; the convergence residual is
+ * reduced in FP64. On graphs of 65,536 edges or more (below 12,000,000 edges:
+ * with a row of 3,072 in-edges or more) PageRank and SpMV sweeps are cut by
+ * edges; the first such call lays the in-edges out for it (4 bytes an edge and
+ * 24 to 40 a vertex meanwhile, 4 and up to 8 kept with the graph). Which way a
+ * graph is swept, and so the bits of the result, depends on the graph alone,
+ * as long as there is memory for the layout. */
 int gbx_pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon, float *ranks,
                       gbx_pr_result *result, void *stream);
 
