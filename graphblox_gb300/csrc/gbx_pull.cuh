@@ -30,7 +30,7 @@
 //
 // Rows of up to `span` edges lie in one unit; longer rows are cut where a unit
 // begins, each piece leaves a partial sum, and the warp that brings the last
-// one adds them up in order (Kahan per lane) and runs the epilogue. Every
+// one adds them up in order (compensated per lane) and runs the epilogue. Every
 // order of additions is fixed by the layout: results repeat bit for bit. Rows
 // without edges are in no unit.
 //
@@ -88,6 +88,18 @@ inline size_t pull_smem(const gbx_pull_layout &l) {
     return ((size_t)l.hot + 4 + kPullWarps * kPullBuf) * sizeof(float);
 }
 
+// A running sum and the errors of its additions (Knuth 1969, two-sum). Past an
+// infinity the errors are NaN and the plain sum is the value.
+struct PullSum {
+    float s = 0.f, err = 0.f;
+    __device__ __forceinline__ void add(float x) {
+        const float t = __fadd_rn(s, x), y = __fsub_rn(t, s);
+        err = __fadd_rn(err, __fadd_rn(__fsub_rn(s, __fsub_rn(t, y)), __fsub_rn(x, y)));
+        s = t;
+    }
+    __device__ __forceinline__ float value() const { return err == err ? __fadd_rn(s, err) : s; }
+};
+
 // Memory of one sweep in flight: piece sums [2 * units] and tickets [units]
 // (zero between sweeps).
 struct PullPieces {
@@ -144,7 +156,7 @@ struct PullSweep {
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t != count - 1) return;
         __syncwarp();
-        Kahan k;
+        PullSum k;
         for (uint32_t i = lane; i < count; i += 32)
             k.add(__ldcg(pieces.sums + 2 * (size_t)(first + i) + (i ? 0 : 1)));
         const float total = warp_sum(k.value());
@@ -206,7 +218,7 @@ struct PullSweep {
         uint32_t row = me.y;          // row of the first pending sum
         uint32_t pending = 0;         // sums in buf
         bool cut = me.z != ~0u;       // the first row began in an earlier unit
-        Kahan carry;                  // the current row's edges of earlier groups
+        PullSum carry;                // the current row's edges of earlier groups
         uint32_t e = (e0 & ~3u) + lane * 4;
         const uint4 *words = reinterpret_cast<const uint4 *>(l.edges) + e / 4;
         float v1[4];
@@ -270,7 +282,7 @@ struct PullSweep {
                 }
                 __syncwarp();
                 pending += total;
-                carry = Kahan();
+                carry = PullSum();
                 uint32_t start = 0;
                 if (cut) {  // the first of them ends a cut row
                     piece(2 * u, buf[0], me.z, me.w, row);
