@@ -39,8 +39,9 @@ struct SpmvHotTerm {
         float w[4];
     };
     __device__ __forceinline__ void factors(uint32_t e, uint32_t e0, uint32_t e1, Factors &f) const {
-        if (!val) {
-            f.w[0] = f.w[1] = f.w[2] = f.w[3] = dflt;
+        if (!val) {  // (an edge outside the unit counts 0 * 0, also where dflt is not finite)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f.w[k] = e + k >= e0 && e + k < e1 ? dflt : 0.f;
         } else if (wide && e >= e0 && e + 4 <= e1) {
             const float4 w = __ldcs(reinterpret_cast<const float4 *>(val + e));
             f.w[0] = w.x, f.w[1] = w.y, f.w[2] = w.z, f.w[3] = w.w;
