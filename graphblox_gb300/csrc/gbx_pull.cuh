@@ -26,7 +26,8 @@
 // less room, and every miss in flight holds a sector of it: a sweep of RMAT-22
 // takes 236 us without slots, 188 with 16,000, 184 with 20,000, 178 with
 // 28,000, 198 with 40,000 and 316 with 52,000; SpMV over a crawl graph, whose
-// ids are local and hit L1, 416, 433, 430, 459, 629 and 1055 us.
+// ids are local and hit L1, 416, 433, 430, 459, 629 and 1055 us (both with
+// plain additions).
 //
 // Rows of up to `span` edges lie in one unit; longer rows are cut where a unit
 // begins, each piece leaves a partial sum, and the warp that brings the last
@@ -34,8 +35,8 @@
 // order of additions is fixed by the layout: results repeat bit for bit. Rows
 // without edges are in no unit.
 //
-// Against the row engine (RMAT-22, 65M edges): a PageRank iteration 310 -> 178
-// us, SpMV 427 -> 209 us; SpMV over 150M crawl edges 640 -> 425 us.
+// Against the row engine (RMAT-22, 65M edges): a PageRank iteration 332 -> 187
+// us, SpMV 453 -> 229 us; SpMV over 142M crawl edges 641 -> 458 us.
 #pragma once
 
 #include <algorithm>
@@ -88,8 +89,10 @@ inline size_t pull_smem(const gbx_pull_layout &l) {
     return ((size_t)l.hot + 4 + kPullWarps * kPullBuf) * sizeof(float);
 }
 
-// A running sum and the errors of its additions (Knuth 1969, two-sum). Past an
-// infinity the errors are NaN and the plain sum is the value.
+// A running sum and the errors of its additions: of any two numbers (Knuth
+// 1969, two-sum), or in half the instructions where the sum mostly is the
+// larger one (Kahan 1965). Past an infinity the errors are not finite and
+// the plain sum is the value.
 struct PullSum {
     float s = 0.f, err = 0.f;
     __device__ __forceinline__ void add(float x) {
@@ -97,7 +100,12 @@ struct PullSum {
         err = __fadd_rn(err, __fadd_rn(__fsub_rn(s, __fsub_rn(t, y)), __fsub_rn(x, y)));
         s = t;
     }
-    __device__ __forceinline__ float value() const { return err == err ? __fadd_rn(s, err) : s; }
+    __device__ __forceinline__ void add_small(float x) {
+        const float t = __fadd_rn(s, x);
+        err = __fadd_rn(err, __fsub_rn(x, __fsub_rn(t, s)));
+        s = t;
+    }
+    __device__ __forceinline__ float value() const { return fabsf(err) < INFINITY ? __fadd_rn(s, err) : s; }
 };
 
 // Memory of one sweep in flight: piece sums [2 * units] and tickets [units]
@@ -159,7 +167,13 @@ struct PullSweep {
         PullSum k;
         for (uint32_t i = lane; i < count; i += 32)
             k.add(__ldcg(pieces.sums + 2 * (size_t)(first + i) + (i ? 0 : 1)));
-        const float total = warp_sum(k.value());
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float err = __shfl_xor_sync(0xffffffffu, k.err, o);
+            k.add(__shfl_xor_sync(0xffffffffu, k.s, o));
+            k.err = __fadd_rn(k.err, err);
+        }
+        const float total = k.value();
         if (lane == 0) {
             const uint2 r = __ldg(l.rows + row);
             epi(row, r.x, r.y, total);
@@ -245,27 +259,45 @@ struct PullSweep {
             term.scale(f, v);
             // this lane's pieces: the sum up to its first row end, sums of
             // rows inside, the sum after its last row end
-            float acc = 0.f, done[4];
+            PullSum acc, head;
+            float done[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                acc = __fadd_rn(acc, v[k]);
-                done[k] = acc;
-                if ((ends >> k) & 1u) acc = 0.f;
+                if (k == 0) acc.s = v[0]; else acc.add_small(v[k]);
+                done[k] = acc.s;
+                if ((ends >> k) & 1u) {
+                    if ((ends & ((1u << k) - 1u)) == 0) head = acc;
+                    acc = PullSum();
+                }
             }
             // segmented scan of the trailing pieces; a lane with a row end starts a segment
             const unsigned m = __ballot_sync(0xffffffffu, ends != 0);
             const unsigned upto = m & (lt | (1u << lane));
             const uint32_t back = upto ? lane - (31u - __clz(upto)) : lane;
-            float scan = acc;
+            // (inside 8 lanes: longer chains are joined below)
+            float scan = acc.value();
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
+            for (int o = 1; o < 8; o <<= 1) {
                 const float t = __shfl_up_sync(0xffffffffu, scan, o);
-                if ((uint32_t)o <= back) scan = __fadd_rn(scan, t);
+                if ((uint32_t)o <= min(back, lane % 8u)) scan = __fadd_rn(scan, t);
             }
+            // the open row's sum after this lane: earlier groups, whole runs
+            // of 8 lanes, and the lanes of the lane's own run
+            PullSum open;
+            if (upto == 0) open = carry;
+#pragma unroll
+            for (int b = 8; b < 32; b += 8) {
+                const float run = __shfl_sync(0xffffffffu, scan, b - 1);
+                open.add_small(lane >= (uint32_t)b && (upto >> b) == 0 ? run : 0.f);
+            }
+            open.add_small(scan);
             if (m) {
-                float in = __shfl_up_sync(0xffffffffu, scan, 1);
-                if (lane == 0) in = 0.f;
-                if ((m & lt) == 0) in = __fadd_rn(in, carry.value());
+                PullSum in;
+                in.s = __shfl_up_sync(0xffffffffu, open.s, 1);
+                in.err = __shfl_up_sync(0xffffffffu, open.err, 1);
+                if (lane == 0) in = carry;
+                in.add_small(head.s);
+                in.err = __fadd_rn(in.err, head.err);
                 // row sums go to buf in row order
                 uint32_t pos = pending, total = 0;
 #pragma unroll
@@ -277,12 +309,11 @@ struct PullSweep {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if ((ends >> k) & 1u) {
-                        buf[pos++] = (ends & ((1u << k) - 1u)) ? done[k] : __fadd_rn(in, done[k]);
+                        buf[pos++] = (ends & ((1u << k) - 1u)) ? done[k] : in.value();
                     }
                 }
                 __syncwarp();
                 pending += total;
-                carry = PullSum();
                 uint32_t start = 0;
                 if (cut) {  // the first of them ends a cut row
                     piece(2 * u, buf[0], me.z, me.w, row);
@@ -299,7 +330,8 @@ struct PullSweep {
                     __syncwarp();
                 }
             }
-            carry.add(__shfl_sync(0xffffffffu, scan, 31));
+            carry.s = __shfl_sync(0xffffffffu, open.s, 31);
+            carry.err = __shfl_sync(0xffffffffu, open.err, 31);
         }
         emit(row, buf, pending);
         row += pending;
