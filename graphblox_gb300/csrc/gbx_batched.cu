@@ -985,7 +985,9 @@ extern "C" int gbx_pr_batched(gbx_batch *b, uint32_t max_iterations, double epsi
     GBX_CUDA(cudaMemsetAsync(cursor.p, 0, 4, s));
     const uint32_t smem_v = bp_smem_v(b), room = (b->max_v + 31) & ~31u;
     const size_t smem = ((size_t)smem_v + kBpWarps * kBpBuf) * sizeof(float);
-    GBX_CUDA(cudaFuncSetAttribute(pr_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the limit holds for the process: always the most that any batch takes
+    GBX_CUDA(cudaFuncSetAttribute(pr_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)((kBpSmemV + kBpWarps * kBpBuf) * sizeof(float))));
     const unsigned grid = std::min<unsigned>((unsigned)num_sms(), b->G);
     if (2 * (uint64_t)room > smem_v) GBX_TRY(next.alloc((size_t)grid * room, s));
     if (room > smem_v) GBX_TRY(scratch.alloc((size_t)grid * room, s));

@@ -392,7 +392,7 @@ int pr_run_hot(gbx_graph *g, const gbx_pull_layout &l, uint32_t max_it, double e
     GBX_LAUNCH_CHECK();
     PrHotArgs a{l, c->rbuf, c->cbuf, c->row_degree, c->st, {c->sums, c->tickets}, &c->tail->sync, max_it, epsilon};
     const size_t smem = pull_smem(l);
-    GBX_CUDA(cudaFuncSetAttribute(pr_hot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBX_CUDA(cudaFuncSetAttribute(pr_hot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPullSmemLimit));
     // a CTA per SM, fewer where there is less than a unit per warp
     const unsigned ctas = std::min<unsigned>((unsigned)num_sms(), ceil_div(l.n_units, kPullWarps));
     void *args[] = {&a};

@@ -85,9 +85,12 @@ constexpr uint32_t kPullSpanMax = 3072;
 
 // shared memory: the slots, four zeros (the first is the value of no edge),
 // the warps' pending sums
-inline size_t pull_smem(const gbx_pull_layout &l) {
-    return ((size_t)l.hot + 4 + kPullWarps * kPullBuf) * sizeof(float);
-}
+constexpr size_t pull_smem_of(uint32_t hot) { return ((size_t)hot + 4 + kPullWarps * kPullBuf) * sizeof(float); }
+inline size_t pull_smem(const gbx_pull_layout &l) { return pull_smem_of(l.hot); }
+// A kernel's limit on dynamic shared memory holds for the process: it is
+// always set to the most that any layout takes, so that no thread lowers it
+// between another one's setting and launch.
+constexpr int kPullSmemLimit = (int)pull_smem_of(kHotMax);
 
 // A running sum and the errors of its additions: of any two numbers (Knuth
 // 1969, two-sum), or in half the instructions where the sum mostly is the

@@ -97,7 +97,7 @@ static int spmv_run_hot(const gbx_pull_layout &l, SpmvHotTerm term, float *y, ui
         GBX_LAUNCH_CHECK();
     }
     const size_t smem = pull_smem(l);
-    GBX_CUDA(cudaFuncSetAttribute(spmv_hot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBX_CUDA(cudaFuncSetAttribute(spmv_hot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPullSmemLimit));
     const unsigned ctas = std::min<unsigned>((unsigned)num_sms(), ceil_div(l.n_units, kPullWarps));
     for (uint32_t it = 0; it < iterations; ++it) {
         const uint32_t at = it % kPullCursors;
