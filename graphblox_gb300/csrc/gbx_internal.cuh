@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstddef>
 #include <cstdio>
+#include <mutex>
 
 #include "gbx.h"
 
@@ -242,6 +243,7 @@ struct gbx_graph {
     // no memory for it
     struct gbx_pull_layout *pull_layout = nullptr;
     uint32_t pull_layout_tries = 0;
+    std::mutex pull_layout_mutex;
     // betweenness centrality: successor CSR with ascending rows (gbx_bc.cu)
     struct gbx_bc_cache *bc_cache = nullptr;
     // device scratch lent to one synchronous call at a time (gbx::Scratch)

@@ -8,7 +8,6 @@
 // serves far better than a word per vertex, and only sources with a slot in
 // their slot's number.
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "gbx_pull.cuh"
@@ -196,8 +195,6 @@ int build_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout *l) {
     return GBX_OK;
 }
 
-std::mutex g_layout_mutex;
-
 }  // namespace
 
 int get_pull_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout **out) {
@@ -207,7 +204,7 @@ int get_pull_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout **out) {
     if (g->E < kLayoutLocalEdges && longest < kLayoutLongRow) return GBX_OK;
     bool captured = false;
     GBX_TRY(is_capturing(s, &captured));
-    std::lock_guard<std::mutex> lock(g_layout_mutex);
+    std::lock_guard<std::mutex> lock(g->pull_layout_mutex);
     if (!g->pull_layout && !captured && g->pull_layout_tries < 2) {
         gbx_pull_layout *l = new gbx_pull_layout();
         const int st = build_layout(g, s, l);
