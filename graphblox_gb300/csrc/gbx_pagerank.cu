@@ -216,11 +216,6 @@ __global__ void pr_hot_init_kernel(float *r, float *c, const uint32_t *out_degre
     }
 }
 
-__global__ void pr_row_degree_kernel(const uint2 *rows, uint32_t n, const uint32_t *out_degree, uint32_t *row_degree) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        row_degree[i] = out_degree[rows[i].x];
-}
-
 struct PrHotArgs {
     gbx_pull_layout layout;
     float *r, *c;
@@ -286,11 +281,6 @@ struct gbx_pr_cache {
     } *tail = nullptr;
     gbx::PrIterState *st = nullptr;  // behind *tail
     uint32_t cap = 0;                // states
-    // hot-table engine: pieces of cut rows and their tickets (zero between
-    // sweeps), out-degrees in row order
-    float *sums = nullptr;
-    unsigned *tickets = nullptr;
-    uint32_t *row_degree = nullptr;
     cudaStream_t cap_stream = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint32_t key_it = 0, kernels = 0;
@@ -309,9 +299,6 @@ void gbx_free_pr_cache(gbx_pr_cache *c) {
     cudaFree(c->rbuf);
     cudaFree(c->cbuf);
     cudaFree(c->tail);
-    cudaFree(c->sums);
-    cudaFree(c->tickets);
-    cudaFree(c->row_degree);
     delete c;
 }
 
@@ -319,7 +306,7 @@ using namespace gbx;
 
 namespace {
 
-int pr_cache(gbx_graph *g, const gbx_pull_layout *l, uint32_t max_it, cudaStream_t s, gbx_pr_cache **out) {
+int pr_cache(gbx_graph *g, const gbx_pull_layout *l, uint32_t max_it, gbx_pr_cache **out) {
     gbx_pr_cache *c = g->pr_cache;
     if (!c) c = g->pr_cache = new gbx_pr_cache();
     const size_t need = 2 * contrib_stride(g->V, l ? l->hot : 0);
@@ -342,19 +329,7 @@ int pr_cache(gbx_graph *g, const gbx_pull_layout *l, uint32_t max_it, cudaStream
         c->st = reinterpret_cast<PrIterState *>(c->tail + 1);
         c->cap = cap;
     }
-    if (!l) {
-        if (!c->cap_stream) GBX_CUDA(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
-    } else if (!c->row_degree) {
-        if (!c->sums) GBX_CUDA(cudaMalloc(&c->sums, sizeof(float) * 2 * (size_t)l->n_units));
-        if (!c->tickets) {
-            GBX_CUDA(cudaMalloc(&c->tickets, sizeof(unsigned) * (size_t)l->n_units));
-            GBX_CUDA(cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * (size_t)l->n_units, s));
-        }
-        GBX_CUDA(cudaMalloc(&c->row_degree, sizeof(uint32_t) * (size_t)l->n_rows));
-        pr_row_degree_kernel<<<std::min<unsigned>(ceil_div(l->n_rows, 256), (unsigned)num_sms() * 8), 256, 0, s>>>(
-            l->rows, l->n_rows, g->out_degree, c->row_degree);
-        GBX_LAUNCH_CHECK();
-    }
+    if (!l && !c->cap_stream) GBX_CUDA(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
     *out = c;
     return GBX_OK;
 }
@@ -390,7 +365,7 @@ int pr_run_hot(gbx_graph *g, const gbx_pull_layout &l, uint32_t max_it, double e
     const int grid = (int)std::min<uint64_t>((V + l.hot + 255ull) / 256, (uint64_t)num_sms() * 8);
     pr_hot_init_kernel<<<grid, 256, 0, s>>>(c->rbuf, c->cbuf, g->out_degree, V, l.hot, l.hot_ids);
     GBX_LAUNCH_CHECK();
-    PrHotArgs a{l, c->rbuf, c->cbuf, c->row_degree, c->st, {c->sums, c->tickets}, &c->tail->sync, max_it, epsilon};
+    PrHotArgs a{l, c->rbuf, c->cbuf, l.row_degree, c->st, {l.sums, l.tickets}, &c->tail->sync, max_it, epsilon};
     const size_t smem = pull_smem(l);
     GBX_CUDA(cudaFuncSetAttribute(pr_hot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPullSmemLimit));
     // a CTA per SM, fewer where there is less than a unit per warp
@@ -413,7 +388,7 @@ int gbx::pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon, fl
     OutArray<float> out;
     GBX_TRY(out.bind(ranks, V, s));
     gbx_pr_cache *c = nullptr;
-    GBX_TRY(pr_cache(g, layout, max_iterations, s, &c));
+    GBX_TRY(pr_cache(g, layout, max_iterations, &c));
     if (layout) {
         GBX_TRY(pr_run_hot(g, *layout, max_iterations, epsilon, c, s));
     } else {
@@ -430,7 +405,7 @@ int gbx::pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon, fl
     GBX_CUDA(cudaMemcpyAsync(&h, c->tail, sizeof(h), cudaMemcpyDeviceToHost, s));
     GBX_CUDA(cudaStreamSynchronize(s));
     if (layout && h.sync.error) {
-        GBX_CUDA(cudaMemset(c->tickets, 0, sizeof(unsigned) * (size_t)layout->n_units));  // a sweep was left half done
+        GBX_CUDA(cudaMemset(layout->tickets, 0, sizeof(unsigned) * (size_t)layout->n_units));  // a sweep was left half done
         GBX_REQUIRE(false, GBX_ERR_DEVICE_TIMEOUT, "PageRank: a grid barrier wait ran out");
     }
     if (result) *result = h.res;

@@ -55,11 +55,15 @@ __global__ void pull_flags_kernel(const uint32_t *off, const uint32_t *deg, uint
 
 // rows and slots
 __global__ void pull_rows_kernel(const uint32_t *has_edges, const uint32_t *row_pos, const uint32_t *is_hot,
-                                 const uint32_t *slot_pos, uint32_t V, uint2 *rows, uint32_t *hot_ids) {
+                                 const uint32_t *slot_pos, const uint32_t *deg, uint32_t V, uint2 *rows,
+                                 uint32_t *row_degree, uint32_t *hot_ids) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
         const bool hot = is_hot[v];
         const uint32_t slot = hot ? slot_pos[v] : ~0u;
-        if (has_edges[v]) rows[row_pos[v]] = make_uint2(v, slot);
+        if (has_edges[v]) {
+            rows[row_pos[v]] = make_uint2(v, slot);
+            row_degree[row_pos[v]] = deg[v];
+        }
         if (hot) hot_ids[slot] = v;
     }
 }
@@ -180,9 +184,14 @@ int build_layout(gbx_graph *g, cudaStream_t s, gbx_pull_layout *l) {
     GBX_TRY(dev_alloc((void **)&l->rows, (size_t)std::max(l->n_rows, 1u) * sizeof(uint2), s));
     GBX_TRY(dev_alloc((void **)&l->units, ((size_t)l->n_units + 1) * sizeof(uint4), s));
     GBX_TRY(dev_alloc((void **)&l->work, pull_work_words(*l) * 4, s));
+    GBX_TRY(dev_alloc((void **)&l->row_degree, (size_t)std::max(l->n_rows, 1u) * 4, s));
+    GBX_TRY(dev_alloc((void **)&l->sums, (size_t)l->n_units * 8, s));
+    GBX_TRY(dev_alloc((void **)&l->tickets, (size_t)l->n_units * 4, s));
+    GBX_CUDA(cudaMemsetAsync(l->tickets, 0, (size_t)l->n_units * 4, s));
     GBX_CUDA(cudaMemsetAsync(l->edges + E, 0, kPullPad * 4, s));
     if (l->hot) GBX_CUDA(cudaMemsetAsync(l->hot_ids, 0xFF, (size_t)l->hot * 4, s));
-    pull_rows_kernel<<<grid, 256, 0, s>>>(has.p, row_pos.p, hot.p, slot_pos.p, V, l->rows, l->hot_ids);
+    pull_rows_kernel<<<grid, 256, 0, s>>>(has.p, row_pos.p, hot.p, slot_pos.p, g->out_degree, V, l->rows,
+                                        l->row_degree, l->hot_ids);
     GBX_LAUNCH_CHECK();
     const int egrid = (int)std::min<uint64_t>((E + 2047ull) / 2048, (uint64_t)num_sms() * 8);
     pull_words_kernel<<<egrid, 256, 0, s>>>(g->pull_src(), E, hot_bits.p, slot_pos.p, l->edges);
@@ -233,5 +242,8 @@ void gbx_free_pull_layout(gbx_pull_layout *l) {
     gbx::dev_free(l->rows);
     gbx::dev_free(l->units);
     gbx::dev_free(l->work);
+    gbx::dev_free(l->row_degree);
+    gbx::dev_free(l->sums);
+    gbx::dev_free(l->tickets);
     delete l;
 }

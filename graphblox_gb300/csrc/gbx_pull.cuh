@@ -63,6 +63,12 @@ struct gbx_pull_layout {
     // device [pull_work_words]: working memory of captured SpMV calls (the
     // graph that a capture makes outlives any allocation of the call)
     float *work = nullptr;
+    // PageRank's, allocated here so that a graph that has a layout lacks
+    // nothing: device [n_rows] out-degrees in row order, piece sums
+    // [2 * n_units] and tickets [n_units], zero between sweeps
+    uint32_t *row_degree = nullptr;
+    float *sums = nullptr;
+    unsigned *tickets = nullptr;
 };
 
 __host__ __device__ inline uint32_t pull_unit_edge(const gbx_pull_layout &l, uint32_t t) {

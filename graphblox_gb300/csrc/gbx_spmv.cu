@@ -82,13 +82,19 @@ __global__ void __launch_bounds__(kPullThreads, 1)
 }
 
 // Working memory is the call's own, so that sweeps of one graph on several
-// streams do not meet; a captured call's is the layout's.
-static int spmv_run_hot(const gbx_pull_layout &l, SpmvHotTerm term, float *y, uint32_t iterations, cudaStream_t s) {
+// streams do not meet; a captured call's is the layout's. So is, where there
+// is none to be had, that of a call that holds the graph's lock to its end.
+static int spmv_run_hot(gbx_graph *g, const gbx_pull_layout &l, SpmvHotTerm term, float *y, uint32_t iterations,
+                        cudaStream_t s) {
     bool captured = false;
     GBX_TRY(is_capturing(s, &captured));
     DevBuf<float> own;
-    if (!captured) GBX_TRY(own.alloc(pull_work_words(l), s));
-    float *const hot_x = captured ? l.work : own.p, *const sums = hot_x + std::max(l.hot, 4u);
+    std::unique_lock<std::mutex> lent(g->pull_layout_mutex, std::defer_lock);
+    if (!captured && own.alloc(pull_work_words(l), s) != GBX_OK) {
+        clear_error();
+        lent.lock();
+    }
+    float *const hot_x = own.p ? own.p : l.work, *const sums = hot_x + std::max(l.hot, 4u);
     unsigned *const tickets = reinterpret_cast<unsigned *>(sums + 2 * (size_t)l.n_units);
     unsigned *const cursors = tickets + l.n_units;
     GBX_CUDA(cudaMemsetAsync(tickets, 0, ((size_t)l.n_units + kPullCursors) * sizeof(unsigned), s));
@@ -106,6 +112,7 @@ static int spmv_run_hot(const gbx_pull_layout &l, SpmvHotTerm term, float *y, ui
                                                          cursors + at);
         GBX_LAUNCH_CHECK();
     }
+    if (lent.owns_lock()) GBX_CUDA(cudaStreamSynchronize(s));
     return GBX_OK;
 }
 
@@ -139,7 +146,7 @@ extern "C" int gbx_spmv(gbx_graph *g, const float *values, float default_value, 
     if (yout.to_host()) GBX_CUDA(cudaMemcpyAsync(yout.d, y, (size_t)V * 4, cudaMemcpyHostToDevice, s));
     if (layout) {
         const bool wide = ((uintptr_t)vals & 15u) == 0;
-        GBX_TRY(spmv_run_hot(*layout, SpmvHotTerm{vals, default_value, xin.d, wide}, yout.d, iterations, s));
+        GBX_TRY(spmv_run_hot(g, *layout, SpmvHotTerm{vals, default_value, xin.d, wide}, yout.d, iterations, s));
     } else {
         SpmvTerm term{g->pull_src(), vals, default_value, xin.d};
         SpmvEpi epi{yout.d};

@@ -205,8 +205,8 @@ int gbx_bfs_bottom_up_step(gbx_graph *g, const uint32_t *bitmap_curr, uint32_t *
  * ranks; pull sums use compensated accumulation; the convergence residual is
  * reduced in FP64. On graphs of 65,536 edges or more (below 12,000,000 edges:
  * with a row of 3,072 in-edges or more) PageRank and SpMV sweeps are cut by
- * edges; the first such call lays the in-edges out for it (4 bytes an edge and
- * 24 to 40 a vertex meanwhile, 4 and up to 8 kept with the graph). Which way a
+ * edges; the first such call lays the in-edges out for it (kept with the
+ * graph: 4 bytes an edge and up to 12 a vertex; 16 a vertex meanwhile). Which way a
  * graph is swept, and so the bits of the result, depends on the graph alone,
  * as long as there is memory for the layout. */
 int gbx_pagerank_pull(gbx_graph *g, uint32_t max_iterations, double epsilon, float *ranks,
