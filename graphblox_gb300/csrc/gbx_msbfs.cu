@@ -582,7 +582,7 @@ int ms_plan(gbx_graph *g, cudaStream_t s, gbx_ms_plan **out) {
 // 100 sources, one at a time / 2 / 4 / 8: R-MAT of 1,000 vertices 481 / 405 /
 // 376 / 358, 250,000 613 / 543 / 515 / 495; local graph of 30,000 842 / 706 /
 // 684 / 728; RMAT-20 with 256 sources 1,622 / 1,543 / 1,519 / 1,494. Masks above
-// kAheadBytes are not allocated ahead.
+// kAheadBytes, or that there is no memory for, are not allocated ahead.
 constexpr uint32_t kAhead = 8, kAheadLater = 4;
 constexpr size_t kAheadBytes = size_t(64) << 20;
 
@@ -611,6 +611,7 @@ int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, 
     GBX_TRY(q0.alloc(std::max(V, S), s));
     GBX_TRY(q1.alloc(std::max(V, S), s));
     GBX_TRY(cnt.alloc(ahead + 1, s));
+    GBX_TRY(per_source.alloc(2 * (size_t)S, s));
     GBX_CUDA(cudaMemsetAsync(seen.p, 0, words * 4, s));
     GBX_CUDA(cudaMemsetAsync(lvbuf[0].p, 0, words * 4, s));
     GBX_CUDA(cudaMemsetAsync(cnt.p, 0, (ahead + 1) * sizeof(MsCounters), s));
@@ -618,11 +619,7 @@ int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, 
     GBX_LAUNCH_CHECK();
     MsCounters h[kAhead + 1] = {};
     h[0].qn = S;
-    bool known = ahead == 1;  // the host has read the batch's first frontier
-    if (known) {
-        GBX_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h[0]), cudaMemcpyDeviceToHost, s));
-        GBX_CUDA(cudaStreamSynchronize(s));
-    }
+    bool known = false;  // the host has read the batch's first frontier
     // the mask of a level: kept while it fits, else one of two in turn
     auto mask_of = [&](uint32_t l, uint32_t **out) -> int {
         DevBuf<uint32_t> &d = l < max_stored ? lvbuf[l] : deep[l & 1];
@@ -630,7 +627,28 @@ int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, 
         *out = d.p;
         return GBX_OK;
     };
+    // The masks of a batch's levels before its first step. Where there is no
+    // memory for them, steps go one at a time from here on and allocate what
+    // each needs.
+    auto reserve = [&](uint32_t level) -> int {
+        uint32_t *mask = nullptr;
+        int st = GBX_OK;
+        for (uint32_t l = level + 1; ahead > 1 && st == GBX_OK && l <= level + 1 + ahead; ++l) st = mask_of(l, &mask);
+        if (st == GBX_ERR_NOMEM) {
+            clear_error();
+            for (uint32_t l = level + 2; l < max_stored; ++l) lvbuf[l].release();
+            ahead = 1;
+            st = GBX_OK;
+        }
+        if (st == GBX_OK && ahead == 1 && !known) {
+            GBX_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof(h[0]), cudaMemcpyDeviceToHost, s));
+            GBX_CUDA(cudaStreamSynchronize(s));
+            known = true;
+        }
+        return st;
+    };
     uint32_t *F = lvbuf[0].p, *Fn = nullptr, *q = q0.p, *qn = q1.p;
+    GBX_TRY(reserve(0));
     if (ahead > 1) {
         GBX_TRY(mask_of(1, &Fn));
         GBX_CUDA(cudaMemsetAsync(Fn, 0, words * 4, s));
@@ -693,6 +711,7 @@ int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, 
         }
         known = true;
         ahead = std::min(ahead, kAheadLater);
+        if (h[0].qn > 0) GBX_TRY(reserve(level));
     }
     GBX_REQUIRE(h[0].qn == 0, GBX_ERR_ITER_CAP, "multi-source BFS level cap reached");
     // distances of the stored levels, zeros for unreached pairs, and the
@@ -700,7 +719,6 @@ int msbfs_impl(gbx_graph *g, uint32_t S, const uint32_t *src_d, uint32_t *dist, 
     MsLevels lv{};
     lv.n = stored;
     for (uint32_t L = 0; L < stored; ++L) lv.m[L] = lvbuf[L].p;
-    GBX_TRY(per_source.alloc(2 * (size_t)S, s));
     GBX_CUDA(cudaMemsetAsync(per_source.p, 0, 16 * (size_t)S, s));
     unsigned long long *const re = per_source.p;
     uint32_t *const rc = reinterpret_cast<uint32_t *>(re + S), *const rd = rc + S;
