@@ -747,17 +747,21 @@ __global__ void __launch_bounds__(kSsspSmallThreads, 1)
 
 int sssp_small(gbx_graph *g, uint32_t source, uint32_t *distances, gbx_sssp_result *result, cudaStream_t s) {
     const uint32_t V = g->V;
+    const int out_dev = is_device_ptr(distances) ? 1 : 0;
+    Scratch sc;
+    GBX_TRY(sc.take(g, (out_dev ? 0 : Scratch::round_up((size_t)V * 4)) + Scratch::round_up(sizeof(SsspSmallResult)), s));
+    uint32_t *const stage = out_dev ? nullptr : sc.carve<uint32_t>(V);
+    SsspSmallResult *const res = sc.carve<SsspSmallResult>(1);
+    GBX_REQUIRE(res != nullptr, GBX_ERR_CUDA, "SSSP scratch carve overflow");
     OutArray<uint32_t> out;
-    GBX_TRY(out.bind(distances, V, s));
-    DevBuf<SsspSmallResult> res;
-    GBX_TRY(res.alloc(1, s));
+    GBX_TRY(out.bind(distances, V, s, stage, out_dev));
     GBX_CUDA(cudaFuncSetAttribute(sssp_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSsspSmallV * 4)));
     sssp_small_kernel<<<1, kSsspSmallThreads, (size_t)V * 4, s>>>(g->offsets, g->dest, g->weight, V, source,
-                                                                 4 * V + 64, out.d, res.p);
+                                                                 4 * V + 64, out.d, res);
     GBX_LAUNCH_CHECK();
     GBX_TRY(out.finish(s));
     SsspSmallResult h;
-    GBX_CUDA(cudaMemcpyAsync(&h, res.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+    GBX_CUDA(cudaMemcpyAsync(&h, res, sizeof(h), cudaMemcpyDeviceToHost, s));
     GBX_CUDA(cudaStreamSynchronize(s));
     GBX_REQUIRE(h.status == 0, GBX_ERR_ITER_CAP, "SSSP round cap reached");
     if (result) {
