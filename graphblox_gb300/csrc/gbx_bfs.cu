@@ -346,8 +346,8 @@ __device__ void top_down_phase(const BfsArgs &a, Team team, const uint32_t *qin,
             __syncwarp();
         }
     }
+    clock.stop(cur);  // before the flush, which waits for the CTA's other warps
     claim.flush();
-    clock.stop(cur);
 }
 
 // Probe in-edges [j, el) of one vertex, N at a time: the ids, then their
@@ -501,8 +501,8 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
         }
         __syncwarp();
     }
-    step_flush(wq, qout, cnt, nf, 0, edges);
     clock.stop(cnt);
+    step_flush(wq, qout, cnt, nf, 0, edges);
 }
 
 // arrayQueueToBitmap (arrayQueue.c:284-308) from the lists themselves, into a
