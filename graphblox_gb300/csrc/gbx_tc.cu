@@ -155,7 +155,9 @@ __device__ __forceinline__ unsigned long long pair_hash(uint32_t a, uint32_t b) 
     return z ^ (z >> 31);
 }
 
-// flags: bit 0 = some row repeats a neighbour. *asym accumulates, over all
+// flags: bit 0 = some row repeats a neighbour or is not in ascending order (the
+// fast path's bitmaps and tables are sized by N+(v) being a row's first ids,
+// and ids above v would lie past them). *asym accumulates, over all
 // edges v->u, hash(v,u) - hash(u,v) (mod 2^64): zero when the edge multiset
 // equals its reverse (the CSR is symmetric); a non-symmetric CSR sums to zero
 // only by a 64-bit hash coincidence. One streaming pass instead of a search
@@ -201,7 +203,7 @@ __global__ void tc_shape_check_kernel(const uint32_t *off, const uint32_t *dest,
                     begin = end;
                     end = __ldg(off + r + 1);
                 }
-                if (j > begin && u[q] == before[q]) f |= 1u;
+                if (j > begin && u[q] <= before[q]) f |= 1u;
                 h += pair_hash(r, u[q]) - pair_hash(u[q], r);
             }
         }
