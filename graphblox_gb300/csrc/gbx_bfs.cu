@@ -235,12 +235,13 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t r) {
     return pos;
 }
 
+template <bool kTraced>
 __device__ void top_down_phase(const BfsArgs &a, Team team, const uint32_t *qin, uint32_t qn, const uint32_t *hvin,
                                const uint32_t *hcin, uint32_t nh, uint32_t nc, BfsStep *cur, uint32_t *qout,
                                uint32_t *hvout, uint32_t *hcout, uint32_t lnext, uint32_t *fbm, uint32_t *clear_bm,
                                uint32_t *s_pre, uint32_t *s_base, uint32_t *s_v, uint32_t *s_wq) {
     const uint32_t lane = threadIdx.x & 31;
-    BusyClock clock(a.trace != 0);
+    BusyClock clock(kTraced && a.trace != 0);
     if (clear_bm) {
         // the bitmap the next top-down step fills (not read during this one)
         for (uint32_t w = team.thread(); w < a.words; w += team.threads())
@@ -380,11 +381,12 @@ __device__ __forceinline__ uint32_t bu_probe(const BfsArgs &a, const uint32_t *c
 // next-frontier word of every word of the unit (zero when nothing was
 // found). Found vertices are also appended to the next generation's queue /
 // hub list, so leaving bottom-up needs no bitmap-to-list pass.
+template <bool kTraced>
 __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur_bm, uint32_t *next_bm, uint32_t lnext,
                                 BfsStep *cnt, uint32_t *qout, uint32_t *hvout, uint32_t *hcout, uint32_t *s_wq,
                                 uint32_t *s_found) {
     const uint32_t lane = threadIdx.x & 31;
-    BusyClock clock(a.trace != 0);
+    BusyClock clock(kTraced && a.trace != 0);
     unsigned nf = 0;
     unsigned long long edges = 0;
     WarpQueue wq(s_wq, kBfsQueueCap);
@@ -601,7 +603,10 @@ __global__ void bfs_init_kernel(uint32_t *level, int32_t *parent, uint32_t *visi
     bfs_init(level, parent, visited, bm0, bm1, V, words, source, outdeg, q0, hv0, hc0, st, whole_grid());
 }
 
-// One traversal by a team, whose barrier is gs.
+// One traversal by a team, whose barrier is gs. kTraced: the warps' busy times
+// may be asked for (teams of several traversals have none, and no registers
+// for the clock).
+template <bool kTraced>
 __device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSync *gs) {
     __shared__ uint32_t s_pre[kBfsWarps][33];
     __shared__ uint32_t s_base[kBfsWarps][32];
@@ -665,7 +670,7 @@ __device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSy
                 nf_prev = qsize;
                 in_bu = true;
             }
-            bottom_up_phase(a, team, a.bm[ib], a.bm[ob], L + 1, cur, a.q[ob], a.hv[ob], a.hc[ob], s_wq[wid],
+            bottom_up_phase<kTraced>(a, team, a.bm[ib], a.bm[ob], L + 1, cur, a.q[ob], a.hv[ob], a.hc[ob], s_wq[wid],
                             s_found[wid]);
             bm_clean[ob] = false;
             if (!grid_barrier(gs, team.ctas)) { failed = true; break; }
@@ -698,7 +703,7 @@ __device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSy
             mu -= mf;
             // bm[ob] is clear here while tracking: bfs_init_kernel cleared both
             // bitmaps, and each tracking step clears bm[ib] for the next one
-            top_down_phase(a, team, a.q[ib], qn, a.hv[ib], a.hc[ib], nh, nc, cur, a.q[ob], a.hv[ob], a.hc[ob], L + 1,
+            top_down_phase<kTraced>(a, team, a.q[ib], qn, a.hv[ib], a.hc[ib], nh, nc, cur, a.q[ob], a.hv[ob], a.hc[ob], L + 1,
                            bm_track ? a.bm[ob] : nullptr, bm_track && s > 0 ? a.bm[ib] : nullptr, s_pre[wid],
                            s_base[wid], s_v[wid], s_wq[wid]);
             if (bm_track) {
@@ -748,7 +753,7 @@ __device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSy
 
 __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs a) {
     grid_barrier_init();
-    bfs_traverse(a, whole_grid(), &a.st->gs);
+    bfs_traverse<true>(a, whole_grid(), &a.st->gs);
 }
 
 // ---- several traversals at once ----------------------------------------------
@@ -812,7 +817,7 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_teams_kernel(BfsTeams t) {
         bfs_init(a.level, a.parent, a.visited, a.bm[0], a.bm[1], a.V, a.words, a.source, a.outdeg, a.q[0], a.hv[0],
                  a.hc[0], a.st, team);
         if (!grid_barrier(&ctl->gs, team.ctas)) return;
-        bfs_traverse(a, team, &ctl->gs);
+        bfs_traverse<false>(a, team, &ctl->gs);
         // nobody writes the next trial's state before all have left this one's
         if (team.leader()) ctl->next = count + atomicAdd(t.queue, 1u);
         if (!grid_barrier(&ctl->gs, team.ctas)) return;
