@@ -241,7 +241,7 @@ __device__ void top_down_phase(const BfsArgs &a, Team team, const uint32_t *qin,
                                uint32_t *hvout, uint32_t *hcout, uint32_t lnext, uint32_t *fbm, uint32_t *clear_bm,
                                uint32_t *s_pre, uint32_t *s_base, uint32_t *s_v, uint32_t *s_wq) {
     const uint32_t lane = threadIdx.x & 31;
-    BusyClock clock(kTraced && a.trace != 0);
+    BusyClock clock(a.trace != 0);
     if (clear_bm) {
         // the bitmap the next top-down step fills (not read during this one)
         for (uint32_t w = team.thread(); w < a.words; w += team.threads())
@@ -347,8 +347,9 @@ __device__ void top_down_phase(const BfsArgs &a, Team team, const uint32_t *qin,
             __syncwarp();
         }
     }
-    clock.stop(cur);  // before the flush, which waits for the CTA's other warps
+    if (kTraced) clock.stop(cur);  // before the flush, which waits for the CTA's other warps
     claim.flush();
+    if (!kTraced) clock.stop(cur);
 }
 
 // Probe in-edges [j, el) of one vertex, N at a time: the ids, then their
@@ -386,7 +387,7 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
                                 BfsStep *cnt, uint32_t *qout, uint32_t *hvout, uint32_t *hcout, uint32_t *s_wq,
                                 uint32_t *s_found) {
     const uint32_t lane = threadIdx.x & 31;
-    BusyClock clock(kTraced && a.trace != 0);
+    BusyClock clock(a.trace != 0);
     unsigned nf = 0;
     unsigned long long edges = 0;
     WarpQueue wq(s_wq, kBfsQueueCap);
@@ -503,8 +504,9 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
         }
         __syncwarp();
     }
-    clock.stop(cnt);
+    if (kTraced) clock.stop(cnt);
     step_flush(wq, qout, cnt, nf, 0, edges);
+    if (!kTraced) clock.stop(cnt);
 }
 
 // arrayQueueToBitmap (arrayQueue.c:284-308) from the lists themselves, into a
@@ -603,9 +605,10 @@ __global__ void bfs_init_kernel(uint32_t *level, int32_t *parent, uint32_t *visi
     bfs_init(level, parent, visited, bm0, bm1, V, words, source, outdeg, q0, hv0, hc0, st, whole_grid());
 }
 
-// One traversal by a team, whose barrier is gs. kTraced: the warps' busy times
-// may be asked for (teams of several traversals have none, and no registers
-// for the clock).
+// One traversal by a team, whose barrier is gs. kTraced: the trace may be asked
+// for. Teams of several traversals have none; their phases read the clock, if
+// they did, after the flush, where it costs them no registers (before it, or
+// without a clock, 64 trials on RMAT-22 take 6.40 to 6.43 ms instead of 6.32).
 template <bool kTraced>
 __device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSync *gs) {
     __shared__ uint32_t s_pre[kBfsWarps][33];
@@ -761,11 +764,12 @@ __global__ void __launch_bounds__(kBfsThreads, 1) bfs_persistent_kernel(BfsArgs 
 // traversal DRAM runs at 14% and the issue slots at 22%, and what a step waits
 // for -- its barrier, the counters, dependent loads, its slowest unit -- does
 // not get shorter with more SMs. So trials that leave their outputs on the
-// device are taken by teams of CTAs: one cooperative grid, a traversal per team with its own
-// working arrays and its own barrier, the next trial from a counter when one
-// is done. A team also writes its trial's initial state, which is a kernel of
-// its own otherwise. 8 trials: RMAT-22 (64M edges) 1,430 us one after the
-// other, 695 by eight teams; 250,000 vertices and 3M edges 543, 137.
+// device are taken by teams of CTAs: one cooperative grid, a traversal per team
+// with its own working arrays and its own barrier, the next trial from a counter
+// when one is done. A team also writes its trial's initial state, which is a
+// kernel of its own otherwise. 8 trials: RMAT-22 (64M edges) 1,242 us one after
+// the other, 710 by eight teams; 250,000 vertices and 3M edges 521, 141 (the
+// same inputs again and again; new inputs each time 810 to 840).
 struct BfsTeams {
     BfsArgs first;            // team 0's working arrays; level / parent: its own, for trials without outputs
     size_t pitch;             // bytes from one team's working arrays to the next's
@@ -1175,14 +1179,14 @@ bool bfs_is_small(const gbx_graph *g, uint32_t n) {
 // their frontiers and outputs push one another out of the L2 or a step is too
 // much work for a team's few SMs: each factor of four in edges halves the
 // count. us for 8 (first four) or 64 R-MAT trials with 1 / 4 / 8 / 16 / 32 / 64 teams:
-//   edges 144M   2609 / 2240 / 2504
-//          96M   2049 / 1400 / 1553
-//          64M   1430 /  864 /  775
-//          12M    806 /  311 /  271
-//      64: 48M      - / 6053 / 5513 / 5804 / 7048 / 7852
-//          12M      - / 2031 / 1570 / 1471 / 1699 / 1870
-//           3M      - / 1233 /  788 /  595 /  537 /  538
-//         770K      - / 1014 /  575 /  374 /  284 /  246
+//   edges 144M   2154 / 2039 / 2282
+//          96M   1843 / 1302 / 1378
+//          64M   1242 /  891 /  710
+//          12M    648 /  311 /  278
+//      64: 48M      - / 5779 / 5061 / 5080 / 6184 / 6917
+//          12M      - / 2017 / 1533 / 1354 / 1536 / 1656
+//           3M      - / 1242 /  800 /  585 /  535 /  508
+//         770K      - /  973 /  594 /  373 /  287 /  243
 // The teams' working arrays are held to kTeamsBytes.
 constexpr uint32_t kMaxTeams = 64, kMinTeams = 4;
 constexpr uint64_t kMaxTeamsEdges = 1'250'000;
