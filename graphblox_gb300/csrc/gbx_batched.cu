@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kBbThreads, 2) bfs_batched_kernel(BbArgs a) {
 // ids in 32 bits: 20.9 ms.
 struct BpArgs {
     uint32_t G;
-    const uint32_t *vbase, *off, *poff, *order;
+    const uint32_t *vbase, *off, *order;
     const uint4 *words;
     const uint32_t *wbase;
     const uint2 *starts, *rows;
@@ -625,8 +625,9 @@ __global__ void bp_bounds_kernel(const uint32_t *vbase, uint32_t G, const uint32
 
 // One CTA lays a graph's words out.
 __global__ void __launch_bounds__(kBpThreads)
-    bp_layout_kernel(uint32_t G, const uint32_t *order, const uint32_t *vbase, const uint32_t *off, const uint32_t *poff, const uint32_t *psrc,
-                     const uint32_t *wbase, uint32_t smem_v, uint4 *words, uint2 *rows, uint2 *starts) {
+    bp_layout_kernel(uint32_t G, const uint32_t *order, const uint32_t *vbase, const uint32_t *off,
+                     const uint32_t *poff, const uint32_t *psrc, const uint32_t *wbase, uint32_t smem_v, uint4 *words,
+                     uint2 *rows, uint2 *starts) {
     __shared__ uint32_t s_wsum[kBpWarps], s_base;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t i = blockIdx.x; i < G; i += gridDim.x) {
@@ -853,7 +854,7 @@ int bp_layout(gbx_batch *b, cudaStream_t s) {
         dev_free(b->words);
         dev_free(b->wbase);
         dev_free(b->rows);
-            dev_free(b->starts);
+        dev_free(b->starts);
         b->words = nullptr;
         b->wbase = nullptr;
         b->rows = b->starts = nullptr;
@@ -995,7 +996,6 @@ extern "C" int gbx_pr_batched(gbx_batch *b, uint32_t max_iterations, double epsi
     a.G = b->G;
     a.vbase = b->vbase;
     a.off = b->offsets;
-    a.poff = b->poff();
     a.order = b->order;
     a.words = b->words;
     a.wbase = b->wbase;

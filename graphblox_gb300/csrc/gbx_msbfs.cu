@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kMsThreads)
     // next-frontier appends are staged per warp in shared memory; what the
     // warps hold at the end and the out-degree sum go out once per CTA, since
     // atomics on one address take about a nanosecond each, one after the other
-    // (RMAT-20, 256 sources, 8 levels: 1,660 -> 1,570 us)
+    // (RMAT-20, 256 sources, 8 levels, one step at a time: 1,660 -> 1,570 us)
     __shared__ uint32_t s_q[kMsThreads / 32][kWarpQueueCap];
     __shared__ uint32_t s_alive[NW];
     __shared__ unsigned long long s_mf;
@@ -581,7 +581,8 @@ int ms_plan(gbx_graph *g, cudaStream_t s, gbx_ms_plan **out) {
 // first, then fewer, since those past a sweep's end are empty launches. us for
 // 100 sources, one at a time / 2 / 4 / 8: R-MAT of 1,000 vertices 481 / 405 /
 // 376 / 358, 250,000 613 / 543 / 515 / 495; local graph of 30,000 842 / 706 /
-// 684 / 728; RMAT-20 with 256 sources 1,622 / 1,543 / 1,519 / 1,494. Masks above
+// 684 / 728; RMAT-20 with 256 sources 1,622 / 1,543 / 1,519 / 1,494 (the same
+// inputs again and again; new inputs each time 1,605 with 8). Masks above
 // kAheadBytes, or that there is no memory for, are not allocated ahead.
 constexpr uint32_t kAhead = 8, kAheadLater = 4;
 constexpr size_t kAheadBytes = size_t(64) << 20;

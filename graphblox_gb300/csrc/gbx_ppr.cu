@@ -351,7 +351,6 @@ __global__ void __launch_bounds__(kPprThreads)
     check_sweep(check, res_out, 32 * KPL, ctl);
 }
 
-
 // Per-column L1 norms of a [V][K] block (FP32 partials per thread, FP64 sums).
 __global__ void ppr_col_norm_kernel(const float *__restrict__ B, uint32_t V, uint32_t K, double *norms) {
     // thread t of the grid owns column t % K and rows t / K, t / K + stride, ...

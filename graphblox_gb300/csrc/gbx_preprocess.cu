@@ -22,37 +22,25 @@ __global__ void max_u32_of_kernel(const uint32_t *a, uint32_t n, uint32_t *out) 
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
-// out[0] = largest id, out[1] = largest id without the mask bits
-__global__ void id_range_kernel(const uint32_t *s, const uint32_t *d, uint32_t n, uint32_t *out) {
-    uint32_t m = 0, mm = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t a = s[i], b = d[i];
-        m = max(m, max(a, b));
-        mm = max(mm, max(a & kIdMask, b & kIdMask));
-    }
+__global__ void max_id_kernel(const uint32_t *s, const uint32_t *d, uint32_t n, uint32_t *out) {
+    uint32_t m = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        m = max(m, max(s[i], d[i]));
     m = __reduce_max_sync(0xffffffffu, m);
-    mm = __reduce_max_sync(0xffffffffu, mm);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(out, m);
-        atomicMax(out + 1, mm);
-    }
+    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
 // Largest id of an edge list (device scalar read back), 0 for no edges.
-static int max_edge_id(const uint32_t *s, const uint32_t *d, uint32_t n, cudaStream_t st, uint32_t *full,
-                       uint32_t *masked) {
-    *full = *masked = 0;
+static int max_edge_id(const uint32_t *s, const uint32_t *d, uint32_t n, cudaStream_t st, uint32_t *out) {
+    *out = 0;
     if (!n) return GBX_OK;
     DevBuf<uint32_t> r;
-    GBX_TRY(r.alloc(2, st));
-    GBX_CUDA(cudaMemsetAsync(r.p, 0, 8, st));
-    id_range_kernel<<<grid1d(n), 256, 0, st>>>(s, d, n, r.p);
+    GBX_TRY(r.alloc(1, st));
+    GBX_CUDA(cudaMemsetAsync(r.p, 0, 4, st));
+    max_id_kernel<<<grid1d(n), 256, 0, st>>>(s, d, n, r.p);
     GBX_LAUNCH_CHECK();
-    uint32_t h[2];
-    GBX_CUDA(cudaMemcpyAsync(h, r.p, 8, cudaMemcpyDeviceToHost, st));
+    GBX_CUDA(cudaMemcpyAsync(out, r.p, 4, cudaMemcpyDeviceToHost, st));
     GBX_CUDA(cudaStreamSynchronize(st));
-    *full = h[0];
-    *masked = h[1];
     return GBX_OK;
 }
 
@@ -461,8 +449,8 @@ extern "C" int gbx_relabel(uint32_t num_vertices, uint32_t num_edges, uint32_t *
     if (os.to_host() && E) GBX_CUDA(cudaMemcpyAsync(os.d, src, (size_t)E * 4, cudaMemcpyHostToDevice, s));
     if (od.to_host() && E) GBX_CUDA(cudaMemcpyAsync(od.d, dst, (size_t)E * 4, cudaMemcpyHostToDevice, s));
     if (ol.to_host()) GBX_CUDA(cudaMemcpyAsync(ol.d, labels, (size_t)V * 4, cudaMemcpyHostToDevice, s));
-    uint32_t id_max = 0, id_masked = 0;
-    GBX_TRY(max_edge_id(os.d, od.d, E, s, &id_max, &id_masked));
+    uint32_t id_max = 0;
+    GBX_TRY(max_edge_id(os.d, od.d, E, s, &id_max));
     GBX_REQUIRE(E == 0 || id_max < V, GBX_ERR_INVALID, "vertex id %u >= num_vertices %u", id_max, V);
     if (E) {
         relabel_edges_kernel<<<grid1d(E), 256, 0, s>>>(os.d, od.d, E, nl.d);
@@ -494,14 +482,15 @@ extern "C" int gbx_mask_graph(uint32_t num_vertices, uint32_t num_edges, uint32_
     GBX_TRY(om.bind(mask_array, V, s));
     if (os.to_host() && E) GBX_CUDA(cudaMemcpyAsync(os.d, src, (size_t)E * 4, cudaMemcpyHostToDevice, s));
     if (od.to_host() && E) GBX_CUDA(cudaMemcpyAsync(od.d, dst, (size_t)E * 4, cudaMemcpyHostToDevice, s));
-    uint32_t id_max = 0, id_masked = 0;
-    GBX_TRY(max_edge_id(os.d, od.d, E, s, &id_max, &id_masked));
+    uint32_t id_max = 0;
+    GBX_TRY(max_edge_id(os.d, od.d, E, s, &id_max));
     GBX_REQUIRE(E == 0 || id_max < V, GBX_ERR_INVALID,
                 "vertex id %u >= num_vertices %u (ids must not carry mask bits yet)", id_max, V);
     DevBuf<uint32_t> key, ids, seen;
     GBX_TRY(key.alloc(V, s));
     GBX_TRY(ids.alloc(V, s));
     GBX_TRY(seen.alloc(1, s));  // the largest id again, not read
+    GBX_CUDA(cudaMemsetAsync(seen.p, 0, 4, s));
     GBX_CUDA(cudaMemsetAsync(key.p, 0, (size_t)V * 4, s));
     // maskGraphProcessGenerateInOutDegrees (reorder.c:1260-1306): in-degrees
     // for 2, 4, in + out for 5, 6, out-degrees otherwise

@@ -237,7 +237,7 @@ struct PullSweep {
         const uint32_t lt = (1u << lane) - 1u;
         const uint4 me = st.me, next = st.next;
         const uint32_t e0 = me.x, e1 = next.x;
-        if (e0 == e1) return;  // several units' first edges lie in one short row: the first has it
+        if (e0 == e1) return;  // several units' first edges lie in one short row: the last has it
         uint32_t row = me.y;          // row of the first pending sum
         uint32_t pending = 0;         // sums in buf
         bool cut = me.z != ~0u;       // the first row began in an earlier unit

@@ -831,7 +831,7 @@ extern "C" int gbx_sssp(gbx_graph *g, uint32_t source, uint32_t delta, uint32_t 
     a.in_far = in_far;
     a.touched = touched;
     a.words = words;
-        // (V / 1024: 1,239 us on RMAT-22, V / 256: 1,229, V / 64: 1,221)
+    // V / 1024: 1,239 us on RMAT-22, V / 256: 1,229, V / 64: 1,221
     a.scan_min = std::max<uint32_t>(8192u, V / 64);
     a.q[0] = q0;
     a.q[1] = q1;

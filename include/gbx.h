@@ -157,7 +157,9 @@ int gbx_bfs(gbx_graph *g, uint32_t source, int mode, uint32_t *distances, int32_
  * graphRun.c:463-595: one breadthFirstSearchGraphCSR per trial, each from a
  * new root): one gbx_bfs traversal per source, enqueued back to back on
  * `stream` with a single host synchronisation after the last; without host
- * outputs several trials run at once. sources and
+ * outputs several trials run at once (with working memory of their own, up to
+ * 4 GB in all, which the device's pool keeps; where there is none they run one
+ * after the other). sources and
  * results are host arrays of num_sources entries; results[i] is what gbx_bfs
  * returns for sources[i]. distances / parents: NULL, or device or host
  * arrays; with out_stride 0 every trial writes the same V entries (the last
