@@ -51,7 +51,7 @@ PR_ITERS = 20
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of each
 # kernel, from ncu captures of this workload on a GB300 (profiles/): bfs the 64
 # roots, sssp the mean of the 4 sources, pr the 20 iterations, spmv one sweep.
-NCU_TRAFFIC_PER_LAUNCH = {"pr": 5.664e9, "bfs": 14.48e9, "sssp": 1.706e9, "spmv": 0.5826e9}
+NCU_TRAFFIC_PER_LAUNCH = {"pr": 5.618e9, "bfs": 14.48e9, "sssp": 1.706e9, "spmv": 0.5818e9}
 W_LO, W_HI = 1, 255
 # differentiable personalised PageRank: RMAT-20, 2^24 edges as generated,
 # lognormal(0,1) weights, 64 teleport columns of 32 seeds, d 0.85 to 1e-7 L1
