@@ -421,7 +421,10 @@ int gbx_tc(gbx_graph *g, uint64_t *total, void *stream);
 /* ---- SpMV ----------------------------------------------------------------- */
 /* y[v] += sum over pull edges (u->v) of w_uv * x[u], `iterations` times.
  * values: per-edge values in pull-CSR order; NULL uses the graph's weights
- * in that order, or default_value when the graph has none. */
+ * in that order, or default_value when the graph has none. With device arrays
+ * the call is stream-ordered and, after a first PageRank or SpMV call on the
+ * graph, may be captured into a CUDA graph; what is captured works in memory
+ * kept with g, so replays of calls captured on one graph must not overlap. */
 int gbx_spmv(gbx_graph *g, const float *values, float default_value, const float *x, float *y,
              uint32_t iterations, void *stream);
 
