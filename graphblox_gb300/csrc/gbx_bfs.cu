@@ -106,12 +106,13 @@ __device__ __forceinline__ void trace_step(Team team, BfsState *st, unsigned kin
 // warps, tells a load-imbalanced step (max close to the step) from a
 // throughput-bound one (mean close to the step).
 struct BusyClock {
-    bool on;
-    unsigned long long t0;
-    __device__ __forceinline__ explicit BusyClock(bool trace) : on(trace), t0(trace ? global_ns() : 0) {}
+    const uint32_t &on;
+    uint32_t t0;  // low word of the start time: registers are short, and a phase is below its four seconds
+    __device__ __forceinline__ explicit BusyClock(const uint32_t &trace)
+        : on(trace), t0(trace ? (uint32_t)global_ns() : 0u) {}
     __device__ __forceinline__ void stop(BfsStep *cnt) {
         if (!on || (threadIdx.x & 31) != 0) return;
-        const unsigned long long d = global_ns() - t0;
+        const unsigned long long d = (uint32_t)global_ns() - t0;
         atomicAdd(&cnt->busy_sum, d);
         atomicMax(&cnt->busy_max, d);
     }
@@ -241,7 +242,7 @@ __device__ void top_down_phase(const BfsArgs &a, Team team, const uint32_t *qin,
                                uint32_t *hvout, uint32_t *hcout, uint32_t lnext, uint32_t *fbm, uint32_t *clear_bm,
                                uint32_t *s_pre, uint32_t *s_base, uint32_t *s_v, uint32_t *s_wq) {
     const uint32_t lane = threadIdx.x & 31;
-    BusyClock clock(a.trace != 0);
+    BusyClock clock(a.trace);
     if (clear_bm) {
         // the bitmap the next top-down step fills (not read during this one)
         for (uint32_t w = team.thread(); w < a.words; w += team.threads())
@@ -387,7 +388,7 @@ __device__ void bottom_up_phase(const BfsArgs &a, Team team, const uint32_t *cur
                                 BfsStep *cnt, uint32_t *qout, uint32_t *hvout, uint32_t *hcout, uint32_t *s_wq,
                                 uint32_t *s_found) {
     const uint32_t lane = threadIdx.x & 31;
-    BusyClock clock(a.trace != 0);
+    BusyClock clock(a.trace);
     unsigned nf = 0;
     unsigned long long edges = 0;
     WarpQueue wq(s_wq, kBfsQueueCap);
@@ -608,7 +609,7 @@ __global__ void bfs_init_kernel(uint32_t *level, int32_t *parent, uint32_t *visi
 // One traversal by a team, whose barrier is gs. kTraced: the trace may be asked
 // for. Teams of several traversals have none; their phases read the clock, if
 // they did, after the flush, where it costs them no registers (before it, or
-// without a clock, 64 trials on RMAT-22 take 6.40 to 6.43 ms instead of 6.32).
+// without a clock, 64 trials on RMAT-22 take 6.40 to 6.43 ms instead of 6.31).
 template <bool kTraced>
 __device__ __forceinline__ void bfs_traverse(const BfsArgs &a, Team team, GridSync *gs) {
     __shared__ uint32_t s_pre[kBfsWarps][33];
